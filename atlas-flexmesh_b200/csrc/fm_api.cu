@@ -101,8 +101,10 @@ struct fm_ctx {
     // reference-pattern assembly
     DevBuf<int32_t> ref_slot;
     DevBuf<double> ke_scratch;
-    DevBuf<unsigned char> elem_rec;  // assembly element-pass records
-    DevBuf<uint32_t> inc_pos, nbr_members;  // node-pass scatter structure
+    DevBuf<double> fvert;            // element pass: vertex forces
+    DevBuf<unsigned char> tan_rec;   // element pass: tangent records
+    DevBuf<uint32_t> act_ptr, act_v, act_pos, nbr_members;  // node-pass scatter structure
+    uint32_t max_pairs = 96;
 
     // solver state
     Work<double> w64;
@@ -274,8 +276,6 @@ fm::MeshDev mesh_view(const fm_ctx* c) {
     m.conn = c->conn.p;
     m.nbr_ptr = c->nbr_ptr.p;
     m.nbr = c->nbr.p;
-    m.inc_ptr = c->inc_ptr.p;
-    m.inc = c->inc_e.p;
     m.mask = c->has_bc ? c->mask.p : nullptr;
     m.mat_mode = c->mat_mode;
     m.m0 = c->m0.p;
@@ -285,9 +285,13 @@ fm::MeshDev mesh_view(const fm_ctx* c) {
     m.c_mu = c->c_mu;
     m.c_lam = c->c_lam;
     m.inv_cnu = c->inv_cnu;
-    m.elem_rec = c->elem_rec.p;
-    m.inc_pos = c->inc_pos.p;
+    m.fvert = c->fvert.p;
+    m.tan_rec = c->tan_rec.p;
+    m.act_ptr = c->act_ptr.p;
+    m.act_v = c->act_v.p;
+    m.act_pos = c->act_pos.p;
     m.nbr_members = c->nbr_members.p;
+    m.max_pairs = c->max_pairs;
     return m;
 }
 
@@ -835,8 +839,8 @@ fm_status fm_set_mesh(fm_ctx* c, uint32_t n_nodes, const double* xyz, uint32_t n
         // assembly's scatter structure, built on the device
         fm::MeshSetupDev md{&c->inc_ptr,      &c->inc_e,    &c->nbr_ptr,  &c->nbr,
                             &c->self_pos,     &c->node_fwd, &c->node_bwd, &c->node_fwd_rec,
-                            &c->node_bwd_rec, &c->emap_ptr, &c->emap,     &c->inc_pos,
-                            &c->nbr_members};
+                            &c->node_bwd_rec, &c->emap_ptr, &c->emap,     &c->act_ptr,
+                            &c->act_v,        &c->act_pos,  &c->nbr_members};
         fm::MeshSetupHost mh;
         int res = fm::kSetupOk;
         CK(fm::build_mesh_device(n_nodes, n_elems, c->conn.p, md, mh, c->status(), &res,
@@ -882,7 +886,9 @@ fm_status fm_set_mesh(fm_ctx* c, uint32_t n_nodes, const double* xyz, uint32_t n
         c->ref_slot.release();
         CK(c->vec_a.reserve(c->n));
         CK(c->vec_b.reserve(c->n));
-        CK(c->elem_rec.reserve(std::max<size_t>(1, (size_t)c->ne * fm::kElemRecBytes)));
+        c->max_pairs = std::max(32u, 3 * mh.max_act);
+        CK(c->fvert.reserve(12 * (size_t)c->ne));
+        CK(c->tan_rec.reserve((size_t)c->ne * fm::kTanRecBytes));
         CK(cudaStreamSynchronize(c->stream));
     } catch (const std::bad_alloc&) {
         return fail(c, FM_ERR_OOM, "host allocation failed in fm_set_mesh");

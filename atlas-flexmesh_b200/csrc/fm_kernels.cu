@@ -1,13 +1,12 @@
 // fm_kernels.cu — sm_100a kernels of the FlexMesh hot path.
 //
-// Assembly: one warp owns one node and writes that node's three CSR rows
-// exactly once (no atomics, deterministic).  Lanes first evaluate the
-// node's incident tets (kinematics, Neo-Hookean stress, tangent scalars) in
-// FP64, stage the per-tet data in shared memory, then each lane forms the
-// 3x3 block of one neighbour node by summing over the tets that contain the
-// edge (node, neighbour).  The diagonal block is minus the sum of the
-// off-diagonal blocks (rows of every element tangent sum to zero because
-// the shape gradients do).
+// Assembly: an element pass evaluates every tet once (kinematics,
+// Neo-Hookean stress, tangent scalars, FP64); in the node pass one warp owns
+// one node and writes that node's three CSR rows exactly once (no atomics,
+// deterministic), from the 3x3 blocks its lanes form, one tet each.  The
+// diagonal block is minus the sum of the off-diagonal blocks (rows of every
+// element tangent sum to zero because the shape gradients do).  Without a
+// tangent the node pass is a gather of the vertex forces.
 //
 // Solvers: SpMV over the node-block pattern, and sync-free ILU(0) and
 // triangular solves: a persistent grid walks the rows in a topological
@@ -25,102 +24,83 @@ namespace fm {
 // ===========================================================================
 constexpr int kAsmWarps = 8;
 
+// The element pass leaves per tet the 12 components of its vertex forces
+// vol M dN_a (fvert, FP64: 96 bytes) and, when a tangent is assembled, a
+// record in the tangent's type: the shape gradients and the tangent scalars
+// vol a, vol b, vol mu.  dN_0 = -dN_1 - dN_2 - dN_3, as tet_kinematics forms
+// it, so the FP64 record leaves it out (96 bytes); the FP32 record keeps it
+// (64 bytes): summing the rounded gradients would lose precision.
 template <typename KT>
-struct AsmStage {
-    KT d[32][12];     // shape gradients of the 4 nodes of incident tet l; after
-                      // phase 2 reused as the [lane][9] gather of the row blocks
-    KT fI[32][3];     // vol M dN_owner of tet l (force, and geometric term)
-    KT vabm[32][3];   // vol*a, vol*b, vol*mu (tangent scalars)
-    double f64[3][32];  // FP64 node-force contributions of the incident tets
-    uint32_t pos[32]; // 4 x u8: position of each tet node in the owner's neighbour list
-};
-
-__device__ __forceinline__ int find_sorted(const uint32_t* a, int len, uint32_t key) {
-    int lo = 0, hi = len - 1;
-    while (lo <= hi) {
-        const int mid = (lo + hi) >> 1;
-        const uint32_t v = a[mid];
-        if (v == key) return mid;
-        if (v < key) lo = mid + 1;
-        else hi = mid - 1;
-    }
-    return -1;
-}
-
-__device__ __forceinline__ int byte_index(uint32_t packed, uint32_t key) {
-    // which of the 4 bytes equals key (0..3), -1 if none
-    if ((packed & 0xffu) == key) return 0;
-    if (((packed >> 8) & 0xffu) == key) return 1;
-    if (((packed >> 16) & 0xffu) == key) return 2;
-    if ((packed >> 24) == key) return 3;
-    return -1;
-}
-
-// Element record (AoS, 16-byte multiple): vertex forces vol M dN_a (FP64,
-// 4x3), shape gradients dN_a (4x3) and tangent scalars vol a, vol b, vol mu
-// in the tangent's type, and an activity mark (0: skipped or degenerate).
-template <typename KT>
-struct ElemRec;
+struct TanRec;
 template <>
-struct __align__(16) ElemRec<double> {
-    double f[12];
-    double d[12];
+struct __align__(16) TanRec<double> {
+    static constexpr int kFirst = 1;  // first stored gradient
+    double d[9];
     double s[3];
-    double active;
 };
 template <>
-struct __align__(16) ElemRec<float> {
-    double f[12];
+struct __align__(16) TanRec<float> {
+    static constexpr int kFirst = 0;
     float d[12];
     float s[3];
-    float active;
+    float pad;
 };
-static_assert(sizeof(ElemRec<double>) <= kElemRecBytes && sizeof(ElemRec<double>) % 16 == 0, "");
-static_assert(sizeof(ElemRec<float>) <= kElemRecBytes && sizeof(ElemRec<float>) % 16 == 0, "");
+static_assert(sizeof(TanRec<double>) <= kTanRecBytes && sizeof(TanRec<double>) % 16 == 0, "");
+static_assert(sizeof(TanRec<float>) <= kTanRecBytes && sizeof(TanRec<float>) % 16 == 0, "");
 
-// 16-byte stores of a whole record from registers
-__device__ __forceinline__ void store_rec(ElemRec<double>* dst, const ElemRec<double>& r) {
-    double2* f = reinterpret_cast<double2*>(dst->f);
-    double2* d = reinterpret_cast<double2*>(dst->d);
+// The lanes' records (W 8-byte words each, in registers) to consecutive
+// records of global memory, through the warp's stage so that every store
+// instruction writes whole 512-byte runs: a lane's own 16-byte stores, one
+// record apart from the next lane's, took 128 us of the 64^3 residual's
+// element pass against 44 us.  The stage rows are padded to an odd number of
+// words, so neither side has bank conflicts.
+template <int W>
+__device__ __forceinline__ void store_records(double* dst, uint32_t n_rec, const double (&r)[W],
+                                              double* stage, int lane) {
+    static_assert(W % 2 == 0, "records are whole 16-byte units");
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        f[i] = make_double2(r.f[2 * i], r.f[2 * i + 1]);
-        d[i] = make_double2(r.d[2 * i], r.d[2 * i + 1]);
+    for (int i = 0; i < W; ++i) stage[lane * (W + 1) + i] = r[i];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < W / 2; ++i) {
+        const int t = lane + 32 * i, rec = t / (W / 2), o = 2 * (t % (W / 2));
+        if (rec < (int)n_rec) {
+            const double* q = stage + rec * (W + 1) + o;
+            reinterpret_cast<double2*>(dst)[t] = make_double2(q[0], q[1]);
+        }
     }
-    double2* t = reinterpret_cast<double2*>(dst->s);
-    t[0] = make_double2(r.s[0], r.s[1]);
-    t[1] = make_double2(r.s[2], r.active);
-}
-__device__ __forceinline__ void store_rec(ElemRec<float>* dst, const ElemRec<float>& r) {
-    double2* f = reinterpret_cast<double2*>(dst->f);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) f[i] = make_double2(r.f[2 * i], r.f[2 * i + 1]);
-    float4* d = reinterpret_cast<float4*>(dst->d);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) d[i] = make_float4(r.d[4 * i], r.d[4 * i + 1], r.d[4 * i + 2], r.d[4 * i + 3]);
-    *reinterpret_cast<float4*>(dst->s) = make_float4(r.s[0], r.s[1], r.s[2], r.active);
+    __syncwarp();
 }
 
-// One tet of the element pass: kinematics, Mandel stress, the four vertex
-// forces (FP64) and, with_k, the tangent scalars and shape gradients in the
-// tangent's type, stored as one 16-byte-aligned record.  Returns the flags.
-template <typename KT>
-__device__ __forceinline__ unsigned asm_element(const MeshDev& m, const double* __restrict__ u,
-                                                uint32_t e, ElemRec<KT>* dst_rec, int with_k) {
+// 8-byte word i of a record held in registers
+__device__ __forceinline__ double word_of(const double* r, int i) { return r[i]; }
+__device__ __forceinline__ double word_of(const float* r, int i) {
+    return __hiloint2double(__float_as_int(r[2 * i + 1]), __float_as_int(r[2 * i]));
+}
+
+// Element pass: one thread per tet.  WithK = false (residual only) leaves
+// out the tangent records.
+template <typename KT, bool WithK>
+__global__ void __launch_bounds__(128, 4)
+    k_asm_elements(MeshDev m, const double* __restrict__ u, double* __restrict__ fvert,
+                   TanRec<KT>* __restrict__ tan, unsigned* __restrict__ status) {
+    __shared__ double stage_s[4][32 * 13];
+    const int lane = threadIdx.x & 31;
+    double* stage = stage_s[threadIdx.x >> 5];
+    const uint32_t e0 = blockIdx.x * 128u + (threadIdx.x & ~31u);  // the warp's first tet
+    if (e0 >= m.n_elems) return;                                   // uniform per warp
+    const uint32_t e = e0 + lane, n_rec = min(32u, m.n_elems - e0);
     unsigned flags = 0;
-    uint4 c = m.conn[e];
-    const bool active = !(c.x & 0x80000000u);
-    c.x &= 0x7fffffffu;
-    const uint32_t cn[4] = {c.x, c.y, c.z, c.w};
-    ElemRec<KT> r;
+    double f[12];
+    KT r[sizeof(TanRec<KT>) / sizeof(KT)];  // the tangent record
 #pragma unroll
-    for (int i = 0; i < 12; ++i) {
-        r.f[i] = 0.0;
-        r.d[i] = KT(0);
-    }
-    r.s[0] = r.s[1] = r.s[2] = KT(0);
-    r.active = KT(0);
-    if (active) {
+    for (int i = 0; i < 12; ++i) f[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(TanRec<KT>) / sizeof(KT)); ++i) r[i] = KT(0);
+    uint4 c = make_uint4(0x80000000u, 0, 0, 0);
+    if (e < m.n_elems) c = m.conn[e];
+    if (!(c.x & 0x80000000u)) {
+        const uint32_t cn[4] = {c.x, c.y, c.z, c.w};
         double x[12], ue[12];
 #pragma unroll
         for (int a = 0; a < 4; ++a)
@@ -138,189 +118,301 @@ __device__ __forceinline__ unsigned asm_element(const MeshDev& m, const double* 
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
                 const double* dI = k.d[a];
-                r.f[3 * a + 0] = k.vol * (M.m00 * dI[0] + M.m01 * dI[1] + M.m02 * dI[2]);
-                r.f[3 * a + 1] = k.vol * (M.m01 * dI[0] + M.m11 * dI[1] + M.m12 * dI[2]);
-                r.f[3 * a + 2] = k.vol * (M.m02 * dI[0] + M.m12 * dI[1] + M.m22 * dI[2]);
-                fs += r.f[3 * a] + r.f[3 * a + 1] + r.f[3 * a + 2];
+                f[3 * a + 0] = k.vol * (M.m00 * dI[0] + M.m01 * dI[1] + M.m02 * dI[2]);
+                f[3 * a + 1] = k.vol * (M.m01 * dI[0] + M.m11 * dI[1] + M.m12 * dI[2]);
+                f[3 * a + 2] = k.vol * (M.m02 * dI[0] + M.m12 * dI[1] + M.m22 * dI[2]);
+                fs += f[3 * a] + f[3 * a + 1] + f[3 * a + 2];
             }
             if (!(k.J > 0.0)) flags |= FM_FLAG_INVERTED;
             if (k.J < kJSafe) flags |= FM_FLAG_J_CLAMPED;
             if (!isfinite(fs)) flags |= FM_FLAG_NONFINITE;
-            if (with_k) {
+            if (WithK) {
                 double a, b;
                 tangent_ab(mu, lam, k.J, M.lnJ, m.inv_cnu, a, b);
+                constexpr int q0 = TanRec<KT>::kFirst;
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
+                for (int q = q0; q < 4; ++q)
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) r.d[3 * q + d] = (KT)k.d[q][d];
-                r.s[0] = (KT)(k.vol * a);
-                r.s[1] = (KT)(k.vol * b);
-                r.s[2] = (KT)(k.vol * mu);
+                    for (int d = 0; d < 3; ++d) r[3 * (q - q0) + d] = (KT)k.d[q][d];
+                constexpr int s0 = 3 * (4 - q0);
+                r[s0] = (KT)(k.vol * a);
+                r[s0 + 1] = (KT)(k.vol * b);
+                r[s0 + 2] = (KT)(k.vol * mu);
                 if (!isfinite(a + b)) flags |= FM_FLAG_NONFINITE;
             }
-            r.active = KT(1);
         }
     }
-    store_rec(dst_rec, r);
-    return flags;
-}
-
-// Element pass: one thread per tet.  with_k = 0 (residual only) skips the
-// tangent scalars and gradients.
-template <typename KT>
-__global__ void __launch_bounds__(128, 4)
-    k_asm_elements(MeshDev m, const double* __restrict__ u, ElemRec<KT>* __restrict__ rec,
-                   int with_k, unsigned* __restrict__ status) {
-    unsigned flags = 0;
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m.n_elems;
-         e += gridDim.x * blockDim.x)
-        flags |= asm_element<KT>(m, u, e, rec + e, with_k);
+    store_records<12>(fvert + 12 * (size_t)e0, n_rec, f, stage, lane);
+    if (WithK) {
+        constexpr int W = (int)(sizeof(TanRec<KT>) / 8);
+        double w[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i) w[i] = word_of(r, i);
+        store_records<W>(reinterpret_cast<double*>(tan + e0), n_rec, w, stage, lane);
+    }
     if (flags) raise_flag(status, flags);
 }
 
-// Node pass for one node: one warp owns it.  Lane l < mi stages incident
-// tet l's record (gradients, the owner's vertex force, tangent scalars) in
-// shared memory; lane k then forms block (n, nbr[k]).
-template <typename KT>
-__device__ __forceinline__ void asm_node(const MeshDev& m, const ElemRec<KT>* __restrict__ rec,
-                                         uint32_t n, KT* __restrict__ K,
-                                         double* __restrict__ f, double* __restrict__ R,
-                                         int apply_bc, AsmStage<KT>& S, int lane) {
+// Sum of the vertex forces of each node's tets, ascending element order: one
+// thread per DOF (36 us at 64^3, L2-bound; a warp per node that staged whole
+// records took 217).  f (may be null) gets the sums, R (may be null) minus them,
+// zero on constrained DOFs.
+__global__ void __launch_bounds__(256)
+    k_gather_forces(uint32_t n_nodes, const uint32_t* __restrict__ act_ptr,
+                    const uint32_t* __restrict__ act_v, const double* __restrict__ fvert,
+                    const uint8_t* __restrict__ mask, double* __restrict__ f,
+                    double* __restrict__ R) {
+    const uint32_t row = blockIdx.x * 256u + threadIdx.x;
+    if (row >= 3 * n_nodes) return;
+    const uint32_t n = row / 3, c = row - 3 * n;
+    const uint32_t b = __ldg(act_ptr + n), e = __ldg(act_ptr + n + 1);
+    double s = 0.0;
+    uint32_t i = b;
+    for (; i + 8 <= e; i += 8) {  // eight gathers in flight
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = __ldg(fvert + 3 * (size_t)__ldg(act_v + i + q) + c);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s += v[q];
+    }
+    for (; i < e; ++i) s += __ldg(fvert + 3 * (size_t)__ldg(act_v + i) + c);
+    if (f) f[row] = s;
+    if (R) R[row] = (mask && mask[row]) ? 0.0 : -s;
+}
 
-    const uint32_t nb0 = m.nbr_ptr[n];
-    const int deg = (int)(m.nbr_ptr[n + 1] - nb0);
-    const uint32_t e0 = m.inc_ptr[n];
-    const int mi = (int)(m.inc_ptr[n + 1] - e0);
-    const uint32_t my_nbr = lane < deg ? __ldg(m.nbr + nb0 + lane) : 0xffffffffu;
-    const int self_k = __ffs(__ballot_sync(kFull, my_nbr == n)) - 1;
-    // edge lists of the tangent blocks: structural, built on the host
-    const uint32_t my_members = (K != nullptr && lane < deg) ? __ldg(m.nbr_members + nb0 + lane) : 0u;
+void launch_gather_forces(const MeshDev& m, double* f, double* R, cudaStream_t s) {
+    k_gather_forces<<<(3 * m.n_nodes + 255) / 256, 256, 0, s>>>(m.n_nodes, m.act_ptr, m.act_v,
+                                                               m.fvert, m.mask, f, R);
+}
 
-    double fi0 = 0.0, fi1 = 0.0, fi2 = 0.0;
-    uint32_t packed = 0xffffffffu;
-    if (lane < mi) {
-        const uint32_t e = __ldg(m.inc + e0 + lane);
-        packed = __ldg(m.inc_pos + e0 + lane);
-        const ElemRec<KT>& r = rec[e];
-        const bool act = r.active != KT(0);
-        if (act) {
-            const int il = byte_index(packed, (uint32_t)self_k);
-            fi0 = r.f[3 * il];
-            fi1 = r.f[3 * il + 1];
-            fi2 = r.f[3 * il + 2];
-        }
-        if (K != nullptr) {
-            // an inactive tet (degenerate at this state) stays in the edge
-            // lists with zero data: it adds exact zeros
+// gradients of a tet's four vertices and its tangent scalars
+__device__ __forceinline__ void load_tan(const TanRec<double>* p, double D[4][3], double s[3]) {
+    const double2* q = reinterpret_cast<const double2*>(p);
+    double w[12];
 #pragma unroll
-            for (int q = 0; q < 12; ++q) S.d[lane][q] = act ? r.d[q] : KT(0);
-            S.fI[lane][0] = (KT)fi0;
-            S.fI[lane][1] = (KT)fi1;
-            S.fI[lane][2] = (KT)fi2;
-            S.vabm[lane][0] = act ? r.s[0] : KT(0);
-            S.vabm[lane][1] = act ? r.s[1] : KT(0);
-            S.vabm[lane][2] = act ? r.s[2] : KT(0);
-        }
+    for (int i = 0; i < 6; ++i) {
+        const double2 v = __ldg(q + i);
+        w[2 * i] = v.x;
+        w[2 * i + 1] = v.y;
     }
-    S.pos[lane] = packed;
-    S.f64[0][lane] = fi0;
-    S.f64[1][lane] = fi1;
-    S.f64[2][lane] = fi2;
-    __syncwarp();
-
-    // internal force of the node: lane p < 3 sums component p over the
-    // incident tets in ascending element order (deterministic).  Shared
-    // gathers replace FP64 shuffle trees, which are slow after divergence.
-    if (lane < 3) {
-        double fv = 0.0;
-        for (int l = 0; l < mi; ++l) fv += S.f64[lane][l];
-        const uint32_t row = 3 * n + lane;
-        if (f) f[row] = fv;
-        if (R) R[row] = (m.mask && m.mask[row]) ? 0.0 : -fv;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        D[1][c] = w[c];
+        D[2][c] = w[3 + c];
+        D[3][c] = w[6 + c];
+        D[0][c] = -w[c] - w[3 + c] - w[6 + c];
+        s[c] = w[9 + c];
     }
-    if (K == nullptr) return;
-    __syncwarp();
-
-    // phase 2: lane k forms block (n, nbr[k]) from the tets on that edge
-    KT acc[9];
+}
+__device__ __forceinline__ void load_tan(const TanRec<float>* p, float D[4][3], float s[3]) {
+    const float4* q = reinterpret_cast<const float4*>(p);
+    float w[16];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) acc[q] = KT(0);
-    if (lane < deg && lane != self_k) {
-        uint32_t members = my_members;
-        while (members) {
-            const int l = __ffs(members) - 1;
-            members &= members - 1;
-            const uint32_t pk = S.pos[l];
-            const int j = byte_index(pk, (uint32_t)lane);
-            const int il = byte_index(pk, (uint32_t)self_k);
-            tangent_block_acc<KT>(&S.d[l][3 * il], &S.d[l][3 * j], S.fI[l], S.vabm[l][0],
-                                  S.vabm[l][1], S.vabm[l][2], acc);
-        }
+    for (int i = 0; i < 4; ++i) {
+        const float4 v = __ldg(q + i);
+        w[4 * i] = v.x;
+        w[4 * i + 1] = v.y;
+        w[4 * i + 2] = v.z;
+        w[4 * i + 3] = v.w;
     }
-    // diagonal block = - sum of off-diagonal blocks of the row block: lane
-    // q < 9 sums entry q over the neighbour lanes (fixed order)
-    __syncwarp();
-    KT* red = &S.d[0][0];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) red[9 * lane + q] = acc[q];
-    __syncwarp();
-    if (lane < 9) {
-        KT s = KT(0);
-        for (int l = 0; l < deg; ++l) s += red[9 * l + lane];
-        red[9 * self_k + lane] = -s;
-    }
-    __syncwarp();
-    if (lane == self_k) {
+    for (int c = 0; c < 3; ++c) {
 #pragma unroll
-        for (int q = 0; q < 9; ++q) acc[q] = red[9 * self_k + q];
-    }
-    if (lane < deg) {
-        const uint32_t col0 = 3 * my_nbr;
-#pragma unroll
-        for (int p = 0; p < 3; ++p) {
-            const uint32_t row = 3 * n + p;
-            const size_t base = 9 * (size_t)nb0 + 3 * (size_t)p * deg + 3 * lane;
-            const bool mrow = apply_bc && m.mask && m.mask[row];
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                KT v = acc[3 * p + q];
-                if (apply_bc && m.mask && (mrow || m.mask[col0 + q]))
-                    v = (row == col0 + q) ? KT(1) : KT(0);
-                K[base + q] = v;
-            }
-        }
+        for (int a = 0; a < 4; ++a) D[a][c] = w[3 * a + c];
+        s[c] = w[12 + c];
     }
 }
 
-// CTAs per SM: the FP64 pass fits 64 registers for four without spilling
-// (32 resident warps instead of 24: 0.784 -> 0.733 ms at 64^3), the FP32
-// pass 40 for six (0.540 -> 0.531 ms).
+// Node pass: one warp owns node n and writes its three CSR rows once (no
+// atomics, every sum in a fixed order).
+//   1. Lane l takes the node's l-th active tet: loads its record, turns it so
+//      that the owner's gradient comes first, and forms the 3x3 blocks
+//      against the tet's three other vertices.  The blocks go to shared
+//      memory grouped by neighbour: block (l, k) in slot start[k] + (number
+//      of tets before l on the edge to k).
+//   2. Lane c takes column c of the rows (c = 3k + q) and sums the slots of
+//      neighbour k, ascending element order, for the three rows at once.
+//   3. The diagonal block is minus the sum of the row's other blocks.
+// Bound: the L1 data pipe (78% busy at 64^3 FP64: about 340 shared-memory and
+// 120 global wavefronts per node, half of the shared ones bank conflicts of
+// the slot exchange).  One lane per neighbour walking its tets kept 15 of 32
+// lanes busy; this keeps 23 (whole assembly: 128^3 FP64 5.67 -> 4.99 ms, 33^3
+// FP32 88 -> 70 us).
 template <typename KT>
-__global__ void __launch_bounds__(kAsmWarps * 32, sizeof(KT) == 4 ? 6 : 4)
-    k_assemble(MeshDev m, const ElemRec<KT>* __restrict__ rec, KT* __restrict__ K,
-               double* __restrict__ f, double* __restrict__ R, int apply_bc,
-               unsigned* __restrict__ status) {
-    (void)status;
-    __shared__ AsmStage<KT> stage[kAsmWarps];
-    const int lane = threadIdx.x & 31;
-    const int wi = threadIdx.x >> 5;
+__global__ void __launch_bounds__(kAsmWarps * 32, sizeof(KT) == 4 ? 4 : 3)
+    k_assemble(MeshDev m, const TanRec<KT>* __restrict__ tan, KT* __restrict__ K,
+               double* __restrict__ f, double* __restrict__ R, int apply_bc) {
+    extern __shared__ __align__(16) unsigned char asm_smem[];
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    double* F = reinterpret_cast<double*>(asm_smem) + wi * 96;
+    KT* C = reinterpret_cast<KT*>(asm_smem + kAsmWarps * 96 * sizeof(double)) +
+            (size_t)wi * 9 * m.max_pairs;
     const uint32_t n = blockIdx.x * kAsmWarps + wi;
     if (n >= m.n_nodes) return;  // uniform per warp
-    asm_node<KT>(m, rec, n, K, f, R, apply_bc, stage[wi], lane);
+    const uint32_t nb0 = m.nbr_ptr[n];
+    const int deg = (int)(m.nbr_ptr[n + 1] - nb0);
+    const uint32_t a0 = m.act_ptr[n];
+    const int ma = (int)(m.act_ptr[n + 1] - a0);
+    const uint32_t v = lane < ma ? __ldg(m.act_v + a0 + lane) : 0u;
+    uint32_t pos = lane < ma ? __ldg(m.act_pos + a0 + lane) : 0xffffffffu;
+    const uint32_t my_nbr = lane < deg ? __ldg(m.nbr + nb0 + lane) : 0xffffffffu;
+    const uint32_t memb = lane < deg ? __ldg(m.nbr_members + nb0 + lane) : 0u;
+    const bool bc = apply_bc && m.mask;
+    uint32_t fixed = 0;  // the neighbour's constrained DOFs, one bit each
+    if (bc && lane < deg) {
+        const uint8_t* q = m.mask + 3 * (size_t)my_nbr;
+        fixed = (q[0] ? 1u : 0u) | (q[1] ? 2u : 0u) | (q[2] ? 4u : 0u);
+    }
+    KT D[4][3], sc[3];
+    double fo[3] = {0.0, 0.0, 0.0};
+    if (lane < ma) {
+        load_tan(tan + (v >> 2), D, sc);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) fo[c] = __ldg(m.fvert + 3 * (size_t)v + c);
+    }
+    const int self_k = __ffs(__ballot_sync(kFull, my_nbr == n)) - 1;
+    const int cnt = __popc(memb);
+    int start = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(kFull, start, o);
+        if (lane >= o) start += t;
+    }
+    start -= cnt;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) F[32 * c + lane] = fo[c];
+    // rotate by the owner's local index: D[0] is its gradient
+    const bool r1 = v & 1u, r2 = v & 2u;
+    pos = __funnelshift_r(pos, pos, 8 * (v & 3u));
+    KT dI[3], hI[3], aI[3], bI[3], mI[3];
+    if (lane < ma) {
+        KT T[4][3];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) T[a][c] = r1 ? D[(a + 1) & 3][c] : D[a][c];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) D[a][c] = r2 ? T[(a + 2) & 3][c] : T[a][c];
+        // K_pq = va dI_p dJ_q (p==q) + vb dI_p dJ_q (p!=q)
+        //      + vm (p==q ? sum_{r!=p} dI_r dJ_r : dI_q dJ_p) + (p==q) fI.dJ
+        // with the products by dI formed once per tet
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            dI[c] = D[0][c];
+            bI[c] = sc[1] * dI[c];
+            mI[c] = sc[2] * dI[c];
+            aI[c] = sc[0] * dI[c] - mI[c];
+            hI[c] = (KT)fo[c] + mI[c];
+        }
+    }
+#pragma unroll
+    for (int j = 1; j < 4; ++j) {
+        const uint32_t k = (pos >> (8 * j)) & 0xffu;  // 0xff: no block there
+        const uint32_t mk = __shfl_sync(kFull, memb, k & 31u);
+        const int st = __shfl_sync(kFull, start, k & 31u);
+        if (k != 0xffu && ((mk >> lane) & 1u)) {
+            KT* o = C + 9 * (st + __popc(mk & ((1u << lane) - 1u)));
+            const KT* dJ = D[j];
+            const KT S = hI[0] * dJ[0] + hI[1] * dJ[1] + hI[2] * dJ[2];
+            o[0] = S + aI[0] * dJ[0];
+            o[1] = bI[0] * dJ[1] + mI[1] * dJ[0];
+            o[2] = bI[0] * dJ[2] + mI[2] * dJ[0];
+            o[3] = bI[1] * dJ[0] + mI[0] * dJ[1];
+            o[4] = S + aI[1] * dJ[1];
+            o[5] = bI[1] * dJ[2] + mI[2] * dJ[1];
+            o[6] = bI[2] * dJ[0] + mI[0] * dJ[2];
+            o[7] = bI[2] * dJ[1] + mI[1] * dJ[2];
+            o[8] = S + aI[2] * dJ[2];
+        }
+    }
+    __syncwarp();
+    if (lane < 3 && (f || R)) {
+        double s = 0.0;
+        for (int l = 0; l < ma; ++l) s += F[32 * lane + l];
+        const uint32_t row = 3 * n + lane;
+        if (f) f[row] = s;
+        if (R) R[row] = (m.mask && m.mask[row]) ? 0.0 : -s;
+    }
+    const int rl = 3 * deg;
+    KT acc[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        acc[r][0] = acc[r][1] = acc[r][2] = KT(0);
+        if (32 * r < rl) {  // uniform
+            const int c = lane + 32 * r, k = c / 3;
+            const int st = __shfl_sync(kFull, start, k & 31), ck = __shfl_sync(kFull, cnt, k & 31);
+            if (c < rl) {
+                const KT* q = C + 9 * st + (c - 3 * k);
+                for (int i = 0; i < ck; ++i, q += 9) {
+                    acc[r][0] += q[0];
+                    acc[r][1] += q[3];
+                    acc[r][2] += q[6];
+                }
+            }
+        }
+    }
+    __syncwarp();  // the slots are read: reuse them for the rows
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const int c = lane + 32 * r;
+        if (c < rl)
+#pragma unroll
+            for (int p = 0; p < 3; ++p) C[p * rl + c] = acc[r][p];
+    }
+    __syncwarp();
+    // diagonal block: lane (third, p, q) sums entry (p, q) of every third
+    // neighbour, then the thirds are added
+    {
+        const int third = lane / 9, pq = lane - 9 * third, p = pq / 3, q = pq - 3 * p;
+        KT s = KT(0);
+        if (lane < 27)
+            for (int k = third; k < deg; k += 3) s += C[p * rl + 3 * k + q];
+        const KT s1 = __shfl_sync(kFull, s, pq + 9), s2 = __shfl_sync(kFull, s, (pq + 18) & 31);
+        if (lane < 9 && deg) C[p * rl + 3 * self_k + q] = -(s + s1 + s2);
+    }
+    __syncwarp();
+    KT* out = K + 9 * (size_t)nb0;
+    const uint32_t fixed_row = __shfl_sync(kFull, fixed, self_k & 31);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        if (32 * r < rl) {  // uniform
+            const int c = lane + 32 * r, k = c / 3, q = c - 3 * k;
+            const uint32_t fc = (__shfl_sync(kFull, fixed, k & 31) >> q) & 1u;
+            if (c < rl)
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    KT val = k == self_k ? C[p * rl + c] : acc[r][p];
+                    if (bc && (fc || ((fixed_row >> p) & 1u)))
+                        val = (k == self_k && p == q) ? KT(1) : KT(0);
+                    out[p * rl + c] = val;
+                }
+        }
+    }
 }
 
 template <typename KT>
 static void launch_assemble_t(const MeshDev& m, const double* u, KT* K, double* f, double* R,
                               int apply_bc, unsigned* status, cudaStream_t s) {
     if (m.n_nodes == 0) return;
-    ElemRec<KT>* rec = static_cast<ElemRec<KT>*>(m.elem_rec);
-    if (m.n_elems) {
-        unsigned ge = (m.n_elems + 127) / 128;
-        if (ge > 148u * 32u) ge = 148u * 32u;
-        k_asm_elements<KT><<<ge, 128, 0, s>>>(m, u, rec, K != nullptr, status);
+    const unsigned ge = (m.n_elems + 127) / 128;
+    TanRec<KT>* tan = static_cast<TanRec<KT>*>(m.tan_rec);
+    if (!K) {
+        if (ge) k_asm_elements<KT, false><<<ge, 128, 0, s>>>(m, u, m.fvert, tan, status);
+        launch_gather_forces(m, f, R, s);
+        return;
     }
+    if (ge) k_asm_elements<KT, true><<<ge, 128, 0, s>>>(m, u, m.fvert, tan, status);
     const unsigned grid = (m.n_nodes + kAsmWarps - 1) / kAsmWarps;
-    k_assemble<KT><<<grid, kAsmWarps * 32, 0, s>>>(m, rec, K, f, R, apply_bc, status);
+    const size_t smem = kAsmWarps * (96 * sizeof(double) + 9 * m.max_pairs * sizeof(KT));
+    // at most 8 x (768 + 9 x 96 x 8) = 61,440 bytes: above the 48 KB every
+    // kernel may use, so the limit is raised (per device, on each launch: the
+    // call is cheap and keeps no state)
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(k_assemble<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem);
+    k_assemble<KT><<<grid, kAsmWarps * 32, smem, s>>>(m, tan, K, f, R, apply_bc);
 }
 void launch_assemble(const MeshDev& m, const double* u, double* K, double* f, double* R,
                      int apply_bc, unsigned* status, cudaStream_t s) {
@@ -520,6 +612,18 @@ void launch_spmv_csr(uint32_t n, const uint32_t* rp, const uint32_t* ci, const T
 // ===========================================================================
 // Sync-free ILU(0) and triangular solves (scalar CSR rows, warp per row)
 // ===========================================================================
+__device__ __forceinline__ int find_sorted(const uint32_t* a, int len, uint32_t key) {
+    int lo = 0, hi = len - 1;
+    while (lo <= hi) {
+        const int mid = (lo + hi) >> 1;
+        const uint32_t v = a[mid];
+        if (v == key) return mid;
+        if (v < key) lo = mid + 1;
+        else hi = mid - 1;
+    }
+    return -1;
+}
+
 constexpr int kSfWarps = 8;  // warps per block of the persistent kernels
 
 // Row i of ILU(0), IKJ form in natural order, which performs the same

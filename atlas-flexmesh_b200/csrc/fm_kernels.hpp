@@ -15,8 +15,6 @@ struct MeshDev {
     const uint4* conn = nullptr;       // n_elems, bit 31 of .x = element skipped
     const uint32_t* nbr_ptr = nullptr; // n_nodes+1
     const uint32_t* nbr = nullptr;     // node neighbours, sorted
-    const uint32_t* inc_ptr = nullptr; // n_nodes+1
-    const uint32_t* inc = nullptr;     // incident elements, ascending
     const uint8_t* mask = nullptr;     // n_dofs Dirichlet mask (may be null)
     // material: mode 0 scalar (mu_s, lam_s), 1 per-element E (m0) with
     // mu = E c_mu, lam = E c_lam, 2 per-element Lame (m0 = mu, m1 = lam)
@@ -24,28 +22,37 @@ struct MeshDev {
     const double* m0 = nullptr;
     const double* m1 = nullptr;
     double mu_s = 0, lam_s = 0, c_mu = 0, c_lam = 0, inv_cnu = 0;
-    // per-element records of the assembly's element pass (n_elems *
-    // kElemRecBytes bytes, 16-byte aligned)
-    void* elem_rec = nullptr;
-    // structural scatter data of the node pass, built once per mesh:
-    // inc_pos[i]: positions (4 x u8) of incidence i's tet vertices in the
-    // owner's neighbour list; nbr_members[j]: bit l set when the owner's
-    // l-th incident tet (not skipped) holds the edge to neighbour entry j
-    const uint32_t* inc_pos = nullptr;
+    // element pass -> node pass: vertex forces (12 per tet) and tangent
+    // records (kTanRecBytes per tet, 16-byte aligned)
+    double* fvert = nullptr;
+    void* tan_rec = nullptr;
+    // the active (not skipped) tets of each node, ascending, built once per
+    // mesh: act_v[i] = 4 tet + the owner's local index; act_pos[i]: positions
+    // (4 x u8) of the tet's vertices in the owner's neighbour list, 0xff for
+    // a vertex that repeats an earlier one; nbr_members[j]: bit l set when
+    // the owner's l-th active tet holds the edge to neighbour entry j;
+    // max_pairs: most (tet, other vertex) pairs of a node, at least 32
+    const uint32_t* act_ptr = nullptr;
+    const uint32_t* act_v = nullptr;
+    const uint32_t* act_pos = nullptr;
     const uint32_t* nbr_members = nullptr;
+    uint32_t max_pairs = 96;
 };
-constexpr size_t kElemRecBytes = 224;
-
+constexpr size_t kTanRecBytes = 96;
 
 // A10/A11/A12: assembly in two passes, an element pass (each tet's
 // kinematics, stress, vertex forces and tangent scalars, once) and a
-// node-owner pass that writes every CSR row block once.  K (double or float,
+// node-owner pass that writes every CSR row block once (without K: a gather
+// of the vertex forces).  K (double or float,
 // may be null for a residual-only call), f (FP64, may be null), R = -f with
-// zeros on constrained DOFs (may be null).  m.elem_rec is required.
+// zeros on constrained DOFs (may be null).  m.fvert and m.tan_rec are required.
 void launch_assemble(const MeshDev& m, const double* u, double* K, double* f, double* R,
                      int apply_bc, unsigned* status, cudaStream_t s);
 void launch_assemble(const MeshDev& m, const double* u, float* K, double* f, double* R,
                      int apply_bc, unsigned* status, cudaStream_t s);
+// f (may be null) = the vertex forces in m.fvert summed per node, R (may be
+// null) = -f with zeros on constrained DOFs
+void launch_gather_forces(const MeshDev& m, double* f, double* R, cudaStream_t s);
 // Element-centric scatter through an int32 slot map (reference pattern).
 // K and f must be zeroed by the caller; Ke_scratch holds 144*n_elems doubles.
 void launch_assemble_slotmap(const MeshDev& m, const double* u, const int32_t* slot, double* K,

@@ -236,36 +236,66 @@ __global__ void __launch_bounds__(kSetupWarps * 32)
     }
 }
 
-// node-pass scatter structure of the assembly: per incidence the 4 vertex
-// positions in the owner's list, per neighbour entry the owner's incident
-// (not skipped) tets holding that edge
+// active (not skipped) incident tets per node
+__global__ void k_act_count(uint32_t nn, const uint4* __restrict__ conn,
+                            const uint32_t* __restrict__ inc_ptr,
+                            const uint32_t* __restrict__ inc_e, uint32_t* cnt,
+                            unsigned* max_act) {
+    const int lane = threadIdx.x & 31;
+    for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; n < nn;
+         n += (gridDim.x * blockDim.x) >> 5) {
+        const uint32_t b = inc_ptr[n], m = inc_ptr[n + 1] - b;
+        const bool act = lane < (int)m && !(conn[inc_e[b + lane]].x & 0x80000000u);
+        const unsigned c = __popc(__ballot_sync(kFull, act));
+        if (lane == 0) {
+            cnt[n] = c;
+            atomicMax(max_act, c);
+        }
+    }
+}
+
+// node-pass scatter structure of the assembly (MeshDev): per active
+// incidence the tet and the owner's local index (its first occurrence) and
+// the 4 vertex positions in the owner's list, per neighbour entry the
+// owner's active tets holding that edge
 __global__ void __launch_bounds__(kSetupWarps * 32)
     k_scatter_struct(uint32_t nn, const uint4* __restrict__ conn,
                      const uint32_t* __restrict__ inc_ptr, const uint32_t* __restrict__ inc_e,
                      const uint32_t* __restrict__ nbr_ptr, const uint32_t* __restrict__ nbr,
-                     uint32_t* inc_pos, uint32_t* members) {
+                     const uint32_t* __restrict__ act_ptr, uint32_t* act_v, uint32_t* act_pos,
+                     uint32_t* members) {
     __shared__ uint32_t list_s[kSetupWarps][32];
     __shared__ unsigned memb_s[kSetupWarps][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (uint32_t n = blockIdx.x * kSetupWarps + w; n < nn; n += gridDim.x * kSetupWarps) {
         const uint32_t b = nbr_ptr[n], deg = nbr_ptr[n + 1] - b;
-        const uint32_t ib = inc_ptr[n], mi = inc_ptr[n + 1] - ib;
+        const uint32_t ib = inc_ptr[n], mi = inc_ptr[n + 1] - ib, ab = act_ptr[n];
         if (lane < (int)deg) list_s[w][lane] = nbr[b + lane];
         memb_s[w][lane] = 0u;
         __syncwarp();
+        uint32_t e = 0;
+        uint4 c = make_uint4(0x80000000u, 0, 0, 0);
         if (lane < (int)mi) {
-            const uint32_t e = inc_e[ib + lane];
-            const uint4 c = conn[e];
-            const bool skip = (c.x & 0x80000000u) != 0;
-            uint32_t pk = 0;
+            e = inc_e[ib + lane];
+            c = conn[e];
+        }
+        const bool act = !(c.x & 0x80000000u);
+        const unsigned all = __ballot_sync(kFull, act);
+        if (act) {
+            const int l = __popc(all & ((1u << lane) - 1u));  // position among the active
+            uint32_t pk = 0, own = 0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (int q = 3; q >= 0; --q) {
                 const uint32_t v = vtx(c, q);
-                const uint32_t p = pos_in(list_s[w], deg, v);
+                uint32_t p = pos_in(list_s[w], deg, v);
+                for (int r = 0; r < q; ++r)
+                    if (vtx(c, r) == v) p = 0xffu;  // repeats an earlier vertex
                 pk |= p << (8 * q);
-                if (p != 0xffu && v != n && !skip) atomicOr(&memb_s[w][p], 1u << lane);
+                if (v == n) own = (uint32_t)q;
+                else if (p != 0xffu) atomicOr(&memb_s[w][p], 1u << l);
             }
-            inc_pos[ib + lane] = pk;
+            act_v[ab + l] = 4 * e + own;
+            act_pos[ab + l] = pk;
         }
         __syncwarp();
         if (lane < (int)deg) members[b + lane] = memb_s[w][lane];
@@ -306,7 +336,7 @@ cudaError_t build_mesh_device(uint32_t nn, uint32_t ne, const uint4* conn, MeshS
                               MeshSetupHost& h, unsigned* status, int* result, cudaStream_t s) {
     *result = kSetupOk;
     DevBuf<uint32_t> cnt, depth;
-    DevBuf<unsigned> scal;  // max_inc, max_deg, ticket
+    DevBuf<unsigned> scal;  // max_inc, max_deg, ticket, max_act
     DevBuf<unsigned char> tmp;
     DevBuf<unsigned long long> keys, keys_sorted;
     SCK(cnt.reserve((size_t)nn + 1));
@@ -415,11 +445,18 @@ cudaError_t build_mesh_device(uint32_t nn, uint32_t ne, const uint4* conn, MeshS
     SCK(d.emap->reserve(std::max<uint32_t>(n_emap, 1)));
     k_emap_fill<<<blocks_for(nn, kSetupWarps), kSetupWarps * 32, 0, s>>>(
         nn, d.nbr_ptr->p, d.nbr->p, d.self_pos->p, d.emap_ptr->p, d.emap->p);
-    SCK(d.inc_pos->reserve(std::max<size_t>(1, 4 * (size_t)ne)));
+    SCK(cudaMemsetAsync(scal.p + 3, 0, sizeof(unsigned), s));
+    k_act_count<<<blocks_for((size_t)nn * 32, 256), 256, 0, s>>>(nn, conn, d.inc_ptr->p,
+                                                               d.inc_e->p, cnt.p, scal.p + 3);
+    SCK(d.act_ptr->reserve((size_t)nn + 1));
+    SCK(exclusive_scan(cnt.p, d.act_ptr->p, nn, tmp, s));
+    SCK(d.act_v->reserve(std::max<size_t>(1, 4 * (size_t)ne)));
+    SCK(d.act_pos->reserve(std::max<size_t>(1, 4 * (size_t)ne)));
     SCK(d.nbr_members->reserve(std::max<uint32_t>(total, 1)));
     k_scatter_struct<<<blocks_for(nn, kSetupWarps), kSetupWarps * 32, 0, s>>>(
-        nn, conn, d.inc_ptr->p, d.inc_e->p, d.nbr_ptr->p, d.nbr->p, d.inc_pos->p,
-        d.nbr_members->p);
+        nn, conn, d.inc_ptr->p, d.inc_e->p, d.nbr_ptr->p, d.nbr->p, d.act_ptr->p, d.act_v->p,
+        d.act_pos->p, d.nbr_members->p);
+    SCK(cudaMemcpyAsync(hs, scal.p, sizeof hs, cudaMemcpyDeviceToHost, s));
     SCK(cudaGetLastError());
 
     // host copies of the graph
@@ -428,6 +465,7 @@ cudaError_t build_mesh_device(uint32_t nn, uint32_t ne, const uint4* conn, MeshS
     SCK(down(h.graph.nbr, d.nbr->p, total, s));
     SCK(down(h.graph.self, d.self_pos->p, nn, s));
     SCK(cudaStreamSynchronize(s));
+    h.max_act = hs[3];
     return cudaSuccess;
 }
 

@@ -14,7 +14,8 @@
 //               order (a node waits only on nodes with earlier tickets), and
 //               the level lists as a stable sort of the nodes by depth;
 //   ILU maps    fm_setup.hpp ilu_edge_maps; assembly scatter structures
-//               (vertex positions per incidence, tet bitmask per edge).
+//               (active tets and vertex positions per node, tet bitmask per
+//               edge).
 // Every output equals the host construction in fm_setup.cpp entry for entry.
 #pragma once
 
@@ -39,14 +40,16 @@ struct MeshSetupDev {
     DevBuf<uint4>* node_bwd_rec;
     DevBuf<uint32_t>* emap_ptr;     // n_nodes + 1
     DevBuf<uint8_t>* emap;
-    DevBuf<uint32_t>* inc_pos;      // 4 x u8 per incidence
+    DevBuf<uint32_t>* act_ptr;      // n_nodes + 1: active incidences (MeshDev)
+    DevBuf<uint32_t>* act_v;
+    DevBuf<uint32_t>* act_pos;      // 4 x u8 per active incidence
     DevBuf<uint32_t>* nbr_members;  // tet bitmask per neighbour entry
 };
 
 // host copies that host-side planning and the exports use
 struct MeshSetupHost {
     NodeGraph graph;
-    uint32_t max_inc = 0;
+    uint32_t max_inc = 0, max_act = 0;  // most incident / active tets of a node
     std::vector<uint32_t> lp, lo, up, uo;  // node levels: (ptr, order) forward, backward
 };
 
