@@ -335,10 +335,15 @@ class Context:
         t = self.torch
         return t.zeros(n, dtype=dtype or t.float64, device=f"cuda:{self.device}")
 
+    def _empty(self, n, dtype=None):
+        """an output buffer that the call writes in full"""
+        t = self.torch
+        return t.empty(n, dtype=dtype or t.float64, device=f"cuda:{self.device}")
+
     def elements(self, x, u, E, nu):
         n = x.shape[0]
-        K = self._zeros(144 * n)
-        f = self._zeros(12 * n)
+        K = self._empty(144 * n)
+        f = self._empty(12 * n)
         self._check(lib().fm_elements(self._h, n, _dp(x), _dp(u), _dp(E), nu, _dp(K), _dp(f)),
                     "fm_elements")
         return K.view(n, 144), f.view(n, 12)
