@@ -13,6 +13,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "fm_api.h"
@@ -114,6 +115,12 @@ struct fm_ctx {
     unsigned epoch = 0;
     DevBuf<fm::DevScalars> sc;
     fm::DevScalars* h_sc = nullptr;  // pinned mirror
+    // PCG reports: pinned, written by the device (d_rep: its address there);
+    // two iterations are in flight at most, each with its own slot
+    static constexpr unsigned kReports = 4;
+    fm::PcgReport* h_rep = nullptr;
+    fm::PcgReport* d_rep = nullptr;
+    unsigned rep_seq = 0;
     DevBuf<double> partials;
     DevBuf<double> vec_a, vec_b, vec_c, vec_d, vec_e;  // FP64 scratch (R, du, trial/f, v, host u)
     int grid_trsv64 = 0, grid_trsv32 = 0;
@@ -399,7 +406,7 @@ static std::vector<uint4> node_records(const fm::NodeGraph& g, const std::vector
 // 0.436 against 0.450 ms per FP32 pair, 0.616 against 0.708 FP64, at 64^3).
 // The default path; FM_TRSV_PATH=pipe selects the grid-wide pipelined solves
 // (fm_trsv.cu) instead.  FM_TRSV_PUSH_WARPS caps the warps per CTA (default:
-// 32 in FP32, 16 in FP64), FM_TRSV_PUSH_BLOCK sets the interleave block
+// 32 in FP32, 16 in FP64; smaller meshes take fewer), FM_TRSV_PUSH_BLOCK sets the interleave block
 // (default: chosen by the plan), FM_TRSV_PUSH_CLUSTER the cluster size.
 fm_status setup_push_solves(fm_ctx* c, const std::vector<uint32_t>& lp,
                             const std::vector<uint32_t>& lo, const std::vector<uint32_t>& up,
@@ -414,29 +421,57 @@ fm_status setup_push_solves(fm_ctx* c, const std::vector<uint32_t>& lp,
         const char* v = getenv(name);
         return v ? std::min(hi, std::max(lo_, atoi(v))) : dflt;
     };
-    const int warps32 = env("FM_TRSV_PUSH_WARPS", fm::push_max_warps(4), 1, fm::push_max_warps(4));
-    const int warps64 = std::min(warps32, fm::push_max_warps(8));
+    const int cap32 = env("FM_TRSV_PUSH_WARPS", fm::push_max_warps(4), 1, fm::push_max_warps(4));
+    const int cap64 = std::min(cap32, fm::push_max_warps(8));
     const uint32_t block = (uint32_t)env("FM_TRSV_PUSH_BLOCK", 0, 0, 1 << 20);
     // candidate cluster sizes, most resident CTAs first
     std::vector<std::pair<int, uint32_t>> sizes;  // (resident clusters, size)
     const int forced = env("FM_TRSV_PUSH_CLUSTER", 0, 0, (int)fm::kPushMax);
     for (uint32_t cs = 8; cs <= fm::kPushMax; ++cs) {
         if (forced && cs != (uint32_t)forced) continue;
-        const int ncl = std::min(fm::push_max_clusters(4, (int)cs, warps32, kMaxSmem),
-                                 fm::push_max_clusters(8, (int)cs, warps64, kMaxSmem));
+        const int ncl = std::min(fm::push_max_clusters(4, (int)cs, cap32, kMaxSmem),
+                                 fm::push_max_clusters(8, (int)cs, cap64, kMaxSmem));
         if (ncl > 0) sizes.push_back({ncl, cs});
     }
     std::stable_sort(sizes.begin(), sizes.end(), [](const auto& a, const auto& b) {
         return a.first * a.second > b.first * b.second;
     });
+    // Warps and clusters for the mesh's size.  A warp holds two nodes, and
+    // about 14 nodes in flight per node of an average level keep the front
+    // fed (later levels' loads overlap its hops); every further warp only
+    // polls, and every further cluster is one more slab boundary, crossed
+    // through L2.  Small meshes therefore take clusters of at most 16 warps
+    // per CTA, as many as that needs, large ones all clusters and up to 32
+    // warps (FP32; FP64's double-buffered loop 10 or 16).  Per FP32 / FP64 pair
+    // against all clusters with 32 / 16 warps: 8^3 62 -> 45 / 69 -> 52 us, 16^3
+    // 110 -> 83 / 119 -> 102 us, 32^3 201 -> 178 / 220 -> 215 us, 48^3 307 -> 292
+    // us / unchanged; 64^3 takes them all.
+    const uint32_t levels = std::max<uint32_t>(1, (uint32_t)std::max(lp.size(), up.size()) - 1);
+    const uint32_t want = std::max(1u, (7 * c->nn + levels - 1) / levels);  // warps
     fm::PushPlan p;
     bool planned = false;
+    int warps32 = cap32, warps64 = cap64;
+    auto plan = [&](uint32_t ncl, uint32_t cs) {
+        return fm::push_plan(c->graph, lp, lo, up, uo, ncl, cs, block,
+                             (uint32_t)(kMaxSmem / fm::push_smem_bytes(1, 8)), p) ||
+               fm::push_plan(c->graph, lp, lo, up, uo, ncl, cs, block,
+                             (uint32_t)(kMaxSmem / fm::push_smem_bytes(1, 4)), p);
+    };
     for (const auto& sz : sizes) {
-        planned = fm::push_plan(c->graph, lp, lo, up, uo, (uint32_t)sz.first, sz.second, block,
-                                (uint32_t)(kMaxSmem / fm::push_smem_bytes(1, 8)), p) ||
-                  fm::push_plan(c->graph, lp, lo, up, uo, (uint32_t)sz.first, sz.second, block,
-                                (uint32_t)(kMaxSmem / fm::push_smem_bytes(1, 4)), p);
-        if (planned) break;
+        const uint32_t cs = sz.second, all = (uint32_t)sz.first;
+        const uint32_t few = std::min(all, (want + 16 * cs - 1) / (16 * cs));
+        // fewer clusters only where FP64 slots fit as well
+        planned = few < all &&
+                  fm::push_plan(c->graph, lp, lo, up, uo, few, cs, block,
+                                (uint32_t)(kMaxSmem / fm::push_smem_bytes(1, 8)), p);
+        uint32_t ncl = few;
+        if (!planned) planned = plan(ncl = all, cs);
+        if (planned) {
+            const uint32_t per = (want + ncl * cs - 1) / (ncl * cs);
+            warps32 = std::min(cap32, (int)std::max(8u, (per + 3) & ~3u));
+            warps64 = std::min(cap64, warps32 <= 16 ? 10 : 16);
+            break;
+        }
     }
     if (!planned) return FM_OK;
     auto fits = [&](size_t vb) {
@@ -481,20 +516,22 @@ fm_status setup_push_solves(fm_ctx* c, const std::vector<uint32_t>& lp,
 
 // z = U^-1 L^-1 r on the node-block factors (tmp: the intermediate): the
 // slab-partitioned push solves where the context has a plan for this value
-// width, else the grid-wide pipelined ones.  Returns the kernels launched.
+// width, else the grid-wide pipelined ones.  filled: tmp holds the wait
+// sentinel.  Returns the kernels launched.
 template <typename T>
 int precond_nodes(fm_ctx* c, const T* lu, const T* dinv, const T* r, T* tmp, T* z,
-                  unsigned* status) {
+                  unsigned* status, const unsigned* skip = nullptr, bool filled = false) {
     const bool pu = sizeof(T) == 4 ? c->pu_ok32 : c->pu_ok64;
     if (pu && c->nn) {
-        const cudaError_t e =
-            fm::launch_trsv_push<T>(c->pu, node_sched(c), lu, dinv, r, tmp, z, status, c->stream);
-        if (e == cudaSuccess) return z != r ? 3 : 4;
+        const cudaError_t e = fm::launch_trsv_push<T>(c->pu, node_sched(c), lu, dinv, r, tmp, z,
+                                                      status, c->stream, skip, filled);
+        if (e == cudaSuccess) return (z != r ? 3 : 4) - (filled ? 1 : 0);
         // a launch the device refuses: the pipelined solves from now on
         cudaGetLastError();
         c->pu_ok32 = c->pu_ok64 = false;
     }
-    fm::launch_trsv_nodes<T>(node_sched(c), lu, dinv, r, tmp, z, status, c->device, c->stream);
+    fm::launch_trsv_nodes<T>(node_sched(c), lu, dinv, r, tmp, z, status, c->device, c->stream,
+                             skip);
     return 4;
 }
 
@@ -510,66 +547,122 @@ struct Op {
     T* tmp;
     int grid_trsv;
     const T* dinv = nullptr;  // reciprocal pivots (node-block path)
-    void spmv(const T* x, T* y, double* dot) const {
+    // the intermediate that a PCG vector kernel fills with the wait sentinel
+    // just before an apply (the push solves need it; the others fill or flag
+    // their own)
+    T* prefill() const {
+        return node_block && (sizeof(T) == 4 ? c->pu_ok32 : c->pu_ok64) ? tmp : nullptr;
+    }
+    void spmv(const T* x, T* y, double* dot, const unsigned* skip = nullptr) const {
         PROF(FM_PROF_SPMV, 1);
         T* part = reinterpret_cast<T*>(c->partials.p);
         if (node_block)
             fm::launch_spmv_nodes<T>(c->nn, c->nbr_ptr.p, c->nbr.p, K, x, y, part, c->counter(),
-                                     dot, c->stream);
+                                     dot, c->stream, skip);
         else
             fm::launch_spmv_csr<T>(S->n, S->rp.p, S->ci.p, K, x, y, part, c->counter(), dot,
-                                   c->stream);
+                                   c->stream, skip);
     }
-    void precond(const T* r, T* z) const {
+    void precond(const T* r, T* z, const unsigned* skip = nullptr, bool filled = false) const {
         const bool pu = node_block && (sizeof(T) == 4 ? c->pu_ok32 : c->pu_ok64);
-        PROF(FM_PROF_TRSV, pu ? (r != z ? 3 : 4) : node_block ? 4 : 2);
+        PROF(FM_PROF_TRSV, pu ? (r != z ? 3 : 4) - (filled ? 1 : 0) : node_block ? 4 : 2);
         if (node_block) {
-            precond_nodes<T>(c, LU, dinv, r, tmp, z, c->status());
+            precond_nodes<T>(c, LU, dinv, r, tmp, z, c->status(), skip, filled);
             return;
         }
         const fm::CsrDev v = S->view();
         fm::launch_trsv_lower_csr<T>(v, LU, r, tmp, c->done.p, next_epoch(c), c->status(),
-                                     grid_trsv, c->stream);
+                                     grid_trsv, c->stream, skip);
         fm::launch_trsv_upper_csr<T>(v, LU, diag, tmp, z, c->done.p, next_epoch(c), c->status(),
-                                     grid_trsv, c->stream);
+                                     grid_trsv, c->stream, skip);
     }
 };
 
+// Waits for report seq (in its slot of the ring).  The kernel that writes it
+// is queued; should the stream end without it (a launch that failed), the
+// stream's error is returned.
+fm_status wait_report(fm_ctx* c, unsigned seq, fm::PcgReport* out) {
+    const volatile fm::PcgReport* r = c->h_rep + seq % fm_ctx::kReports;
+    for (unsigned spin = 1; __atomic_load_n(&r->seq, __ATOMIC_ACQUIRE) != seq; ++spin) {
+        if (spin % 1024 == 0) {
+            const cudaError_t e = cudaStreamQuery(c->stream);
+            if (e == cudaSuccess) {
+                if (__atomic_load_n(&r->seq, __ATOMIC_ACQUIRE) == seq) break;
+                return fail(c, FM_ERR_CUDA, "pcg: a queued iteration did not run");
+            }
+            if (e != cudaErrorNotReady) CK(e);
+            std::this_thread::yield();
+        }
+    }
+    out->rr = r->rr;
+    out->relres = r->relres;
+    out->status = r->status;
+    out->stop = r->stop;
+    out->done = r->done;
+    return FM_OK;
+}
+
 // PCG-ILU(0) with the reference's stop tests (FEM/adaptive_fem_engine.hpp:1292-1340).
-// b, x: length-n device vectors of type T; x in/out.
+// b, x: length-n device vectors of type T; x in/out (zero_x: x is zero on
+// entry, so that r = b without a product).
+//
+// The stop tests run on the device (sc->done), and each iteration reports to
+// pinned host memory; the host queues iteration k + 1 before it looks at the
+// report of iteration k.  The GPU never waits for the host between
+// iterations (it idled 15-20 us per iteration with a copy and a stream
+// synchronization in each: 104 us of an 8^3 FP64 iteration, 459 us at 48^3);
+// the iteration that turns out to be one too many consists of kernels that
+// return at once.
 template <typename T>
 fm_status pcg_core(fm_ctx* c, const Op<T>& A, uint32_t n, const T* b, T* x, double tol,
-                   int max_iter, int* iters_out, double* relres_out) {
+                   int max_iter, int* iters_out, double* relres_out, bool zero_x = false) {
     Work<T>& w = work<T>(c);
     T* part = reinterpret_cast<T*>(c->partials.p);
     fm::DevScalars* sc = c->sc.p;
-    CK(cudaMemsetAsync(&sc->stop, 0, sizeof(unsigned), c->stream));
+    const unsigned* done = &sc->done;
+    const unsigned seq0 = c->rep_seq + 1;  // report of step k: seq0 + k (0: the entry)
+    auto slot = [&](int k) { return c->d_rep + (seq0 + (unsigned)k) % fm_ctx::kReports; };
     // r = b - A x
-    A.spmv(x, w.r.p, nullptr);
-    { PROF(FM_PROF_VECTOR, 1); fm::launch_residual_init<T>(n, b, w.r.p, part, c->counter(), &sc->rr, c->stream); }
-    TRY(sync_scalars(c));
-    TRY(check_flags(c, c->h_sc->status, "pcg"));
+    if (!zero_x) A.spmv(x, w.r.p, nullptr);
+    T* tmp = A.prefill();
+    { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_init<T>(n, b, w.r.p, zero_x, tmp, tol, part, c->counter(), sc, slot(0), seq0, c->stream); }
+    A.precond(w.r.p, w.z.p, done, tmp != nullptr);
+    { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_start<T>(n, w.r.p, w.z.p, b, w.p.p, part, c->counter(), sc, c->stream); }
+    c->rep_seq = seq0;
+    auto iteration = [&](int k) {
+        c->rep_seq = seq0 + (unsigned)k;
+        if (k > 1) { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_update_p<T>(n, w.z.p, w.p.p, sc, c->stream); }
+        A.spmv(w.p.p, w.Ap.p, &sc->pAp, done);
+        T* t = A.prefill();
+        { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_update_xr<T>(n, w.p.p, w.Ap.p, x, w.r.p, t, sc, c->stream); }
+        A.precond(w.r.p, w.z.p, done, t != nullptr);
+        { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_rz<T>(n, w.r.p, w.z.p, tol, part, c->counter(), sc, slot(k), seq0 + (unsigned)k, c->stream); }
+    };
     int iters = max_iter;
     double relres = 0.0;
-    if (std::sqrt(c->h_sc->rr) < tol * 1e-3) {
-        iters = 0;
-    } else {
-        A.precond(w.r.p, w.z.p);
-        { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_start<T>(n, w.r.p, w.z.p, b, w.p.p, part, c->counter(), sc, c->stream); }
-        for (int it = 0; it < max_iter; ++it) {
-            A.spmv(w.p.p, w.Ap.p, &sc->pAp);
-            { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_update_xr<T>(n, w.p.p, w.Ap.p, x, w.r.p, sc, c->stream); }
-            A.precond(w.r.p, w.z.p);
-            { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_rz<T>(n, w.r.p, w.z.p, part, c->counter(), sc, c->stream); }
-            TRY(sync_scalars(c));
-            TRY(check_flags(c, c->h_sc->status, "pcg"));
-            if (c->h_sc->stop) break;  // |p.Ap| < 1e-60
-            relres = c->h_sc->relres;
-            if (relres < tol) {
-                iters = it + 1;
+    for (int k = 0; k <= max_iter; ++k) {
+        if (k < max_iter) iteration(k + 1);
+        fm::PcgReport rep;
+        fm_status st = wait_report(c, seq0 + (unsigned)k, &rep);
+        if (st == FM_OK) st = check_flags(c, rep.status, "pcg");
+        if (st != FM_OK) {
+            cudaStreamSynchronize(c->stream);
+            return st;
+        }
+        c->h_sc->status = rep.status;
+        if (c->prof_on && k % 64 == 63) TRY(sync_scalars(c));  // bounds the pending events
+        if (k == 0) {
+            if (rep.done) {
+                iters = 0;
                 break;
             }
-            { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_update_p<T>(n, w.z.p, w.p.p, sc, c->stream); }
+            continue;
+        }
+        if (rep.stop) break;  // |p.Ap| < 1e-60
+        relres = rep.relres;
+        if (rep.done) {
+            iters = k;
+            break;
         }
     }
     if (iters_out) *iters_out = iters;
@@ -705,10 +798,20 @@ fm_status fm_create(fm_ctx** out, int device, void* stream) {
         c->own_stream = true;
     }
     if (c->sc.reserve(1) != cudaSuccess || c->partials.reserve(8192) != cudaSuccess ||
-        cudaMallocHost(&c->h_sc, sizeof(fm::DevScalars)) != cudaSuccess) {
+        cudaMallocHost(&c->h_sc, sizeof(fm::DevScalars) +
+                                     fm_ctx::kReports * sizeof(fm::PcgReport)) != cudaSuccess) {
         fm_destroy(c);
         return FM_ERR_OOM;
     }
+    static_assert(sizeof(fm::DevScalars) % alignof(fm::PcgReport) == 0, "");
+    c->h_rep = reinterpret_cast<fm::PcgReport*>(c->h_sc + 1);
+    std::memset(c->h_rep, 0, fm_ctx::kReports * sizeof(fm::PcgReport));
+    void* dp = nullptr;
+    if (cudaHostGetDevicePointer(&dp, c->h_rep, 0) != cudaSuccess) {
+        fm_destroy(c);
+        return FM_ERR_CUDA;
+    }
+    c->d_rep = static_cast<fm::PcgReport*>(dp);
     cudaMemsetAsync(c->sc.p, 0, sizeof(fm::DevScalars), c->stream);
     cudaMemsetAsync(c->partials.p, 0, c->partials.n * sizeof(double), c->stream);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
@@ -1195,7 +1298,9 @@ fm_status fm_pcg(fm_ctx* c, const double* b, double* x, double tol, int max_iter
         if (!c->w64.factor_valid) return fail(c, FM_ERR_ARG, "call fm_ilu0(FM_FP64) first");
         Op<double> A{c, &c->fem, true, c->w64.K.p, c->w64.LU.p, c->w64.diag.p, c->w64.t.p,
                      c->grid_trsv64, c->w64.dinv.p};
-        return pcg_core<double>(c, A, c->n, b, x, tol, max_iter, iters, relres);
+        TRY(pcg_core<double>(c, A, c->n, b, x, tol, max_iter, iters, relres));
+        CK(cudaStreamSynchronize(c->stream));
+        return FM_OK;
     }
     if (prec != FM_MIXED) return fail(c, FM_ERR_ARG, "unknown precision");
     if (!c->w32.factor_valid) return fail(c, FM_ERR_ARG, "call fm_ilu0(FM_MIXED) first");
@@ -1211,9 +1316,10 @@ fm_status fm_pcg(fm_ctx* c, const double* b, double* x, double tol, int max_iter
     { PROF(FM_PROF_VECTOR, 1); fm::launch_to_f32_scaled(c->n, b, 1.0 / s, c->w32.b.p, c->w32.x.p, c->stream); }
     Op<float> A{c, &c->fem, true, c->w32.K.p, c->w32.LU.p, c->w32.diag.p, c->w32.t.p,
                 c->grid_trsv32, c->w32.dinv.p};
-    TRY(pcg_core<float>(c, A, c->n, c->w32.b.p, c->w32.x.p, tol, max_iter, iters, relres));
+    TRY(pcg_core<float>(c, A, c->n, c->w32.b.p, c->w32.x.p, tol, max_iter, iters, relres, true));
     { PROF(FM_PROF_VECTOR, 1); fm::launch_axpy_u_f32(c->n, c->w32.x.p, s, x, c->stream); }
     CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(c->stream));
     return FM_OK;
 }
 
@@ -1353,7 +1459,7 @@ fm_status fm_newton_step_cfg(fm_ctx* c, double* u, double load_frac, const fm_ne
             Op<float> A{c, &c->fem, true, c->w32.K.p, c->w32.LU.p, c->w32.diag.p, c->w32.t.p,
                         c->grid_trsv32, c->w32.dinv.p};
             TRY(pcg_core<float>(c, A, c->n, c->w32.b.p, c->w32.x.p, itol, g->max_pcg, its,
-                                nullptr));
+                                nullptr, !guess));
             if (keep) { PROF(FM_PROF_VECTOR, 1); fm::launch_f32_to_f64_scaled(c->n, c->w32.x.p, rnorm, du, c->stream); }
             else { PROF(FM_PROF_VECTOR, 1); fm::launch_axpy_u_f32(c->n, c->w32.x.p, rnorm, u, c->stream); }
             have_prev = newton;
@@ -1362,7 +1468,7 @@ fm_status fm_newton_step_cfg(fm_ctx* c, double* u, double load_frac, const fm_ne
             CK(cudaMemsetAsync(du, 0, sizeof(double) * c->n, c->stream));
             Op<double> A{c, &c->fem, true, c->w64.K.p, c->w64.LU.p, c->w64.diag.p, c->w64.t.p,
                          c->grid_trsv64, c->w64.dinv.p};
-            TRY(pcg_core<double>(c, A, c->n, R, du, itol, g->max_pcg, its, nullptr));
+            TRY(pcg_core<double>(c, A, c->n, R, du, itol, g->max_pcg, its, nullptr, true));
             if (!keep) { PROF(FM_PROF_VECTOR, 1); fm::launch_axpy_u(c->n, du, u, c->stream); }
         }
         CK(cudaGetLastError());
@@ -1502,9 +1608,9 @@ fm_status fm_newton_step_cfg(fm_ctx* c, double* u, double load_frac, const fm_ne
             }
             { PROF(FM_PROF_VECTOR, 1); fm::launch_trial(c->n, u, alpha, du, u, c->stream); }
             c->h_sc->status = status0;
+            // (pinned; the next write to it is a copy on this stream)
             CK(cudaMemcpyAsync(&c->sc.p->status, &c->h_sc->status, sizeof(unsigned),
                                cudaMemcpyHostToDevice, c->stream));
-            TRY(sync_scalars(c));
         }
         CK(cudaGetLastError());
         update_states();
@@ -1798,7 +1904,7 @@ fm_status fm_adjoint(fm_ctx* c, const double* u, const double* dLdu, double* gmu
             Op<float> A{c, &c->fem, true, c->w32.K.p, c->w32.LU.p, c->w32.diag.p, c->w32.t.p,
                         c->grid_trsv32, c->w32.dinv.p};
             TRY(pcg_core<float>(c, A, c->n, c->w32.b.p, c->w32.x.p, inner_tol, 100000, &its,
-                                nullptr));
+                                nullptr, true));
             {
                 PROF(FM_PROF_VECTOR, 1);
                 fm::launch_f32_to_f64_scaled(c->n, c->w32.x.p, rn, dw, c->stream);
@@ -1807,7 +1913,7 @@ fm_status fm_adjoint(fm_ctx* c, const double* u, const double* dLdu, double* gmu
             CK(cudaMemsetAsync(dw, 0, sizeof(double) * c->n, c->stream));
             Op<double> A{c, &c->fem, true, c->w64.K.p, c->w64.LU.p, c->w64.diag.p, c->w64.t.p,
                          c->grid_trsv64, c->w64.dinv.p};
-            TRY(pcg_core<double>(c, A, c->n, r, dw, inner_tol, 100000, &its, nullptr));
+            TRY(pcg_core<double>(c, A, c->n, r, dw, inner_tol, 100000, &its, nullptr, true));
         }
         pcg_total += its;
         {

@@ -36,6 +36,7 @@ struct DevScalars {
     double scale;    // rhs scaling for the FP32 inner solve
     double guess_xb, guess_xkx;  // x_prev . b and x_prev . K x_prev (initial guess)
     unsigned stop;   // 1: |pAp| < 1e-60 breakdown
+    unsigned done;   // 1: the running PCG has ended; kernels of later iterations return at once
     unsigned status; // FM_FLAG_* bits
     unsigned wait_budget;  // bounded-wait limit in 1024 cycles (0: kWaitCycles); follows status
     unsigned counter[8];  // last-block counters (one per reduction site)
@@ -44,6 +45,22 @@ struct DevScalars {
 };
 
 constexpr int kRedBlocks = 296;  // 2 x 148 SMs: fixed grid => fixed summation order
+// blocks of 256 of a reduction over n values: a small vector does not pay for
+// idle blocks and their turns at the arrival counter (a function of n alone:
+// the summation order stays fixed)
+inline int red_blocks(uint32_t n) {
+    const uint32_t b = (n + 255) / 256;
+    return b < 1 ? 1 : b < (uint32_t)kRedBlocks ? (int)b : kRedBlocks;
+}
+
+// What the host needs to know of a PCG step, written by the step's last
+// kernel straight into pinned host memory: the host reads it without a copy
+// or a stream synchronization, while the next iteration is already queued.
+struct PcgReport {
+    double rr, relres;
+    unsigned status, stop, done;
+    unsigned seq;  // written last
+};
 
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
@@ -66,6 +83,21 @@ __device__ __forceinline__ unsigned ld_volatile_u32(const unsigned* p) {
 // L2-coherent loads of values produced by other SMs during the same kernel
 __device__ __forceinline__ double ld_cg(const double* p) { return __ldcg(p); }
 __device__ __forceinline__ float ld_cg(const float* p) { return __ldcg(p); }
+
+// *skip set (null: never): the kernel has nothing to do
+__device__ __forceinline__ bool skipped(const unsigned* skip) {
+    return skip && ld_volatile_u32(skip) != 0u;
+}
+__device__ __forceinline__ void pcg_report(PcgReport* rep, unsigned seq, const DevScalars* sc) {
+    volatile PcgReport* r = rep;
+    r->rr = sc->rr;
+    r->relres = sc->relres;
+    r->status = ld_volatile_u32(&sc->status);
+    r->stop = sc->stop;
+    r->done = sc->done;
+    __threadfence_system();
+    r->seq = seq;
+}
 
 __device__ __forceinline__ void raise_flag(unsigned* status, unsigned bits) {
     atomicOr(status, bits);

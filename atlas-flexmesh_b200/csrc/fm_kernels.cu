@@ -16,6 +16,7 @@
 #include <cstdio>
 
 #include "fm_kernels.hpp"
+#include "fm_sync.cuh"
 
 namespace fm {
 
@@ -597,7 +598,8 @@ __global__ void __launch_bounds__(256)
     k_spmv_nodes(uint32_t nn, const uint32_t* __restrict__ nbr_ptr,
                  const uint32_t* __restrict__ nbr, const T* __restrict__ val,
                  const T* __restrict__ x, T* __restrict__ y, T* partials, unsigned* counter,
-                 double* dot) {
+                 double* dot, const unsigned* __restrict__ skip) {
+    if (skipped(skip)) return;
     const int lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -637,16 +639,19 @@ __global__ void __launch_bounds__(256)
 template <typename T>
 void launch_spmv_nodes(uint32_t n_nodes, const uint32_t* nbr_ptr, const uint32_t* nbr,
                        const T* val, const T* x, T* y, T* partials, unsigned* counter,
-                       double* dot, cudaStream_t s) {
-    k_spmv_nodes<T><<<kSpmvBlocks, 256, 0, s>>>(n_nodes, nbr_ptr, nbr, val, x, y, partials,
-                                                 counter, dot);
+                       double* dot, cudaStream_t s, const unsigned* skip) {
+    // no blocks without a node: each would still take its turn at the counter
+    const int grid = (int)std::min<uint32_t>(kSpmvBlocks, std::max(1u, (n_nodes + 7) / 8));
+    k_spmv_nodes<T><<<grid, 256, 0, s>>>(n_nodes, nbr_ptr, nbr, val, x, y, partials, counter, dot,
+                                         skip);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256)
     k_spmv_csr(uint32_t n, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
                const T* __restrict__ val, const T* __restrict__ x, T* __restrict__ y,
-               T* partials, unsigned* counter, double* dot) {
+               T* partials, unsigned* counter, double* dot, const unsigned* __restrict__ skip) {
+    if (skipped(skip)) return;
     const int lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -669,8 +674,10 @@ __global__ void __launch_bounds__(256)
 
 template <typename T>
 void launch_spmv_csr(uint32_t n, const uint32_t* rp, const uint32_t* ci, const T* val, const T* x,
-                     T* y, T* partials, unsigned* counter, double* dot, cudaStream_t s) {
-    k_spmv_csr<T><<<kSpmvBlocks, 256, 0, s>>>(n, rp, ci, val, x, y, partials, counter, dot);
+                     T* y, T* partials, unsigned* counter, double* dot, cudaStream_t s,
+                     const unsigned* skip) {
+    const int grid = (int)std::min<uint32_t>(kSpmvBlocks, std::max(1u, (n + 7) / 8));
+    k_spmv_csr<T><<<grid, 256, 0, s>>>(n, rp, ci, val, x, y, partials, counter, dot, skip);
 }
 
 // ===========================================================================
@@ -769,7 +776,9 @@ __global__ void __launch_bounds__(kSfWarps * 32)
 template <typename T>
 __global__ void __launch_bounds__(kSfWarps * 32)
     k_trsv_lower_csr(CsrDev A, const T* __restrict__ lu, const T* __restrict__ r, T* z,
-                     unsigned* __restrict__ done, unsigned epoch, unsigned* __restrict__ status) {
+                     unsigned* __restrict__ done, unsigned epoch, unsigned* __restrict__ status,
+                     const unsigned* __restrict__ skip) {
+    if (skipped(skip)) return;
     const int lane = threadIdx.x & 31;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t W = (gridDim.x * blockDim.x) >> 5;
@@ -795,7 +804,9 @@ template <typename T>
 __global__ void __launch_bounds__(kSfWarps * 32)
     k_trsv_upper_csr(CsrDev A, const T* __restrict__ lu,
                      const T* __restrict__ diag, const T* __restrict__ z, T* y,
-                     unsigned* __restrict__ done, unsigned epoch, unsigned* __restrict__ status) {
+                     unsigned* __restrict__ done, unsigned epoch, unsigned* __restrict__ status,
+                     const unsigned* __restrict__ skip) {
+    if (skipped(skip)) return;
     const int lane = threadIdx.x & 31;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t W = (gridDim.x * blockDim.x) >> 5;
@@ -831,16 +842,18 @@ void launch_ilu0_csr(const CsrDev& A, const T* a_val, T* lu, T* diag, unsigned* 
 }
 template <typename T>
 void launch_trsv_lower_csr(const CsrDev& A, const T* lu, const T* r, T* z, unsigned* done,
-                           unsigned epoch, unsigned* status, int grid, cudaStream_t s) {
+                           unsigned epoch, unsigned* status, int grid, cudaStream_t s,
+                           const unsigned* skip) {
     if (!A.n) return;
-    k_trsv_lower_csr<T><<<grid, kSfWarps * 32, 0, s>>>(A, lu, r, z, done, epoch, status);
+    k_trsv_lower_csr<T><<<grid, kSfWarps * 32, 0, s>>>(A, lu, r, z, done, epoch, status, skip);
 }
 template <typename T>
 void launch_trsv_upper_csr(const CsrDev& A, const T* lu, const T* diag, const T* z, T* y,
                            unsigned* done, unsigned epoch, unsigned* status, int grid,
-                           cudaStream_t s) {
+                           cudaStream_t s, const unsigned* skip) {
     if (!A.n) return;
-    k_trsv_upper_csr<T><<<grid, kSfWarps * 32, 0, s>>>(A, lu, diag, z, y, done, epoch, status);
+    k_trsv_upper_csr<T><<<grid, kSfWarps * 32, 0, s>>>(A, lu, diag, z, y, done, epoch, status,
+                                                       skip);
 }
 
 // All blocks of a sync-free kernel must be resident at once (rows wait on
@@ -876,6 +889,7 @@ __global__ void __launch_bounds__(kVecThreads)
     k_dot(uint32_t n, const T* __restrict__ x, const T* __restrict__ y, T* partials,
           unsigned* counter, double* out) {
     T s = T(0);
+#pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         s += x[i] * y[i];
     __shared__ T sbuf[32];
@@ -885,28 +899,41 @@ __global__ void __launch_bounds__(kVecThreads)
 template <typename T>
 void launch_dot(uint32_t n, const T* x, const T* y, T* partials, unsigned* counter, double* out,
                 cudaStream_t s) {
-    k_dot<T><<<kRedBlocks, kVecThreads, 0, s>>>(n, x, y, partials, counter, out);
+    k_dot<T><<<red_blocks(n), kVecThreads, 0, s>>>(n, x, y, partials, counter, out);
 }
 
+// PCG entry: r = b - r (zero_x: r = b, the start vector is zero), rr = r.r,
+// the early exit ||r|| < tol 1e-3 as the reference takes it (:1298), and the
+// wait sentinel into tmp (null: none) for the solve that follows.
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
-    k_residual_init(uint32_t n, const T* __restrict__ b, T* __restrict__ r, T* partials,
-                    unsigned* counter, double* rr) {
+    k_pcg_init(uint32_t n, const T* __restrict__ b, T* __restrict__ r, int zero_x,
+               T* __restrict__ tmp, double tol, T* partials, unsigned* counter, DevScalars* sc,
+               PcgReport* rep, unsigned seq) {
     T s = T(0);
+#pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x) {
-        const T v = b[i] - r[i];
+        const T v = zero_x ? b[i] : b[i] - r[i];
         r[i] = v;
+        if (tmp) tmp[i] = Sentinel<T>::value();
         s += v * v;
     }
     __shared__ T sbuf[32];
     const T bt = block_sum(s, sbuf);
-    grid_reduce_finish<T>(bt, partials, counter, [&](T total) { *rr = (double)total; });
+    grid_reduce_finish<T>(bt, partials, counter, [&](T total) {
+        sc->rr = (double)total;
+        sc->stop = 0u;
+        sc->done = sqrt((double)total) < tol * 1e-3 ? 1u : 0u;
+        pcg_report(rep, seq, sc);
+    });
 }
 template <typename T>
-void launch_residual_init(uint32_t n, const T* b, T* r, T* partials, unsigned* counter,
-                          double* rr, cudaStream_t s) {
-    k_residual_init<T><<<kRedBlocks, kVecThreads, 0, s>>>(n, b, r, partials, counter, rr);
+void launch_pcg_init(uint32_t n, const T* b, T* r, bool zero_x, T* tmp, double tol, T* partials,
+                     unsigned* counter, DevScalars* sc, PcgReport* rep, unsigned seq,
+                     cudaStream_t s) {
+    k_pcg_init<T><<<red_blocks(n), kVecThreads, 0, s>>>(n, b, r, zero_x, tmp, tol, partials,
+                                                        counter, sc, rep, seq);
 }
 
 // p = z; rz = r.z; bb = b.b.  Two sums share one pass (partials: 2 slots per block)
@@ -915,7 +942,9 @@ __global__ void __launch_bounds__(kVecThreads)
     k_pcg_start(uint32_t n, const T* __restrict__ r, const T* __restrict__ z,
                 const T* __restrict__ b, T* __restrict__ p, T* partials, unsigned* counter,
                 DevScalars* sc) {
+    if (skipped(&sc->done)) return;
     T s1 = T(0), s2 = T(0);
+#pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x) {
         const T zi = z[i];
@@ -936,39 +965,55 @@ __global__ void __launch_bounds__(kVecThreads)
 template <typename T>
 void launch_pcg_start(uint32_t n, const T* r, const T* z, const T* b, T* p, T* partials,
                       unsigned* counter, DevScalars* sc, cudaStream_t s) {
-    k_pcg_start<T><<<kRedBlocks, kVecThreads, 0, s>>>(n, r, z, b, p, partials, counter, sc);
+    k_pcg_start<T><<<red_blocks(n), kVecThreads, 0, s>>>(n, r, z, b, p, partials, counter, sc);
 }
 
 // alpha = rz/pAp (current rz is rz_new); breakdown |pAp| < 1e-60 stops
-// before touching x and r, as the reference breaks out (:1320).
+// before touching x and r, as the reference breaks out (:1320).  Also writes
+// the wait sentinel into tmp (null: none), the intermediate of the
+// triangular solves that follow.
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
     k_pcg_update_xr(uint32_t n, const T* __restrict__ p, const T* __restrict__ Ap,
-                    T* __restrict__ x, T* __restrict__ r, DevScalars* sc) {
+                    T* __restrict__ x, T* __restrict__ r, T* __restrict__ tmp, DevScalars* sc) {
+    if (skipped(&sc->done)) return;
     const double pAp = sc->pAp;
     if (fabs(pAp) < 1e-60) {
         if (blockIdx.x == 0 && threadIdx.x == 0) sc->stop = 1u;
         return;
     }
     const T alpha = (T)(sc->rz_new / pAp);
+#pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x) {
         x[i] += alpha * p[i];
         r[i] -= alpha * Ap[i];
+        if (tmp) tmp[i] = Sentinel<T>::value();
     }
 }
 template <typename T>
-void launch_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* x, T* r, DevScalars* sc,
+void launch_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* x, T* r, T* tmp, DevScalars* sc,
                           cudaStream_t s) {
-    k_pcg_update_xr<T><<<kRedBlocks * 2, kVecThreads, 0, s>>>(n, p, Ap, x, r, sc);
+    k_pcg_update_xr<T><<<2 * red_blocks(n), kVecThreads, 0, s>>>(n, p, Ap, x, r, tmp, sc);
 }
 
-// rz <- rz_new (old value kept for beta), rz_new <- r.z, relres
+// rz <- rz_new (old value kept for beta), rz_new <- r.z, relres, the stop
+// tests, and the report.  After a breakdown only the report.
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
-    k_pcg_rz(uint32_t n, const T* __restrict__ r, const T* __restrict__ z, T* partials,
-             unsigned* counter, DevScalars* sc) {
+    k_pcg_rz(uint32_t n, const T* __restrict__ r, const T* __restrict__ z, double tol, T* partials,
+             unsigned* counter, DevScalars* sc, PcgReport* rep, unsigned seq) {
+    if (skipped(&sc->done)) return;
+    if (ld_volatile_u32(&sc->stop)) {
+        // the other blocks return here or, once done is set, above
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            sc->done = 1u;
+            pcg_report(rep, seq, sc);
+        }
+        return;
+    }
     T s = T(0);
+#pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x)
         s += r[i] * z[i];
@@ -979,25 +1024,30 @@ __global__ void __launch_bounds__(kVecThreads)
         sc->rz_new = (double)total;
         const double bb = sc->bb > 1e-300 ? sc->bb : 1e-300;
         sc->relres = sqrt((double)total / bb);
+        if (sc->relres < tol) sc->done = 1u;
+        pcg_report(rep, seq, sc);
     });
 }
 template <typename T>
-void launch_pcg_rz(uint32_t n, const T* r, const T* z, T* partials, unsigned* counter,
-                   DevScalars* sc, cudaStream_t s) {
-    k_pcg_rz<T><<<kRedBlocks, kVecThreads, 0, s>>>(n, r, z, partials, counter, sc);
+void launch_pcg_rz(uint32_t n, const T* r, const T* z, double tol, T* partials, unsigned* counter,
+                   DevScalars* sc, PcgReport* rep, unsigned seq, cudaStream_t s) {
+    k_pcg_rz<T><<<red_blocks(n), kVecThreads, 0, s>>>(n, r, z, tol, partials, counter, sc, rep,
+                                                      seq);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
     k_pcg_update_p(uint32_t n, const T* __restrict__ z, T* __restrict__ p, const DevScalars* sc) {
+    if (skipped(&sc->done)) return;
     const T beta = (T)(sc->rz_new / sc->rz);
+#pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x)
         p[i] = z[i] + beta * p[i];
 }
 template <typename T>
 void launch_pcg_update_p(uint32_t n, const T* z, T* p, DevScalars* sc, cudaStream_t s) {
-    k_pcg_update_p<T><<<kRedBlocks * 2, kVecThreads, 0, s>>>(n, z, p, sc);
+    k_pcg_update_p<T><<<2 * red_blocks(n), kVecThreads, 0, s>>>(n, z, p, sc);
 }
 
 __global__ void k_set_bc_values(uint32_t n, const uint8_t* __restrict__ mask,
@@ -1013,7 +1063,7 @@ void launch_set_bc_values(uint32_t n, const uint8_t* mask, const double* val, do
 
 void launch_norm2(uint32_t n, const double* R, double* partials, unsigned* counter, double* out,
                   cudaStream_t s) {
-    k_dot<double><<<kRedBlocks, kVecThreads, 0, s>>>(n, R, R, partials, counter, out);
+    k_dot<double><<<red_blocks(n), kVecThreads, 0, s>>>(n, R, R, partials, counter, out);
 }
 
 __global__ void k_to_f32_scaled(uint32_t n, const double* __restrict__ R, double inv_scale,
@@ -1171,25 +1221,29 @@ template void launch_apply_bc_nodes<float>(uint32_t, const uint32_t*, const uint
                                            const uint8_t*, float*, cudaStream_t);
 #define FM_INST(T)                                                                              \
     template void launch_spmv_nodes<T>(uint32_t, const uint32_t*, const uint32_t*, const T*,    \
-                                       const T*, T*, T*, unsigned*, double*, cudaStream_t);     \
+                                       const T*, T*, T*, unsigned*, double*, cudaStream_t,      \
+                                       const unsigned*);                                        \
     template void launch_spmv_csr<T>(uint32_t, const uint32_t*, const uint32_t*, const T*,      \
-                                     const T*, T*, T*, unsigned*, double*, cudaStream_t);       \
+                                     const T*, T*, T*, unsigned*, double*, cudaStream_t,        \
+                                     const unsigned*);                                          \
     template void launch_ilu0_csr<T>(const CsrDev&, const T*, T*, T*, unsigned*, unsigned,      \
                                      unsigned*, int, cudaStream_t);                             \
     template void launch_trsv_lower_csr<T>(const CsrDev&, const T*, const T*, T*, unsigned*,    \
-                                           unsigned, unsigned*, int, cudaStream_t);             \
+                                           unsigned, unsigned*, int, cudaStream_t,              \
+                                           const unsigned*);                                    \
     template void launch_trsv_upper_csr<T>(const CsrDev&, const T*, const T*, const T*, T*,     \
-                                           unsigned*, unsigned, unsigned*, int, cudaStream_t);  \
+                                           unsigned*, unsigned, unsigned*, int, cudaStream_t,   \
+                                           const unsigned*);                                    \
     template void launch_dot<T>(uint32_t, const T*, const T*, T*, unsigned*, double*,           \
                                 cudaStream_t);                                                  \
-    template void launch_residual_init<T>(uint32_t, const T*, T*, T*, unsigned*, double*,       \
-                                          cudaStream_t);                                        \
+    template void launch_pcg_init<T>(uint32_t, const T*, T*, bool, T*, double, T*, unsigned*,   \
+                                     DevScalars*, PcgReport*, unsigned, cudaStream_t);          \
     template void launch_pcg_start<T>(uint32_t, const T*, const T*, const T*, T*, T*,           \
                                       unsigned*, DevScalars*, cudaStream_t);                    \
-    template void launch_pcg_update_xr<T>(uint32_t, const T*, const T*, T*, T*, DevScalars*,    \
-                                          cudaStream_t);                                        \
-    template void launch_pcg_rz<T>(uint32_t, const T*, const T*, T*, unsigned*, DevScalars*,    \
-                                   cudaStream_t);                                               \
+    template void launch_pcg_update_xr<T>(uint32_t, const T*, const T*, T*, T*, T*,             \
+                                          DevScalars*, cudaStream_t);                           \
+    template void launch_pcg_rz<T>(uint32_t, const T*, const T*, double, T*, unsigned*,         \
+                                   DevScalars*, PcgReport*, unsigned, cudaStream_t);            \
     template void launch_pcg_update_p<T>(uint32_t, const T*, T*, DevScalars*, cudaStream_t);
 FM_INST(double)
 FM_INST(float)

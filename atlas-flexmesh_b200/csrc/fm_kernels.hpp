@@ -63,14 +63,17 @@ void launch_elements(uint32_t n, const double* x, const double* u, const double*
 
 // SpMV on the node-block solve pattern (y = A x); with dot != null also
 // finishes dot(x, y) into *dot through the deterministic grid reduction.
+// skip (here and below; null: never): a device word that, when set, makes the
+// kernel return at once.
 template <typename T>
 void launch_spmv_nodes(uint32_t n_nodes, const uint32_t* nbr_ptr, const uint32_t* nbr,
                        const T* val, const T* x, T* y, T* partials, unsigned* counter,
-                       double* dot, cudaStream_t s);
+                       double* dot, cudaStream_t s, const unsigned* skip = nullptr);
 // Generic scalar CSR SpMV (ascending or any column order)
 template <typename T>
 void launch_spmv_csr(uint32_t n, const uint32_t* rp, const uint32_t* ci, const T* val, const T* x,
-                     T* y, T* partials, unsigned* counter, double* dot, cudaStream_t s);
+                     T* y, T* partials, unsigned* counter, double* dot, cudaStream_t s,
+                     const unsigned* skip = nullptr);
 
 // Sync-free ILU(0) and triangular solves on a CSR with ascending columns.
 // order: a topological order of the rows (dependency levels); done: one
@@ -90,37 +93,40 @@ void launch_ilu0_csr(const CsrDev& A, const T* a_val, T* lu, T* diag, unsigned* 
                      unsigned epoch, unsigned* status, int grid, cudaStream_t s);
 template <typename T>
 void launch_trsv_lower_csr(const CsrDev& A, const T* lu, const T* r, T* z, unsigned* done,
-                           unsigned epoch, unsigned* status, int grid, cudaStream_t s);
+                           unsigned epoch, unsigned* status, int grid, cudaStream_t s,
+                           const unsigned* skip = nullptr);
 template <typename T>
 void launch_trsv_upper_csr(const CsrDev& A, const T* lu, const T* diag, const T* z, T* y,
                            unsigned* done, unsigned epoch, unsigned* status, int grid,
-                           cudaStream_t s);
+                           cudaStream_t s, const unsigned* skip = nullptr);
 // persistent grid sizes (all blocks co-resident) for the sync-free kernels
 int persistent_grid_ilu0_csr(int device, bool fp32, const CsrDev& A);
 int persistent_grid_trsv_csr(int device, bool fp32);
 
-// PCG vector kernels; all reductions deterministic (fixed grid kRedBlocks).
+// PCG vector kernels; all reductions deterministic (the grid depends on n
+// alone).  Once sc->done is set they return at once.
 template <typename T>
 void launch_dot(uint32_t n, const T* x, const T* y, T* partials, unsigned* counter, double* out,
                 cudaStream_t s);
-// r = b - r (r holds A x on entry); *rr = r.r
+// r = b - r (r holds A x on entry; zero_x: r = b), rr = r.r, stop = 0, done =
+// early exit (sqrt(rr) < tol 1e-3); tmp (nullable) = wait sentinel
 template <typename T>
-void launch_residual_init(uint32_t n, const T* b, T* r, T* partials, unsigned* counter,
-                          double* rr, cudaStream_t s);
+void launch_pcg_init(uint32_t n, const T* b, T* r, bool zero_x, T* tmp, double tol, T* partials,
+                     unsigned* counter, DevScalars* sc, PcgReport* rep, unsigned seq,
+                     cudaStream_t s);
 // p = z; rz = r.z; bb = b.b (both into sc)
 template <typename T>
 void launch_pcg_start(uint32_t n, const T* r, const T* z, const T* b, T* p, T* partials,
                       unsigned* counter, DevScalars* sc, cudaStream_t s);
-// alpha = rz/pAp; x += alpha p; r -= alpha Ap
+// alpha = rz/pAp; x += alpha p; r -= alpha Ap; tmp (nullable) = wait sentinel
 template <typename T>
-void launch_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* x, T* r, DevScalars* sc,
+void launch_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* x, T* r, T* tmp, DevScalars* sc,
                           cudaStream_t s);
-// rz_new = r.z; relres = sqrt(rz_new / max(bb,1e-300))
+// rz_new = r.z; relres = sqrt(rz_new / max(bb,1e-300)); done when relres < tol
 template <typename T>
-void launch_pcg_rz(uint32_t n, const T* r, const T* z, T* partials, unsigned* counter,
-                   DevScalars* sc, cudaStream_t s);
-// beta = rz_new/rz; p = z + beta p; rz = rz_new (rotation done by thread 0
-// of the grid after all blocks read rz: see kernel)
+void launch_pcg_rz(uint32_t n, const T* r, const T* z, double tol, T* partials, unsigned* counter,
+                   DevScalars* sc, PcgReport* rep, unsigned seq, cudaStream_t s);
+// beta = rz_new/rz; p = z + beta p
 template <typename T>
 void launch_pcg_update_p(uint32_t n, const T* z, T* p, DevScalars* sc, cudaStream_t s);
 

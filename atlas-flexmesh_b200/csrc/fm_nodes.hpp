@@ -27,10 +27,12 @@ struct NodeSched {
 };
 
 // y = U^-1 L^-1 r using tmp for the intermediate (both overwritten);
-// dinv holds the reciprocal pivots written by the factorization
+// dinv holds the reciprocal pivots written by the factorization; skip (null:
+// never): a device word that, when set, makes the kernels return at once
 template <typename T>
 void launch_trsv_nodes(const NodeSched& S, const T* lu, const T* dinv, const T* r, T* tmp, T* y,
-                       unsigned* status, int device, cudaStream_t s);
+                       unsigned* status, int device, cudaStream_t s,
+                       const unsigned* skip = nullptr);
 // LU (nnz entries, a_ii kept on diagonal slots), pivots d and their
 // reciprocals dinv (three kernels: LU and dinv filled with the wait
 // sentinel, then the factorization)
@@ -67,9 +69,11 @@ size_t push_smem_bytes(uint32_t max_slot, size_t value_bytes);
 int push_max_clusters(size_t value_bytes, int cluster, int warps, size_t smem);
 // y = U^-1 L^-1 r through tmp (three kernels: tmp's sentinel fill, the
 // forward solve, which also fills y unless y aliases r, and the backward);
-// returns the first launch error, with nothing left half-done on success
+// returns the first launch error, with nothing left half-done on success.
+// filled: tmp already holds the sentinel (one kernel less)
 template <typename T>
 cudaError_t launch_trsv_push(const PushSolve& P, const NodeSched& S, const T* lu, const T* dinv,
-                             const T* r, T* tmp, T* y, unsigned* status, cudaStream_t s);
+                             const T* r, T* tmp, T* y, unsigned* status, cudaStream_t s,
+                             const unsigned* skip = nullptr, bool filled = false);
 
 }  // namespace fm

@@ -130,7 +130,9 @@ __device__ __forceinline__ void block_sums(const TrsvPre<T>& P, unsigned* status
 template <typename T>
 __global__ void __launch_bounds__(kTrsvWarps * 32)
     k_trsv_lower_pipe(NodeSched S, const T* __restrict__ lu, const T* __restrict__ r,
-                      T* __restrict__ z, unsigned* __restrict__ status, unsigned backoff) {
+                      T* __restrict__ z, unsigned* __restrict__ status, unsigned backoff,
+                      const unsigned* __restrict__ skip) {
+    if (skipped(skip)) return;
     const int lane = threadIdx.x & 31;
     const uint32_t W = (gridDim.x * blockDim.x) >> 5;
     uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -164,7 +166,8 @@ template <typename T>
 __global__ void __launch_bounds__(kTrsvWarps * 32)
     k_trsv_upper_pipe(NodeSched S, const T* __restrict__ lu, const T* __restrict__ dinv,
                       const T* __restrict__ zin, T* __restrict__ y, unsigned* __restrict__ status,
-                      unsigned backoff) {
+                      unsigned backoff, const unsigned* __restrict__ skip) {
+    if (skipped(skip)) return;
     const int lane = threadIdx.x & 31;
     const uint32_t W = (gridDim.x * blockDim.x) >> 5;
     uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -220,7 +223,7 @@ static int trsv_grid(int resident, uint32_t max_width) {
 
 template <typename T>
 void launch_trsv_nodes(const NodeSched& S, const T* lu, const T* dinv, const T* r, T* tmp, T* y,
-                       unsigned* status, int device, cudaStream_t s) {
+                       unsigned* status, int device, cudaStream_t s, const unsigned* skip) {
     if (!S.n_nodes) return;
     static int res_lo[2] = {0, 0}, res_up[2] = {0, 0};
     const int f = sizeof(T) == 4;
@@ -230,16 +233,17 @@ void launch_trsv_nodes(const NodeSched& S, const T* lu, const T* dinv, const T* 
     const uint32_t n = 3 * S.n_nodes;
     launch_fill_sentinel<T>(n, tmp, s);
     k_trsv_lower_pipe<T><<<trsv_grid(res_lo[f], S.max_width_fwd), kTrsvWarps * 32, 0, s>>>(
-        S, lu, r, tmp, status, backoff);
+        S, lu, r, tmp, status, backoff, skip);
     launch_fill_sentinel<T>(n, y, s);
     k_trsv_upper_pipe<T><<<trsv_grid(res_up[f], S.max_width_bwd), kTrsvWarps * 32, 0, s>>>(
-        S, lu, dinv, tmp, y, status, backoff);
+        S, lu, dinv, tmp, y, status, backoff, skip);
 }
 
 template void launch_trsv_nodes<double>(const NodeSched&, const double*, const double*,
                                         const double*, double*, double*, unsigned*, int,
-                                        cudaStream_t);
+                                        cudaStream_t, const unsigned*);
 template void launch_trsv_nodes<float>(const NodeSched&, const float*, const float*, const float*,
-                                       float*, float*, unsigned*, int, cudaStream_t);
+                                       float*, float*, unsigned*, int, cudaStream_t,
+                                       const unsigned*);
 
 }  // namespace fm

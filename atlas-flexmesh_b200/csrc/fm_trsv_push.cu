@@ -259,7 +259,9 @@ template <typename T, bool Lower>
 __global__ void __launch_bounds__(push_max_warps(sizeof(T)) * 32, 1)
     k_trsv_push(PushSolve P, NodeSched S, const T* __restrict__ lu, const T* __restrict__ dinv,
                 const T* __restrict__ rhs, T* __restrict__ out, T* __restrict__ fill,
-                uint32_t n_fill, unsigned* __restrict__ status) {
+                uint32_t n_fill, unsigned* __restrict__ status,
+                const unsigned* __restrict__ skip) {
+    if (skipped(skip)) return;  // the same answer in every CTA: nothing writes the word meanwhile
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(16) T zero_slot[4];
     T* slots = reinterpret_cast<T*>(smem_raw);
@@ -384,7 +386,7 @@ static int max_clusters(K kernel, int cluster, int warps, size_t smem) {
 template <typename T, bool Lower>
 static cudaError_t launch_dir(const PushSolve& P, const NodeSched& S, const T* lu, const T* dinv,
                               const T* rhs, T* out, T* fill, uint32_t n_fill, unsigned* status,
-                              cudaStream_t s) {
+                              const unsigned* skip, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(P.n_ctas);
     cfg.blockDim = dim3(32 * (sizeof(T) == 4 ? P.warps32 : P.warps64));
@@ -398,7 +400,7 @@ static cudaError_t launch_dir(const PushSolve& P, const NodeSched& S, const T* l
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_trsv_push<T, Lower>, P, S, lu, dinv, rhs, out, fill, n_fill,
-                              status);
+                              status, skip);
 }
 
 }  // namespace
@@ -422,24 +424,26 @@ int push_max_clusters(size_t value_bytes, int cluster, int warps, size_t smem) {
 
 template <typename T>
 cudaError_t launch_trsv_push(const PushSolve& P, const NodeSched& S, const T* lu, const T* dinv,
-                             const T* r, T* tmp, T* y, unsigned* status, cudaStream_t s) {
+                             const T* r, T* tmp, T* y, unsigned* status, cudaStream_t s,
+                             const unsigned* skip, bool filled) {
     if (!S.n_nodes) return cudaSuccess;
     const uint32_t n = 3 * S.n_nodes;
-    launch_fill_sentinel<T>(n, tmp, s);
+    if (!filled) launch_fill_sentinel<T>(n, tmp, s);
     // in place (y == r) the forward solve still reads r: fill y after it
     const bool fuse = y != r;
     cudaError_t e =
-        launch_dir<T, true>(P, S, lu, dinv, r, tmp, fuse ? y : nullptr, fuse ? n : 0, status, s);
+        launch_dir<T, true>(P, S, lu, dinv, r, tmp, fuse ? y : nullptr, fuse ? n : 0, status, skip,
+                            s);
     if (e != cudaSuccess) return e;
     if (!fuse) launch_fill_sentinel<T>(n, y, s);
-    return launch_dir<T, false>(P, S, lu, dinv, tmp, y, nullptr, 0, status, s);
+    return launch_dir<T, false>(P, S, lu, dinv, tmp, y, nullptr, 0, status, skip, s);
 }
 
 template cudaError_t launch_trsv_push<double>(const PushSolve&, const NodeSched&, const double*,
                                               const double*, const double*, double*, double*,
-                                              unsigned*, cudaStream_t);
+                                              unsigned*, cudaStream_t, const unsigned*, bool);
 template cudaError_t launch_trsv_push<float>(const PushSolve&, const NodeSched&, const float*,
                                              const float*, const float*, float*, float*,
-                                             unsigned*, cudaStream_t);
+                                             unsigned*, cudaStream_t, const unsigned*, bool);
 
 }  // namespace fm
