@@ -34,6 +34,21 @@ struct SolverCsr {
     uint32_t max_row = 0;
     DevBuf<uint32_t> rp, ci, dpos, upos, fwd, bwd;
     std::vector<uint32_t> h_rp, h_ci;
+    // single-CTA solves (fm_trsv_small.cu): entries per row and side (0: the
+    // matrix is not one of theirs), streams in level order
+    uint32_t small_entries = 0, small_width = 0, nl_f = 0, nl_b = 0;
+    DevBuf<uint32_t> lvl_f, lvl_b, col_f, col_b, src_f, src_b;
+    DevBuf<double> val_f, val_b, dinv_b;
+    fm::SmallTri tri(bool lower) const {
+        fm::SmallTri t;
+        t.n_levels = lower ? nl_f : nl_b;
+        t.level = lower ? lvl_f.p : lvl_b.p;
+        t.row = lower ? fwd.p : bwd.p;
+        t.col = lower ? col_f.p : col_b.p;
+        t.val = lower ? val_f.p : val_b.p;
+        t.dinv = lower ? nullptr : dinv_b.p;
+        return t;
+    }
     fm::CsrDev view() const {
         fm::CsrDev v;
         v.n = n;
@@ -302,6 +317,54 @@ fm::MeshDev mesh_view(const fm_ctx* c) {
     return m;
 }
 
+// Streams of the single-CTA solves for a CSR that fits them: per direction
+// and level position, the columns and LU slots of the row's entries, padded
+// to the same count (zero coefficient, column n).
+fm_status setup_small_tri(fm_ctx* c, SolverCsr& S, const std::vector<uint32_t>& rp,
+                          const std::vector<uint32_t>& ci, const std::vector<uint32_t>& dpos,
+                          const std::vector<uint32_t>& upos, const std::vector<uint32_t>& fp,
+                          const std::vector<uint32_t>& fr, const std::vector<uint32_t>& bp,
+                          const std::vector<uint32_t>& br) {
+    const uint32_t n = S.n;
+    S.small_entries = 0;
+    uint32_t most = 1, width = 1;
+    for (uint32_t i = 0; i < n; ++i)
+        most = std::max({most, dpos[i] - rp[i], rp[i + 1] - upos[i]});
+    S.nl_f = (uint32_t)fp.size() - 1;
+    S.nl_b = (uint32_t)bp.size() - 1;
+    if (most > fm::kSmallMaxEntries ||
+        fm::small_tri_smem(n, S.nl_f, S.nl_b) > fm::kSmallMaxSmem)
+        return FM_OK;
+    for (const auto* p : {&fp, &bp})
+        for (size_t l = 0; l + 1 < p->size(); ++l) width = std::max(width, (*p)[l + 1] - (*p)[l]);
+    const uint32_t M = most <= 2 ? 2 : most <= 4 ? 4 : 8;
+    std::vector<uint32_t> col((size_t)M * n), src((size_t)M * n);
+    for (int lower = 1; lower >= 0; --lower) {
+        const std::vector<uint32_t>& ord = lower ? fr : br;
+        std::fill(col.begin(), col.end(), n);
+        std::fill(src.begin(), src.end(), ~0u);
+        for (uint32_t t = 0; t < n; ++t) {
+            const uint32_t i = ord[t];
+            const uint32_t b = lower ? rp[i] : upos[i], e = lower ? dpos[i] : rp[i + 1];
+            for (uint32_t k = b; k < e; ++k) {
+                col[(size_t)(k - b) * n + t] = ci[k];
+                src[(size_t)(k - b) * n + t] = k;
+            }
+        }
+        CK(upload(lower ? S.lvl_f : S.lvl_b, (lower ? fp : bp).data(), (lower ? fp : bp).size(),
+                  c->stream));
+        CK(upload(lower ? S.col_f : S.col_b, col.data(), col.size(), c->stream));
+        CK(upload(lower ? S.src_f : S.src_b, src.data(), src.size(), c->stream));
+        CK(cudaStreamSynchronize(c->stream));  // col and src are reused
+    }
+    CK(S.val_f.reserve((size_t)M * n));
+    CK(S.val_b.reserve((size_t)M * n));
+    CK(S.dinv_b.reserve(n));
+    S.small_entries = M;
+    S.small_width = width;
+    return FM_OK;
+}
+
 // Build the solver CSR (ascending columns) on host and upload: row
 // pointers, columns, first-diagonal/first-upper positions and the DOF-level
 // dependency orders that the sync-free kernels walk.
@@ -329,6 +392,7 @@ fm_status setup_solver_csr(fm_ctx* c, SolverCsr& S, uint32_t n, std::vector<uint
     CK(upload(S.upos, upos.data(), n, c->stream));
     CK(upload(S.fwd, fr.data(), fr.size(), c->stream));
     CK(upload(S.bwd, br.data(), br.size(), c->stream));
+    TRY(setup_small_tri(c, S, rp, ci, dpos, upos, fp, fr, bp, br));
     S.h_rp = std::move(rp);
     S.h_ci = std::move(ci);
     CK(c->done.reserve(std::max<size_t>(c->done.n, n + 1)));
@@ -560,16 +624,25 @@ struct Op {
             fm::launch_spmv_nodes<T>(c->nn, c->nbr_ptr.p, c->nbr.p, K, x, y, part, c->counter(),
                                      dot, c->stream, skip);
         else
-            fm::launch_spmv_csr<T>(S->n, S->rp.p, S->ci.p, K, x, y, part, c->counter(), dot,
-                                   c->stream, skip);
+            fm::launch_spmv_csr<T>(S->n, S->nnz, S->rp.p, S->ci.p, K, x, y, part, c->counter(),
+                                   dot, c->stream, skip);
     }
     void precond(const T* r, T* z, const unsigned* skip = nullptr, bool filled = false) const {
         const bool pu = node_block && (sizeof(T) == 4 ? c->pu_ok32 : c->pu_ok64);
-        PROF(FM_PROF_TRSV, pu ? (r != z ? 3 : 4) - (filled ? 1 : 0) : node_block ? 4 : 2);
+        PROF(FM_PROF_TRSV, pu ? (r != z ? 3 : 4) - (filled ? 1 : 0)
+                              : node_block ? 4 : S->small_entries ? 1 : 2);
         if (node_block) {
             precond_nodes<T>(c, LU, dinv, r, tmp, z, c->status(), skip, filled);
             return;
         }
+        if constexpr (sizeof(T) == 8)
+            if (S->small_entries) {
+                if (fm::launch_trsv_small(S->tri(true), S->tri(false), S->n, S->small_entries,
+                                          S->small_width, r, z, skip, c->stream) == cudaSuccess)
+                    return;
+                cudaGetLastError();  // refused by the device: the solves below from now on
+                S->small_entries = 0;
+            }
         const fm::CsrDev v = S->view();
         fm::launch_trsv_lower_csr<T>(v, LU, r, tmp, c->done.p, next_epoch(c), c->status(),
                                      grid_trsv, c->stream, skip);
@@ -1343,6 +1416,7 @@ fm_status fm_csr_pcg_ilu0(fm_ctx* c, uint32_t n, const uint32_t* row_ptr,
                 if (ci[k] >= n) return fail(c, FM_ERR_ARG, "column %u out of range", ci[k]);
                 row.emplace_back(ci[k], v[k]);
             }
+            if (std::is_sorted(ci.begin() + rp[i], ci.begin() + rp[i + 1])) continue;
             std::stable_sort(row.begin(), row.end(),
                              [](const auto& a, const auto& b2) { return a.first < b2.first; });
             for (size_t q = 0; q < row.size(); ++q) {
@@ -1361,6 +1435,13 @@ fm_status fm_csr_pcg_ilu0(fm_ctx* c, uint32_t n, const uint32_t* row_ptr,
         CK(cudaMemcpyAsync(c->vec_a.p, b, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemcpyAsync(c->vec_b.p, x, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
         TRY(ilu_core<double>(c, c->gen, c->gen_K.p, c->gen_LU.p, c->gen_diag.p));
+        if (c->gen.small_entries) {
+            PROF(FM_PROF_ILU, 1);
+            fm::launch_pack_small(n, c->gen.small_entries, c->gen.src_f.p, c->gen.src_b.p,
+                                  c->gen.bwd.p, c->gen_LU.p, c->gen_diag.p, c->gen.val_f.p,
+                                  c->gen.val_b.p, c->gen.dinv_b.p, c->stream);
+            CK(cudaGetLastError());
+        }
         Op<double> A{c, &c->gen, false, c->gen_K.p, c->gen_LU.p, c->gen_diag.p, c->w64.t.p,
                      c->grid_trsv64};
         TRY(pcg_core<double>(c, A, n, c->vec_a.p, c->vec_b.p, tol, max_iter, iters, relres));

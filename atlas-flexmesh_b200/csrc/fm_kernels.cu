@@ -646,21 +646,29 @@ void launch_spmv_nodes(uint32_t n_nodes, const uint32_t* nbr_ptr, const uint32_t
                                          skip);
 }
 
-template <typename T>
+// G lanes per row (a power of two near the mean row length: a warp per
+// five-entry row leaves 27 of its lanes idle)
+template <typename T, int G>
 __global__ void __launch_bounds__(256)
     k_spmv_csr(uint32_t n, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
                const T* __restrict__ val, const T* __restrict__ x, T* __restrict__ y,
                T* partials, unsigned* counter, double* dot, const unsigned* __restrict__ skip) {
     if (skipped(skip)) return;
-    const int lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & (G - 1);
+    const uint32_t group = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const uint32_t ngroups = gridDim.x * blockDim.x / G;
     T dsum = T(0);
-    for (uint32_t i = warp; i < n; i += nwarps) {
+    // whole warps step together: the group sum shuffles over the full warp
+    const uint32_t steps = (n + ngroups - 1) / ngroups;
+    for (uint32_t q = 0; q < steps; ++q) {
+        const uint32_t i = group + q * ngroups;
         T s = T(0);
-        for (uint32_t k = rp[i] + lane; k < rp[i + 1]; k += 32) s += __ldg(val + k) * __ldg(x + ci[k]);
-        s = warp_sum(s);
-        if (lane == 0) {
+        if (i < n)
+            for (uint32_t k = rp[i] + lane; k < rp[i + 1]; k += G)
+                s += __ldg(val + k) * __ldg(x + ci[k]);
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+        if (i < n && lane == 0) {
             y[i] = s;
             if (dot) dsum += s * x[i];
         }
@@ -672,12 +680,26 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+template <typename T, int G>
+static void launch_spmv_csr_g(uint32_t n, const uint32_t* rp, const uint32_t* ci, const T* val,
+                              const T* x, T* y, T* partials, unsigned* counter, double* dot,
+                              cudaStream_t s, const unsigned* skip) {
+    const uint32_t per = 256 / G;  // rows per block and step
+    const int grid = (int)std::min<uint32_t>(kSpmvBlocks, std::max(1u, (n + per - 1) / per));
+    k_spmv_csr<T, G><<<grid, 256, 0, s>>>(n, rp, ci, val, x, y, partials, counter, dot, skip);
+}
+
 template <typename T>
-void launch_spmv_csr(uint32_t n, const uint32_t* rp, const uint32_t* ci, const T* val, const T* x,
-                     T* y, T* partials, unsigned* counter, double* dot, cudaStream_t s,
-                     const unsigned* skip) {
-    const int grid = (int)std::min<uint32_t>(kSpmvBlocks, std::max(1u, (n + 7) / 8));
-    k_spmv_csr<T><<<grid, 256, 0, s>>>(n, rp, ci, val, x, y, partials, counter, dot, skip);
+void launch_spmv_csr(uint32_t n, uint64_t nnz, const uint32_t* rp, const uint32_t* ci,
+                     const T* val, const T* x, T* y, T* partials, unsigned* counter, double* dot,
+                     cudaStream_t s, const unsigned* skip) {
+    const uint64_t mean = n ? nnz / n : 0;
+    if (mean <= 6)
+        launch_spmv_csr_g<T, 4>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
+    else if (mean <= 16)
+        launch_spmv_csr_g<T, 8>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
+    else
+        launch_spmv_csr_g<T, 32>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
 }
 
 // ===========================================================================
@@ -1223,9 +1245,9 @@ template void launch_apply_bc_nodes<float>(uint32_t, const uint32_t*, const uint
     template void launch_spmv_nodes<T>(uint32_t, const uint32_t*, const uint32_t*, const T*,    \
                                        const T*, T*, T*, unsigned*, double*, cudaStream_t,      \
                                        const unsigned*);                                        \
-    template void launch_spmv_csr<T>(uint32_t, const uint32_t*, const uint32_t*, const T*,      \
-                                     const T*, T*, T*, unsigned*, double*, cudaStream_t,        \
-                                     const unsigned*);                                          \
+    template void launch_spmv_csr<T>(uint32_t, uint64_t, const uint32_t*, const uint32_t*,      \
+                                     const T*, const T*, T*, T*, unsigned*, double*,            \
+                                     cudaStream_t, const unsigned*);                            \
     template void launch_ilu0_csr<T>(const CsrDev&, const T*, T*, T*, unsigned*, unsigned,      \
                                      unsigned*, int, cudaStream_t);                             \
     template void launch_trsv_lower_csr<T>(const CsrDev&, const T*, const T*, T*, unsigned*,    \

@@ -71,9 +71,9 @@ void launch_spmv_nodes(uint32_t n_nodes, const uint32_t* nbr_ptr, const uint32_t
                        double* dot, cudaStream_t s, const unsigned* skip = nullptr);
 // Generic scalar CSR SpMV (ascending or any column order)
 template <typename T>
-void launch_spmv_csr(uint32_t n, const uint32_t* rp, const uint32_t* ci, const T* val, const T* x,
-                     T* y, T* partials, unsigned* counter, double* dot, cudaStream_t s,
-                     const unsigned* skip = nullptr);
+void launch_spmv_csr(uint32_t n, uint64_t nnz, const uint32_t* rp, const uint32_t* ci,
+                     const T* val, const T* x, T* y, T* partials, unsigned* counter, double* dot,
+                     cudaStream_t s, const unsigned* skip = nullptr);
 
 // Sync-free ILU(0) and triangular solves on a CSR with ascending columns.
 // order: a topological order of the rows (dependency levels); done: one
@@ -102,6 +102,32 @@ void launch_trsv_upper_csr(const CsrDev& A, const T* lu, const T* diag, const T*
 // persistent grid sizes (all blocks co-resident) for the sync-free kernels
 int persistent_grid_ilu0_csr(int device, bool fp32, const CsrDev& A);
 int persistent_grid_trsv_csr(int device, bool fp32);
+
+// One direction of a small generic factorization, rows in level order
+// (fm_trsv_small.cu): level pointers, row and, per entry m and position t,
+// column (n: padding) and coefficient at [m * n + t]; dinv per position
+// (backward only).
+struct SmallTri {
+    uint32_t n_levels = 0;
+    const uint32_t* level = nullptr;
+    const uint32_t* row = nullptr;
+    const uint32_t* col = nullptr;
+    const double* val = nullptr;
+    const double* dinv = nullptr;
+};
+constexpr uint32_t kSmallMaxEntries = 8;
+constexpr size_t kSmallMaxSmem = 220 * 1024;
+size_t small_tri_smem(uint32_t n, uint32_t nlf, uint32_t nlb);
+// gathers the packed coefficients of both directions from LU (src ~0u: zero)
+// and the reciprocal pivots in the backward order
+void launch_pack_small(uint32_t n, uint32_t entries, const uint32_t* src_f, const uint32_t* src_b,
+                       const uint32_t* row_b, const double* lu, const double* diag, double* val_f,
+                       double* val_b, double* dinv, cudaStream_t s);
+// out = U^-1 L^-1 r; entries: per row and side (2, 4 or 8), width: the
+// widest level of either direction
+cudaError_t launch_trsv_small(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t entries,
+                              uint32_t width, const double* r, double* out, const unsigned* skip,
+                              cudaStream_t s);
 
 // PCG vector kernels; all reductions deterministic (the grid depends on n
 // alone).  Once sc->done is set they return at once.

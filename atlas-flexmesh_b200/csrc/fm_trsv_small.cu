@@ -1,0 +1,165 @@
+// fm_trsv_small.cu — triangular solves of a generic CSR factorization whose
+// vector fits one SM's shared memory.
+//
+// On short rows the solves are chains of dependency levels with little work
+// in each (2 x 299 levels of at most 150 rows on a 150 x 150 five-point
+// matrix), so their time is the cost of passing values from one level to the
+// next.  Through L2, with a warp per row and a release flag each, a level
+// cost 3.7 us (2.2 ms per apply there).  Here one CTA keeps the whole vector
+// in shared memory and takes a level at a time, one thread per row, with a
+// block barrier between levels: 0.1 us per level.
+//
+// The factors come as one stream per direction in level order, entry m of
+// position t at [m * n + t] (rows with fewer entries are padded with zero
+// coefficients that read a zero), packed after each factorization; a
+// thread's entries of the next kDepth levels are in flight in registers.
+//
+// Used when the vector and the level pointers fit shared memory and no row
+// has more than kSmallMaxEntries off-diagonal entries on one side: longer
+// rows would leave a thread with a long serial sum, and belong to the
+// warp-per-row solves.
+#include <algorithm>
+
+#include "fm_kernels.hpp"
+
+namespace fm {
+
+namespace {
+
+template <int M>
+struct Row {
+    double v[M];
+    uint32_t c[M];
+    double d;
+    uint32_t row;
+};
+
+template <int M, bool Upper>
+__device__ __forceinline__ void load_row(const SmallTri& S, const uint32_t* lvl, uint32_t nl,
+                                         uint32_t l, uint32_t n, Row<M>& E) {
+    E.row = ~0u;
+    if (l >= nl) return;
+    const uint32_t t = lvl[l] + threadIdx.x;
+    if (t >= lvl[l + 1]) return;
+    E.row = __ldg(S.row + t);
+    if (Upper) E.d = __ldg(S.dinv + t);
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        E.c[m] = __ldg(S.col + (size_t)m * n + t);
+        E.v[m] = __ldg(S.val + (size_t)m * n + t);
+    }
+}
+
+template <int M, bool Upper>
+__device__ __forceinline__ void solve_row(const Row<M>& E, double* z) {
+    double s = z[E.row];
+#pragma unroll
+    for (int m = 0; m < M; ++m) s -= E.v[m] * z[E.c[m]];
+    z[E.row] = Upper ? s * E.d : s;
+}
+
+// one direction, in place on z (z[n] = 0 for the padding)
+template <int M, int D, bool Upper>
+__device__ __forceinline__ void sweep(const SmallTri& S, const uint32_t* lvl, uint32_t n,
+                                      double* z) {
+    Row<M> e[D];
+#pragma unroll
+    for (int q = 0; q < D; ++q) load_row<M, Upper>(S, lvl, S.n_levels, q, n, e[q]);
+    for (uint32_t l0 = 0; l0 < S.n_levels; l0 += D) {
+#pragma unroll
+        for (int q = 0; q < D; ++q) {
+            const uint32_t l = l0 + q;
+            if (l < S.n_levels) {  // uniform
+                if (e[q].row != ~0u) solve_row<M, Upper>(e[q], z);
+                // rows of a level beyond the block's width
+                for (uint32_t t = lvl[l] + threadIdx.x + blockDim.x; t < lvl[l + 1];
+                     t += blockDim.x) {
+                    Row<M> x;
+                    x.row = __ldg(S.row + t);
+                    if (Upper) x.d = __ldg(S.dinv + t);
+#pragma unroll
+                    for (int m = 0; m < M; ++m) {
+                        x.c[m] = __ldg(S.col + (size_t)m * n + t);
+                        x.v[m] = __ldg(S.val + (size_t)m * n + t);
+                    }
+                    solve_row<M, Upper>(x, z);
+                }
+                load_row<M, Upper>(S, lvl, S.n_levels, l + D, n, e[q]);
+                __syncthreads();
+            }
+        }
+    }
+}
+
+template <int M, int D, int Threads>
+__global__ void __launch_bounds__(Threads, 1)
+    k_trsv_small(SmallTri L, SmallTri U, uint32_t n, const double* __restrict__ r,
+                 double* __restrict__ out, const unsigned* __restrict__ skip) {
+    if (skipped(skip)) return;
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    double* z = reinterpret_cast<double*>(small_smem);
+    uint32_t* lf = reinterpret_cast<uint32_t*>(z + n + 1);
+    uint32_t* lb = lf + L.n_levels + 1;
+#pragma unroll 8
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) z[i] = r[i];
+    if (threadIdx.x == 0) z[n] = 0.0;
+    for (uint32_t i = threadIdx.x; i <= L.n_levels; i += blockDim.x) lf[i] = __ldg(L.level + i);
+    for (uint32_t i = threadIdx.x; i <= U.n_levels; i += blockDim.x) lb[i] = __ldg(U.level + i);
+    __syncthreads();
+    sweep<M, D, false>(L, lf, n, z);
+    sweep<M, D, true>(U, lb, n, z);
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) out[i] = z[i];
+}
+
+__global__ void k_pack_small(uint32_t n, uint32_t total, const uint32_t* __restrict__ src_f,
+                             const uint32_t* __restrict__ src_b,
+                             const uint32_t* __restrict__ row_b, const double* __restrict__ lu,
+                             const double* __restrict__ diag, double* __restrict__ val_f,
+                             double* __restrict__ val_b, double* __restrict__ dinv) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total;
+         i += gridDim.x * blockDim.x) {
+        const uint32_t a = src_f[i], b = src_b[i];
+        val_f[i] = a != ~0u ? lu[a] : 0.0;
+        val_b[i] = b != ~0u ? lu[b] : 0.0;
+        if (i < n) dinv[i] = 1.0 / diag[row_b[i]];
+    }
+}
+
+template <int M, int D, int Threads>
+cudaError_t launch_t(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t width,
+                     const double* r, double* out, const unsigned* skip, cudaStream_t s) {
+    const size_t smem = small_tri_smem(n, L.n_levels, U.n_levels);
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_trsv_small<M, D, Threads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    // no more threads than the widest level has rows (fewer warps, a cheaper
+    // barrier) or than the copies in and out can use
+    const unsigned th =
+        std::min<unsigned>(Threads, std::max(32u, (std::max(width, n / 64) + 31u) & ~31u));
+    k_trsv_small<M, D, Threads><<<1, th, smem, s>>>(L, U, n, r, out, skip);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+size_t small_tri_smem(uint32_t n, uint32_t nlf, uint32_t nlb) {
+    return 8 * ((size_t)n + 1) + 4 * ((size_t)nlf + nlb + 2);
+}
+
+void launch_pack_small(uint32_t n, uint32_t entries, const uint32_t* src_f, const uint32_t* src_b,
+                       const uint32_t* row_b, const double* lu, const double* diag, double* val_f,
+                       double* val_b, double* dinv, cudaStream_t s) {
+    const uint32_t total = entries * n;
+    k_pack_small<<<(total + 255) / 256, 256, 0, s>>>(n, total, src_f, src_b, row_b, lu, diag,
+                                                     val_f, val_b, dinv);
+}
+
+cudaError_t launch_trsv_small(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t entries,
+                              uint32_t width, const double* r, double* out, const unsigned* skip,
+                              cudaStream_t s) {
+    if (entries <= 2) return launch_t<2, 4, 1024>(L, U, n, width, r, out, skip, s);
+    if (entries <= 4) return launch_t<4, 4, 512>(L, U, n, width, r, out, skip, s);
+    return launch_t<8, 2, 512>(L, U, n, width, r, out, skip, s);
+}
+
+}  // namespace fm
