@@ -7,12 +7,14 @@
 // next.  Through L2, with a warp per row and a release flag each, a level
 // cost 3.7 us (2.2 ms per apply there).  Here one CTA keeps the whole vector
 // in shared memory and takes a level at a time, one thread per row, with a
-// block barrier between levels: 0.1 us per level.
+// block barrier between levels: 0.22 us per level.
 //
 // The factors come as one stream per direction in level order, entry m of
 // position t at [m * n + t] (rows with fewer entries are padded with zero
 // coefficients that read a zero), packed after each factorization; a
-// thread's entries of the next kDepth levels are in flight in registers.
+// thread's entries of the next two levels are in flight in registers (131 us
+// per apply there, 90 of them without any loads; three to six levels ahead
+// took 141 to 178, as did 16-byte packed rows, and a cp.async ring 143).
 //
 // Used when the vector and the level pointers fit shared memory and no row
 // has more than kSmallMaxEntries off-diagonal entries on one side: longer
@@ -26,6 +28,8 @@ namespace fm {
 
 namespace {
 
+constexpr int kMaxDepth = 2;  // levels whose entries are in flight
+
 template <int M>
 struct Row {
     double v[M];
@@ -34,13 +38,10 @@ struct Row {
     uint32_t row;
 };
 
+// the row at position t (unconditional, so that nothing waits for the loads
+// before the row is solved: the caller clamps t)
 template <int M, bool Upper>
-__device__ __forceinline__ void load_row(const SmallTri& S, const uint32_t* lvl, uint32_t nl,
-                                         uint32_t l, uint32_t n, Row<M>& E) {
-    E.row = ~0u;
-    if (l >= nl) return;
-    const uint32_t t = lvl[l] + threadIdx.x;
-    if (t >= lvl[l + 1]) return;
+__device__ __forceinline__ void load_row(const SmallTri& S, uint32_t t, uint32_t n, Row<M>& E) {
     E.row = __ldg(S.row + t);
     if (Upper) E.d = __ldg(S.dinv + t);
 #pragma unroll
@@ -58,33 +59,28 @@ __device__ __forceinline__ void solve_row(const Row<M>& E, double* z) {
     z[E.row] = Upper ? s * E.d : s;
 }
 
-// one direction, in place on z (z[n] = 0 for the padding)
+// one direction, in place on z (z[n] = 0 for the padding); lvl[n_levels ..
+// n_levels + D] = n
 template <int M, int D, bool Upper>
 __device__ __forceinline__ void sweep(const SmallTri& S, const uint32_t* lvl, uint32_t n,
                                       double* z) {
     Row<M> e[D];
 #pragma unroll
-    for (int q = 0; q < D; ++q) load_row<M, Upper>(S, lvl, S.n_levels, q, n, e[q]);
+    for (int q = 0; q < D; ++q) load_row<M, Upper>(S, min(lvl[q] + threadIdx.x, n - 1), n, e[q]);
     for (uint32_t l0 = 0; l0 < S.n_levels; l0 += D) {
 #pragma unroll
         for (int q = 0; q < D; ++q) {
             const uint32_t l = l0 + q;
             if (l < S.n_levels) {  // uniform
-                if (e[q].row != ~0u) solve_row<M, Upper>(e[q], z);
+                const uint32_t b = lvl[l], end = lvl[l + 1], next = lvl[l + D];
+                if (b + threadIdx.x < end) solve_row<M, Upper>(e[q], z);
                 // rows of a level beyond the block's width
-                for (uint32_t t = lvl[l] + threadIdx.x + blockDim.x; t < lvl[l + 1];
-                     t += blockDim.x) {
+                for (uint32_t t = b + threadIdx.x + blockDim.x; t < end; t += blockDim.x) {
                     Row<M> x;
-                    x.row = __ldg(S.row + t);
-                    if (Upper) x.d = __ldg(S.dinv + t);
-#pragma unroll
-                    for (int m = 0; m < M; ++m) {
-                        x.c[m] = __ldg(S.col + (size_t)m * n + t);
-                        x.v[m] = __ldg(S.val + (size_t)m * n + t);
-                    }
+                    load_row<M, Upper>(S, t, n, x);
                     solve_row<M, Upper>(x, z);
                 }
-                load_row<M, Upper>(S, lvl, S.n_levels, l + D, n, e[q]);
+                load_row<M, Upper>(S, min(next + threadIdx.x, n - 1), n, e[q]);
                 __syncthreads();
             }
         }
@@ -99,12 +95,14 @@ __global__ void __launch_bounds__(Threads, 1)
     extern __shared__ __align__(16) unsigned char small_smem[];
     double* z = reinterpret_cast<double*>(small_smem);
     uint32_t* lf = reinterpret_cast<uint32_t*>(z + n + 1);
-    uint32_t* lb = lf + L.n_levels + 1;
+    uint32_t* lb = lf + L.n_levels + 1 + D;
 #pragma unroll 8
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) z[i] = r[i];
     if (threadIdx.x == 0) z[n] = 0.0;
-    for (uint32_t i = threadIdx.x; i <= L.n_levels; i += blockDim.x) lf[i] = __ldg(L.level + i);
-    for (uint32_t i = threadIdx.x; i <= U.n_levels; i += blockDim.x) lb[i] = __ldg(U.level + i);
+    for (uint32_t i = threadIdx.x; i <= L.n_levels + D; i += blockDim.x)
+        lf[i] = i < L.n_levels ? __ldg(L.level + i) : n;
+    for (uint32_t i = threadIdx.x; i <= U.n_levels + D; i += blockDim.x)
+        lb[i] = i < U.n_levels ? __ldg(U.level + i) : n;
     __syncthreads();
     sweep<M, D, false>(L, lf, n, z);
     sweep<M, D, true>(U, lb, n, z);
@@ -143,7 +141,7 @@ cudaError_t launch_t(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t 
 }  // namespace
 
 size_t small_tri_smem(uint32_t n, uint32_t nlf, uint32_t nlb) {
-    return 8 * ((size_t)n + 1) + 4 * ((size_t)nlf + nlb + 2);
+    return 8 * ((size_t)n + 1) + 4 * ((size_t)nlf + nlb + 2 + 2 * kMaxDepth);
 }
 
 void launch_pack_small(uint32_t n, uint32_t entries, const uint32_t* src_f, const uint32_t* src_b,
@@ -157,8 +155,8 @@ void launch_pack_small(uint32_t n, uint32_t entries, const uint32_t* src_f, cons
 cudaError_t launch_trsv_small(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t entries,
                               uint32_t width, const double* r, double* out, const unsigned* skip,
                               cudaStream_t s) {
-    if (entries <= 2) return launch_t<2, 4, 1024>(L, U, n, width, r, out, skip, s);
-    if (entries <= 4) return launch_t<4, 4, 512>(L, U, n, width, r, out, skip, s);
+    if (entries <= 2) return launch_t<2, 2, 1024>(L, U, n, width, r, out, skip, s);
+    if (entries <= 4) return launch_t<4, 2, 512>(L, U, n, width, r, out, skip, s);
     return launch_t<8, 2, 512>(L, U, n, width, r, out, skip, s);
 }
 

@@ -65,8 +65,8 @@ CASES = {
     "nine_per_side": (300, band(300, 9, 5), False),
     "diagonal": (2050, [], False),
     "wide_shift": (5000, band(5000, 1, 1100), False),
-    "at_the_limit": (28000, band(28000, 2, 7000), True),
-    "past_the_limit": (28200, band(28200, 2, 7000), False),
+    "at_the_limit": (27000, band(27000, 2, 7000), True),
+    "past_the_limit": (28600, band(28600, 2, 7000), False),
 }
 
 
