@@ -84,6 +84,38 @@ __device__ __forceinline__ unsigned ld_volatile_u32(const unsigned* p) {
 __device__ __forceinline__ double ld_cg(const double* p) { return __ldcg(p); }
 __device__ __forceinline__ float ld_cg(const float* p) { return __ldcg(p); }
 
+// Programmatic dependent launch (sm_90 and later): a kernel launched with
+// launch_chained may start while the kernel before it in the stream is still
+// running, and chain_begin holds it until that one has completed and its
+// writes are visible.  Every thread calls it before it touches anything that
+// earlier kernels write or read; the successor is let in at once, so that its
+// blocks are scheduled as this kernel's leave.
+__device__ __forceinline__ void chain_let_next() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void chain_begin() {
+    chain_let_next();
+    chain_wait();
+}
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                           cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // *skip set (null: never): the kernel has nothing to do
 __device__ __forceinline__ bool skipped(const unsigned* skip) {
     return skip && ld_volatile_u32(skip) != 0u;

@@ -599,6 +599,7 @@ __global__ void __launch_bounds__(256)
                  const uint32_t* __restrict__ nbr, const T* __restrict__ val,
                  const T* __restrict__ x, T* __restrict__ y, T* partials, unsigned* counter,
                  double* dot, const unsigned* __restrict__ skip) {
+    chain_begin();
     if (skipped(skip)) return;
     const int lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -642,8 +643,8 @@ void launch_spmv_nodes(uint32_t n_nodes, const uint32_t* nbr_ptr, const uint32_t
                        double* dot, cudaStream_t s, const unsigned* skip) {
     // no blocks without a node: each would still take its turn at the counter
     const int grid = (int)std::min<uint32_t>(kSpmvBlocks, std::max(1u, (n_nodes + 7) / 8));
-    k_spmv_nodes<T><<<grid, 256, 0, s>>>(n_nodes, nbr_ptr, nbr, val, x, y, partials, counter, dot,
-                                         skip);
+    launch_chained(k_spmv_nodes<T>, grid, 256, 0, s, n_nodes, nbr_ptr, nbr, val, x, y, partials,
+                   counter, dot, skip);
 }
 
 // G lanes per row (a power of two near the mean row length: a warp per
@@ -653,6 +654,7 @@ __global__ void __launch_bounds__(256)
     k_spmv_csr(uint32_t n, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
                const T* __restrict__ val, const T* __restrict__ x, T* __restrict__ y,
                T* partials, unsigned* counter, double* dot, const unsigned* __restrict__ skip) {
+    chain_begin();
     if (skipped(skip)) return;
     const int lane = threadIdx.x & (G - 1);
     const uint32_t group = (blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -686,7 +688,8 @@ static void launch_spmv_csr_g(uint32_t n, const uint32_t* rp, const uint32_t* ci
                               cudaStream_t s, const unsigned* skip) {
     const uint32_t per = 256 / G;  // rows per block and step
     const int grid = (int)std::min<uint32_t>(kSpmvBlocks, std::max(1u, (n + per - 1) / per));
-    k_spmv_csr<T, G><<<grid, 256, 0, s>>>(n, rp, ci, val, x, y, partials, counter, dot, skip);
+    launch_chained(k_spmv_csr<T, G>, grid, 256, 0, s, n, rp, ci, val, x, y, partials, counter, dot,
+                   skip);
 }
 
 template <typename T>
@@ -932,6 +935,7 @@ __global__ void __launch_bounds__(kVecThreads)
     k_pcg_init(uint32_t n, const T* __restrict__ b, T* __restrict__ r, int zero_x,
                T* __restrict__ tmp, double tol, T* partials, unsigned* counter, DevScalars* sc,
                PcgReport* rep, unsigned seq) {
+    chain_begin();
     T s = T(0);
 #pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -954,8 +958,8 @@ template <typename T>
 void launch_pcg_init(uint32_t n, const T* b, T* r, bool zero_x, T* tmp, double tol, T* partials,
                      unsigned* counter, DevScalars* sc, PcgReport* rep, unsigned seq,
                      cudaStream_t s) {
-    k_pcg_init<T><<<red_blocks(n), kVecThreads, 0, s>>>(n, b, r, zero_x, tmp, tol, partials,
-                                                        counter, sc, rep, seq);
+    launch_chained(k_pcg_init<T>, red_blocks(n), kVecThreads, 0, s, n, b, r, zero_x, tmp, tol,
+                   partials, counter, sc, rep, seq);
 }
 
 // p = z; rz = r.z; bb = b.b.  Two sums share one pass (partials: 2 slots per block)
@@ -964,6 +968,7 @@ __global__ void __launch_bounds__(kVecThreads)
     k_pcg_start(uint32_t n, const T* __restrict__ r, const T* __restrict__ z,
                 const T* __restrict__ b, T* __restrict__ p, T* partials, unsigned* counter,
                 DevScalars* sc) {
+    chain_begin();
     if (skipped(&sc->done)) return;
     T s1 = T(0), s2 = T(0);
 #pragma unroll 4
@@ -987,7 +992,8 @@ __global__ void __launch_bounds__(kVecThreads)
 template <typename T>
 void launch_pcg_start(uint32_t n, const T* r, const T* z, const T* b, T* p, T* partials,
                       unsigned* counter, DevScalars* sc, cudaStream_t s) {
-    k_pcg_start<T><<<red_blocks(n), kVecThreads, 0, s>>>(n, r, z, b, p, partials, counter, sc);
+    launch_chained(k_pcg_start<T>, red_blocks(n), kVecThreads, 0, s, n, r, z, b, p, partials,
+                   counter, sc);
 }
 
 // alpha = rz/pAp (current rz is rz_new); breakdown |pAp| < 1e-60 stops
@@ -998,6 +1004,7 @@ template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
     k_pcg_update_xr(uint32_t n, const T* __restrict__ p, const T* __restrict__ Ap,
                     T* __restrict__ x, T* __restrict__ r, T* __restrict__ tmp, DevScalars* sc) {
+    chain_begin();
     if (skipped(&sc->done)) return;
     const double pAp = sc->pAp;
     if (fabs(pAp) < 1e-60) {
@@ -1016,7 +1023,8 @@ __global__ void __launch_bounds__(kVecThreads)
 template <typename T>
 void launch_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* x, T* r, T* tmp, DevScalars* sc,
                           cudaStream_t s) {
-    k_pcg_update_xr<T><<<2 * red_blocks(n), kVecThreads, 0, s>>>(n, p, Ap, x, r, tmp, sc);
+    launch_chained(k_pcg_update_xr<T>, 2 * red_blocks(n), kVecThreads, 0, s, n, p, Ap, x, r, tmp,
+                   sc);
 }
 
 // rz <- rz_new (old value kept for beta), rz_new <- r.z, relres, the stop
@@ -1025,6 +1033,7 @@ template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
     k_pcg_rz(uint32_t n, const T* __restrict__ r, const T* __restrict__ z, double tol, T* partials,
              unsigned* counter, DevScalars* sc, PcgReport* rep, unsigned seq) {
+    chain_begin();
     if (skipped(&sc->done)) return;
     if (ld_volatile_u32(&sc->stop)) {
         // the other blocks return here or, once done is set, above
@@ -1053,13 +1062,14 @@ __global__ void __launch_bounds__(kVecThreads)
 template <typename T>
 void launch_pcg_rz(uint32_t n, const T* r, const T* z, double tol, T* partials, unsigned* counter,
                    DevScalars* sc, PcgReport* rep, unsigned seq, cudaStream_t s) {
-    k_pcg_rz<T><<<red_blocks(n), kVecThreads, 0, s>>>(n, r, z, tol, partials, counter, sc, rep,
-                                                      seq);
+    launch_chained(k_pcg_rz<T>, red_blocks(n), kVecThreads, 0, s, n, r, z, tol, partials, counter,
+                   sc, rep, seq);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
     k_pcg_update_p(uint32_t n, const T* __restrict__ z, T* __restrict__ p, const DevScalars* sc) {
+    chain_begin();
     if (skipped(&sc->done)) return;
     const T beta = (T)(sc->rz_new / sc->rz);
 #pragma unroll 4
@@ -1069,7 +1079,7 @@ __global__ void __launch_bounds__(kVecThreads)
 }
 template <typename T>
 void launch_pcg_update_p(uint32_t n, const T* z, T* p, DevScalars* sc, cudaStream_t s) {
-    k_pcg_update_p<T><<<2 * red_blocks(n), kVecThreads, 0, s>>>(n, z, p, sc);
+    launch_chained(k_pcg_update_p<T>, 2 * red_blocks(n), kVecThreads, 0, s, n, z, p, sc);
 }
 
 __global__ void k_set_bc_values(uint32_t n, const uint8_t* __restrict__ mask,

@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(push_max_warps(sizeof(T)) * 32, 1)
                 const T* __restrict__ rhs, T* __restrict__ out, T* __restrict__ fill,
                 uint32_t n_fill, unsigned* __restrict__ status,
                 const unsigned* __restrict__ skip) {
-    if (skipped(skip)) return;  // the same answer in every CTA: nothing writes the word meanwhile
+    chain_let_next();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(16) T zero_slot[4];
     T* slots = reinterpret_cast<T*>(smem_raw);
@@ -272,6 +272,9 @@ __global__ void __launch_bounds__(push_max_warps(sizeof(T)) * 32, 1)
     const uint32_t ns = Lower ? P.nslot_f[g] : P.nslot_b[g];
     for (uint32_t i = threadIdx.x; i < 4 * ns; i += blockDim.x) slots[i] = Sentinel<T>::value();
     cluster_barrier();  // every slot of the cluster holds the sentinel before any push
+    // so far nothing but the plan was read: this much overlaps the kernel before
+    chain_wait();
+    if (skipped(skip)) return;  // the same answer in every CTA: nothing writes the word meanwhile
 
     const uint32_t base = smem_u32(slots);
     const int lane = threadIdx.x & 31, hl = lane & 15;
@@ -392,13 +395,15 @@ static cudaError_t launch_dir(const PushSolve& P, const NodeSched& S, const T* l
     cfg.blockDim = dim3(32 * (sizeof(T) == 4 ? P.warps32 : P.warps64));
     cfg.dynamicSmemBytes = push_smem_bytes(Lower ? P.max_slot_f : P.max_slot_b, sizeof(T));
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = P.cluster;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // chain_wait in the kernel
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, k_trsv_push<T, Lower>, P, S, lu, dinv, rhs, out, fill, n_fill,
                               status, skip);
 }

@@ -91,6 +91,7 @@ template <int M, int D, int Threads>
 __global__ void __launch_bounds__(Threads, 1)
     k_trsv_small(SmallTri L, SmallTri U, uint32_t n, const double* __restrict__ r,
                  double* __restrict__ out, const unsigned* __restrict__ skip) {
+    chain_begin();
     if (skipped(skip)) return;
     extern __shared__ __align__(16) unsigned char small_smem[];
     double* z = reinterpret_cast<double*>(small_smem);
@@ -134,8 +135,7 @@ cudaError_t launch_t(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t 
     // barrier) or than the copies in and out can use
     const unsigned th =
         std::min<unsigned>(Threads, std::max(32u, (std::max(width, n / 64) + 31u) & ~31u));
-    k_trsv_small<M, D, Threads><<<1, th, smem, s>>>(L, U, n, r, out, skip);
-    return cudaGetLastError();
+    return launch_chained(k_trsv_small<M, D, Threads>, 1, th, smem, s, L, U, n, r, out, skip);
 }
 
 }  // namespace
