@@ -599,6 +599,15 @@ int precond_nodes(fm_ctx* c, const T* lu, const T* dinv, const T* r, T* tmp, T* 
     return 4;
 }
 
+// y = K x on the context's K (dot: also x.y)
+template <typename T>
+void spmv_nodes(fm_ctx* c, const T* K, const T* x, T* y, double* dot,
+                const unsigned* skip = nullptr) {
+    fm::launch_spmv_nodes<T>(c->nn, c->graph.max_deg, c->nbr_ptr.p, c->nbr.p, K, x, y,
+                             reinterpret_cast<T*>(c->partials.p), c->counter(), dot, c->status(),
+                             c->stream, skip);
+}
+
 // A linear operator for PCG: the mesh K (node-block SpMV) or a generic CSR.
 template <typename T>
 struct Op {
@@ -621,8 +630,7 @@ struct Op {
         PROF(FM_PROF_SPMV, 1);
         T* part = reinterpret_cast<T*>(c->partials.p);
         if (node_block)
-            fm::launch_spmv_nodes<T>(c->nn, c->nbr_ptr.p, c->nbr.p, K, x, y, part, c->counter(),
-                                     dot, c->stream, skip);
+            spmv_nodes<T>(c, K, x, y, dot, skip);
         else
             fm::launch_spmv_csr<T>(S->n, S->nnz, S->rp.p, S->ci.p, K, x, y, part, c->counter(),
                                    dot, c->stream, skip);
@@ -774,7 +782,7 @@ fm_status need_material(fm_ctx* c) {
 template <typename T>
 fm_status ensure_matrix(fm_ctx* c) {
     Work<T>& w = work<T>(c);
-    CK(w.K.reserve(c->nnz));
+    CK(w.K.reserve(c->nnz + 4));  // room for 16-byte copies of its last entries
     CK(w.LU.reserve(c->nnz));
     CK(w.diag.reserve(c->n));
     CK(w.dinv.reserve(c->n));
@@ -1521,9 +1529,7 @@ fm_status fm_newton_step_cfg(fm_ctx* c, double* u, double load_frac, const fm_ne
                 float* part = reinterpret_cast<float*>(c->partials.p);
                 {
                     PROF(FM_PROF_SPMV, 1);
-                    fm::launch_spmv_nodes<float>(c->nn, c->nbr_ptr.p, c->nbr.p, c->w32.K.p,
-                                                 c->w32.x.p, c->w32.Ap.p, nullptr, nullptr,
-                                                 nullptr, c->stream);
+                    spmv_nodes<float>(c, c->w32.K.p, c->w32.x.p, c->w32.Ap.p, nullptr);
                 }
                 {
                     PROF(FM_PROF_VECTOR, 2);
@@ -1591,16 +1597,13 @@ fm_status fm_newton_step_cfg(fm_ctx* c, double* u, double load_frac, const fm_ne
             double* f = c->vec_c.p;
             if (mixed) {
                 { PROF(FM_PROF_ASSEMBLE, 1); fm::launch_assemble(m, u, c->w32.K.p, f, nullptr, 0, c->status(), c->stream); }
-                { PROF(FM_PROF_SPMV, 1); fm::launch_spmv_nodes<float>(c->nn, c->nbr_ptr.p, c->nbr.p, c->w32.K.p,
-                                             c->w32.b.p, c->w32.Ap.p, nullptr, nullptr, nullptr,
-                                             c->stream); }
+                { PROF(FM_PROF_SPMV, 1); spmv_nodes<float>(c, c->w32.K.p, c->w32.b.p, c->w32.Ap.p, nullptr); }
                 { PROF(FM_PROF_VECTOR, 1); fm::launch_predictor_rhs<float>(c->n, c->mask.p, f, c->w32.Ap.p, R, c->stream); }
                 { PROF(FM_PROF_VECTOR, 1); fm::launch_apply_bc_nodes<float>(c->nn, c->nbr_ptr.p, c->nbr.p, c->mask.p,
                                                  c->w32.K.p, c->stream); }
             } else {
                 { PROF(FM_PROF_ASSEMBLE, 1); fm::launch_assemble(m, u, c->w64.K.p, f, nullptr, 0, c->status(), c->stream); }
-                { PROF(FM_PROF_SPMV, 1); fm::launch_spmv_nodes<double>(c->nn, c->nbr_ptr.p, c->nbr.p, c->w64.K.p, v,
-                                              c->w64.Ap.p, nullptr, nullptr, nullptr, c->stream); }
+                { PROF(FM_PROF_SPMV, 1); spmv_nodes<double>(c, c->w64.K.p, v, c->w64.Ap.p, nullptr); }
                 { PROF(FM_PROF_VECTOR, 1); fm::launch_predictor_rhs<double>(c->n, c->mask.p, f, c->w64.Ap.p, R, c->stream); }
                 { PROF(FM_PROF_VECTOR, 1); fm::launch_apply_bc_nodes<double>(c->nn, c->nbr_ptr.p, c->nbr.p, c->mask.p,
                                                   c->w64.K.p, c->stream); }

@@ -593,60 +593,6 @@ void launch_assemble_slotmap(const MeshDev& m, const double* u, const int32_t* s
 // ===========================================================================
 constexpr int kSpmvBlocks = 148 * 8;
 
-template <typename T>
-__global__ void __launch_bounds__(256)
-    k_spmv_nodes(uint32_t nn, const uint32_t* __restrict__ nbr_ptr,
-                 const uint32_t* __restrict__ nbr, const T* __restrict__ val,
-                 const T* __restrict__ x, T* __restrict__ y, T* partials, unsigned* counter,
-                 double* dot, const unsigned* __restrict__ skip) {
-    chain_begin();
-    if (skipped(skip)) return;
-    const int lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    T dsum = T(0);
-    for (uint32_t n = warp; n < nn; n += nwarps) {
-        const uint32_t nb0 = nbr_ptr[n];
-        const int deg = (int)(nbr_ptr[n + 1] - nb0);
-        const uint32_t my_nbr = lane < deg ? __ldg(nbr + nb0 + lane) : 0u;
-        const T* v = val + 9 * (size_t)nb0;
-        const int rl = 3 * deg;
-        T s[3] = {T(0), T(0), T(0)};
-        for (int i0 = 0; i0 < rl; i0 += 32) {
-            const int idx = i0 + lane;
-            const int k = idx < rl ? idx / 3 : 0;
-            const uint32_t cn = __shfl_sync(kFull, my_nbr, k);
-            if (idx < rl) {
-                const T xv = __ldg(x + 3 * (size_t)cn + (idx - 3 * k));
-#pragma unroll
-                for (int p = 0; p < 3; ++p) s[p] += __ldg(v + (size_t)p * rl + idx) * xv;
-            }
-        }
-#pragma unroll
-        for (int p = 0; p < 3; ++p) s[p] = warp_sum(s[p]);
-        if (lane < 3) {
-            const T yv = lane == 0 ? s[0] : (lane == 1 ? s[1] : s[2]);
-            y[3 * (size_t)n + lane] = yv;
-            if (dot) dsum += yv * x[3 * (size_t)n + lane];
-        }
-    }
-    if (dot) {
-        __shared__ T sbuf[32];
-        const T bt = block_sum(dsum, sbuf);
-        grid_reduce_finish<T>(bt, partials, counter, [&](T total) { *dot = (double)total; });
-    }
-}
-
-template <typename T>
-void launch_spmv_nodes(uint32_t n_nodes, const uint32_t* nbr_ptr, const uint32_t* nbr,
-                       const T* val, const T* x, T* y, T* partials, unsigned* counter,
-                       double* dot, cudaStream_t s, const unsigned* skip) {
-    // no blocks without a node: each would still take its turn at the counter
-    const int grid = (int)std::min<uint32_t>(kSpmvBlocks, std::max(1u, (n_nodes + 7) / 8));
-    launch_chained(k_spmv_nodes<T>, grid, 256, 0, s, n_nodes, nbr_ptr, nbr, val, x, y, partials,
-                   counter, dot, skip);
-}
-
 // G lanes per row (a power of two near the mean row length: a warp per
 // five-entry row leaves 27 of its lanes idle)
 template <typename T, int G>
@@ -1252,9 +1198,6 @@ template void launch_apply_bc_nodes<double>(uint32_t, const uint32_t*, const uin
 template void launch_apply_bc_nodes<float>(uint32_t, const uint32_t*, const uint32_t*,
                                            const uint8_t*, float*, cudaStream_t);
 #define FM_INST(T)                                                                              \
-    template void launch_spmv_nodes<T>(uint32_t, const uint32_t*, const uint32_t*, const T*,    \
-                                       const T*, T*, T*, unsigned*, double*, cudaStream_t,      \
-                                       const unsigned*);                                        \
     template void launch_spmv_csr<T>(uint32_t, uint64_t, const uint32_t*, const uint32_t*,      \
                                      const T*, const T*, T*, T*, unsigned*, double*,            \
                                      cudaStream_t, const unsigned*);                            \

@@ -61,14 +61,16 @@ void launch_assemble_slotmap(const MeshDev& m, const double* u, const int32_t* s
 void launch_elements(uint32_t n, const double* x, const double* u, const double* E, double nu,
                      double* K, double* f, unsigned* status, cudaStream_t s);
 
-// SpMV on the node-block solve pattern (y = A x); with dot != null also
-// finishes dot(x, y) into *dot through the deterministic grid reduction.
-// skip (here and below; null: never): a device word that, when set, makes the
-// kernel return at once.
+// SpMV on the node-block solve pattern (y = A x; fm_spmv.cu); with dot !=
+// null also finishes dot(x, y) into *dot through the deterministic grid
+// reduction.  val and nbr must have 16 bytes of room past their end, nbr_ptr
+// 80.  skip (here and below; null: never): a device word that, when set,
+// makes the kernel return at once.
 template <typename T>
-void launch_spmv_nodes(uint32_t n_nodes, const uint32_t* nbr_ptr, const uint32_t* nbr,
-                       const T* val, const T* x, T* y, T* partials, unsigned* counter,
-                       double* dot, cudaStream_t s, const unsigned* skip = nullptr);
+void launch_spmv_nodes(uint32_t n_nodes, uint32_t max_deg, const uint32_t* nbr_ptr,
+                       const uint32_t* nbr, const T* val, const T* x, T* y, T* partials,
+                       unsigned* counter, double* dot, unsigned* status, cudaStream_t s,
+                       const unsigned* skip = nullptr);
 // Generic scalar CSR SpMV (ascending or any column order)
 template <typename T>
 void launch_spmv_csr(uint32_t n, uint64_t nnz, const uint32_t* rp, const uint32_t* ci,

@@ -365,7 +365,7 @@ cudaError_t build_mesh_device(uint32_t nn, uint32_t ne, const uint4* conn, MeshS
     // node graph: degrees, offsets, sorted unique neighbour sets
     k_graph_degree<<<blocks_for(nn, kSetupWarps), kSetupWarps * 32, 0, s>>>(
         nn, conn, d.inc_ptr->p, d.inc_e->p, cnt.p, scal.p + 1);
-    SCK(d.nbr_ptr->reserve((size_t)nn + 1));
+    SCK(d.nbr_ptr->reserve((size_t)nn + 1 + 20));  // room for whole tiles of the streamed product
     SCK(exclusive_scan(cnt.p, d.nbr_ptr->p, nn, tmp, s));
     uint32_t total = 0;
     SCK(cudaMemcpyAsync(&total, d.nbr_ptr->p + nn, sizeof total, cudaMemcpyDeviceToHost, s));
@@ -376,7 +376,7 @@ cudaError_t build_mesh_device(uint32_t nn, uint32_t ne, const uint4* conn, MeshS
         *result = kSetupLimits;
         return cudaSuccess;
     }
-    SCK(d.nbr->reserve(std::max<uint32_t>(total, 1)));
+    SCK(d.nbr->reserve((size_t)total + 4));  // room for 16-byte copies of its last entries
     SCK(d.self_pos->reserve(std::max<uint32_t>(nn, 1)));
     SCK(cudaMemsetAsync(d.self_pos->p, 0, (size_t)nn * sizeof(uint32_t), s));
     k_graph_fill<<<blocks_for(nn, kSetupWarps), kSetupWarps * 32, 0, s>>>(
