@@ -400,10 +400,16 @@ static cudaError_t launch_dir(const PushSolve& P, const NodeSched& S, const T* l
     at[0].val.clusterDim.x = P.cluster;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // chain_wait in the kernel
+    // Started early (chain_wait in the kernel), the backward solve's clusters
+    // take their SMs as the forward's leave.  The forward solve follows short
+    // kernels that fill the device: there an early start pays only where the
+    // clusters leave most SMs free (8^3 load step 150.6 -> 145.0 ms); with all
+    // of them it delays the clusters that wait for a whole GPC's SMs (64^3
+    // load step 650 -> 722 ms, 48^3 PCG 95.6 -> 98.9 ms).
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = !Lower || 2 * P.n_ctas <= 148 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, k_trsv_push<T, Lower>, P, S, lu, dinv, rhs, out, fill, n_fill,
                               status, skip);
 }
