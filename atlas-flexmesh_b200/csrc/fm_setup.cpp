@@ -195,13 +195,15 @@ bool push_plan(const NodeGraph& g, const std::vector<uint32_t>& fwd_ptr,
         for (uint32_t t = fwd_ptr[l]; t < fwd_ptr[l + 1]; ++t) lf[fwd_order[t]] = l;
     for (uint32_t l = 0; l < nlb; ++l)
         for (uint32_t t = bwd_ptr[l]; t < bwd_ptr[l + 1]; ++t) lb[bwd_order[t]] = l;
-    // busiest CTA's share of one level, either direction
+    // busiest CTA's share of one level, either direction; counting stops once
+    // it exceeds `bound` (the block cannot be the best then: most candidates
+    // end early, which halves the search)
     std::vector<uint32_t> cf((size_t)nc * nlf), cb((size_t)nc * nlb);
-    auto share = [&](uint32_t R) {
+    auto share = [&](uint32_t R, uint32_t bound) {
         std::fill(cf.begin(), cf.end(), 0u);
         std::fill(cb.begin(), cb.end(), 0u);
         uint32_t mx = 0;
-        for (uint32_t n = 0; n < nn; ++n) {
+        for (uint32_t n = 0; n < nn && mx <= bound; ++n) {
             const uint32_t c = push_cta(n, nn, n_clusters, cluster, R);
             mx = std::max(mx, ++cf[(size_t)c * nlf + lf[n]]);
             mx = std::max(mx, ++cb[(size_t)c * nlb + lb[n]]);
@@ -209,10 +211,17 @@ bool push_plan(const NodeGraph& g, const std::vector<uint32_t>& fwd_ptr,
         return mx;
     };
     std::vector<std::pair<uint32_t, uint32_t>> cand;  // (share, block)
+    std::vector<uint32_t> rest;  // blocks whose count was cut short
     if (block) {
-        cand.push_back({share(block), block});
+        cand.push_back({share(block, ~0u), block});
     } else {
-        for (uint32_t R = 16; R <= 512; R += R < 128 ? 1 : 8) cand.push_back({share(R), R});
+        uint32_t best = ~0u;
+        for (uint32_t R = 16; R <= 512; R += R < 128 ? 1 : 8) {
+            const uint32_t sh = share(R, best);
+            if (sh > best) rest.push_back(R);
+            else cand.push_back({sh, R});
+            best = std::min(best, sh);
+        }
         std::sort(cand.begin(), cand.end());
     }
     std::vector<uint32_t> cta(nn);
@@ -248,7 +257,15 @@ bool push_plan(const NodeGraph& g, const std::vector<uint32_t>& fwd_ptr,
         max_slot = *std::max_element(nslot.begin(), nslot.end());
         return true;
     };
-    for (const auto& cs : cand) {
+    for (size_t at = 0; at < cand.size() || !rest.empty(); ++at) {
+        if (at == 1 && !rest.empty()) {
+            // the best block's slots do not fit: the others in order of their
+            // full counts
+            for (uint32_t R : rest) cand.push_back({share(R, ~0u), R});
+            rest.clear();
+            std::sort(cand.begin() + 1, cand.end());
+        }
+        const std::pair<uint32_t, uint32_t> cs = cand[at];
         const uint32_t R = cs.second;
         for (uint32_t n = 0; n < nn; ++n) cta[n] = push_cta(n, nn, n_clusters, cluster, R);
         plan.src.assign(g.nbr.size(), ~0u);
