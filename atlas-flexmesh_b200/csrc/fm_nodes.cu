@@ -247,34 +247,45 @@ __global__ void __launch_bounds__(kNodeWarps * 32, sizeof(T) == 4 ? 3 : 2)
                     val[r][3 * q + c] = fast && fpos[r] != 0xffu && fjb[r] + c > flim[r] + q
                                             ? ld_relaxed(fsrc[r] + (size_t)q * fmrl[r] + c)
                                             : T(0);
-        auto pending = [&]() {
-            bool p = Sentinel<T>::is(dv0) | Sentinel<T>::is(dv1) | Sentinel<T>::is(dv2);
+        auto pending_round = [&](int r) {
+            bool p = false;
 #pragma unroll
-            for (int r = 0; r < kPairRound; ++r)
-#pragma unroll
-                for (int k = 0; k < 9; ++k) p |= Sentinel<T>::is(val[r][k]);
+            for (int k = 0; k < 9; ++k) p |= Sentinel<T>::is(val[r][k]);
             return p;
         };
         bool ok = true;
-        bool need = pending();
-        if (__any_sync(kFull, need)) {
+        bool dneed = Sentinel<T>::is(dv0) | Sentinel<T>::is(dv1) | Sentinel<T>::is(dv2);
+        bool need[kPairRound];
+        bool any = dneed;
+#pragma unroll
+        for (int r = 0; r < kPairRound; ++r) any |= need[r] = pending_round(r);
+        if (__any_sync(kFull, any)) {
             const long long t0 = clock64(), limit = wait_limit(status);
             for (unsigned it = 1;; ++it) {
-                if (need) {
-                    if (Sentinel<T>::is(dv0)) dv0 = ld_relaxed(dsrc);
-                    if (Sentinel<T>::is(dv1)) dv1 = ld_relaxed(dsrc + 1);
-                    if (Sentinel<T>::is(dv2)) dv2 = ld_relaxed(dsrc + 2);
-#pragma unroll
-                    for (int r = 0; r < kPairRound; ++r)
-#pragma unroll
-                        for (int q = 0; q < 3; ++q)
-#pragma unroll
-                            for (int c = 0; c < 3; ++c)
-                                if (Sentinel<T>::is(val[r][3 * q + c]))
-                                    val[r][3 * q + c] = ld_relaxed(fsrc[r] + (size_t)q * fmrl[r] + c);
-                    need = pending();
+                if (dneed) {
+                    dv0 = ld_relaxed(dsrc);
+                    dv1 = ld_relaxed(dsrc + 1);
+                    dv2 = ld_relaxed(dsrc + 2);
                 }
-                if (!__any_sync(kFull, need)) break;
+                // whole rounds without a pending pair are passed over, and a
+                // pending pair is read again as a whole
+#pragma unroll
+                for (int r = 0; r < kPairRound; ++r)
+                    if (__any_sync(kFull, need[r])) {
+                        if (need[r]) {
+#pragma unroll
+                            for (int q = 0; q < 3; ++q)
+#pragma unroll
+                                for (int c = 0; c < 3; ++c)
+                                    if (fjb[r] + c > flim[r] + q)
+                                        val[r][3 * q + c] =
+                                            ld_relaxed(fsrc[r] + (size_t)q * fmrl[r] + c);
+                        }
+                    }
+                any = dneed = Sentinel<T>::is(dv0) | Sentinel<T>::is(dv1) | Sentinel<T>::is(dv2);
+#pragma unroll
+                for (int r = 0; r < kPairRound; ++r) any |= need[r] = pending_round(r);
+                if (!__any_sync(kFull, any)) break;
                 if ((it & 31u) == 0 &&
                     __any_sync(kFull, (ld_volatile_u32(status) & FM_FLAG_TIMEOUT) ||
                                           clock64() - t0 > limit)) {
@@ -360,7 +371,7 @@ __global__ void __launch_bounds__(kNodeWarps * 32, sizeof(T) == 4 ? 3 : 2)
             __syncwarp();  // before the next chunk overwrites G.u
         }
         // the node's own 3x3 block: columns 3n and 3n+1 eliminate rows below
-        T piv[3];
+        T piv[3], rcp[3];
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
             const int c = ds + p, owner = c & 31, sl = c >> 5;
@@ -370,33 +381,41 @@ __global__ void __launch_bounds__(kNodeWarps * 32, sizeof(T) == 4 ? 3 : 2)
                 if (lane == 0) raise_flag(status, FM_FLAG_PIVOT);
             }
             piv[p] = u;
+            rcp[p] = T(1) / u;
 #pragma unroll
             for (int r2 = p + 1; r2 < 3; ++r2) {
-                const T l = __shfl_sync(kFull, pick3(w[r2], sl), owner) / u;
+                const T l = __shfl_sync(kFull, pick3(w[r2], sl), owner) * rcp[p];
                 if (lane == 0) G.lm[r2][c] = l;
                 // columns left of c only hold values write-back replaces
 #pragma unroll
                 for (int s = 0; s < 3; ++s) w[r2][s] = w[r2][s] - l * w[p][s];
             }
         }
-        // write back: multipliers left of the diagonal, a_ii on the diagonal
-        // slot (the pivots go to dg), U right of it
+        // write back, what the readers wait for first: the reciprocal pivots and
+        // U right of the diagonal; then a_ii on the diagonal slot (the pivots
+        // go to dg) and the multipliers left of it
         __syncwarp();
         T* out = lu + 9 * (size_t)nb0;
+        if (lane < 3) dinv[3 * (size_t)n + lane] = pick3(rcp, lane);
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                const int j = lane + 32 * s;
+                if (j < rl && j > ds + p) out[(size_t)p * rl + j] = w[p][s];
+            }
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
             const T ap = __shfl_sync(kFull, adiag, p);
 #pragma unroll
             for (int s = 0; s < 3; ++s) {
                 const int j = lane + 32 * s;
-                if (j < rl)
-                    out[(size_t)p * rl + j] = j < ds + p ? G.lm[p][j] : j == ds + p ? ap : w[p][s];
+                if (j < rl && j <= ds + p) out[(size_t)p * rl + j] = j == ds + p ? ap : G.lm[p][j];
             }
         }
         if (lane < 3) {
             const T pv = pick3(piv, lane);
             dg[3 * (size_t)n + lane] = pv;
-            dinv[3 * (size_t)n + lane] = T(1) / pv;
             if (!isfinite((double)pv)) raise_flag(status, FM_FLAG_NONFINITE);
         }
     }
