@@ -43,8 +43,7 @@ __global__ void k_fill_sentinel(uint32_t n, T* __restrict__ x) {
 // The node's three rows live in registers (lane owns columns lane,
 // lane+32, lane+64).  The U parts of every lower neighbour's rows are
 // loaded in one round of independent loads, re-read while any still holds
-// the sentinel (at 64^3: 1.83 ms per FP32 factorization and 2.40 ms FP64,
-// against 2.00 and 2.65 ms with a per-node release flag), and staged into
+// the sentinel (at 64^3: 1.48 ms per FP32 factorization and 1.99 ms FP64), and staged into
 // shared memory, already scattered to the node's own column positions through a
 // structural map built on the host (ilu_edge_maps): a dense row per
 // (neighbour, row q), zero where the neighbour has no entry.  Each
@@ -79,7 +78,7 @@ __device__ __forceinline__ T pick3(const T v[3], int s) {
 // neighbour's pattern are staged as zeros: x - l 0 = x.  The multipliers go
 // to G.lm; the pivot columns in w are not read again (write-back takes G.lm
 // for every column left of the diagonal), so the updates need no selects.
-template <typename T>
+template <typename T, int Slots = 3>
 __device__ __forceinline__ void ilu_step(IluStage<T>& G, T (&w)[3][3], int k, int k0, int rs,
                                          int nsl, int lane, T dv0, T dv1, T dv2) {
     const T d0 = __shfl_sync(kFull, dv0, k), d1 = __shfl_sync(kFull, dv1, k),
@@ -100,14 +99,13 @@ __device__ __forceinline__ void ilu_step(IluStage<T>& G, T (&w)[3][3], int k, in
         l[p][1] = (wq[1] - l[p][0] * u01) * d1;
         l[p][2] = ((wq[2] - l[p][0] * u02) - l[p][1] * u12) * d2;
     }
-    if (lane == 0)
 #pragma unroll
-        for (int p = 0; p < 3; ++p)
+    for (int p = 0; p < 3; ++p)
 #pragma unroll
-            for (int q = 0; q < 3; ++q) G.lm[p][c0 + q] = l[p][q];
+        for (int q = 0; q < 3; ++q) G.lm[p][c0 + q] = l[p][q];
 #pragma unroll
-    for (int s = 0; s < 3; ++s) {
-        if (s < nsl) {
+    for (int s = 0; s < Slots; ++s) {
+        if (Slots < 3 || s < nsl) {
             const int j = lane + 32 * s;
             const T a0 = ur0[j], a1 = ur1[j], a2 = ur2[j];
 #pragma unroll
@@ -307,9 +305,23 @@ __global__ void __launch_bounds__(kNodeWarps * 32, sizeof(T) == 4 ? 3 : 2)
                         for (int c = 0; c < 3; ++c) G.u[d + q * rs + c] = val[r][3 * q + c];
                 }
             __syncwarp();
+            if (sk == kStageNbrs && nsl == 2) {
+                // every step taken, two column slots, one code path: without
+                // branches between (or in) the steps the next pivot columns'
+                // shuffles overlap this step's updates (31^3 FP64 774 -> 632
+                // us, 64^3 FP32 1698 -> 1480 us).  In FP64 a fence every other
+                // step keeps later steps' stage reads from being hoisted into
+                // more registers than there are (48 bytes of spills without).
 #pragma unroll
-            for (int k = 0; k < kStageNbrs; ++k)
-                if (k < sk) ilu_step(G, w, k, 0, rs, nsl, lane, dv0, dv1, dv2);
+                for (int k = 0; k < kStageNbrs; ++k) {
+                    ilu_step<T, 2>(G, w, k, 0, 64, 2, lane, dv0, dv1, dv2);
+                    if (sizeof(T) == 8 && k % 2 == 1) __syncwarp();
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < kStageNbrs; ++k)
+                    if (k < sk) ilu_step(G, w, k, 0, rs, nsl, lane, dv0, dv1, dv2);
+            }
             __syncwarp();
         }
         for (int k0 = 0; ok && !fast && k0 < sk; k0 += cap_k) {
