@@ -119,8 +119,9 @@ struct fm_ctx {
     DevBuf<double> ke_scratch;
     DevBuf<double> fvert;            // element pass: vertex forces
     DevBuf<unsigned char> tan_rec;   // element pass: tangent records
-    DevBuf<uint32_t> act_ptr, act_v, act_pos, nbr_members;  // node-pass scatter structure
-    uint32_t max_pairs = 96;
+    DevBuf<uint32_t> act_ptr, act_v;  // node-pass scatter structure
+    DevBuf<uint16_t> edge, pair_off;
+    int pair_lane = 33;
 
     // solver state
     Work<double> w64;
@@ -311,9 +312,9 @@ fm::MeshDev mesh_view(const fm_ctx* c) {
     m.tan_rec = c->tan_rec.p;
     m.act_ptr = c->act_ptr.p;
     m.act_v = c->act_v.p;
-    m.act_pos = c->act_pos.p;
-    m.nbr_members = c->nbr_members.p;
-    m.max_pairs = c->max_pairs;
+    m.edge = c->edge.p;
+    m.pair_off = c->pair_off.p;
+    m.pair_lane = c->pair_lane;
     return m;
 }
 
@@ -1024,7 +1025,7 @@ fm_status fm_set_mesh(fm_ctx* c, uint32_t n_nodes, const double* xyz, uint32_t n
         fm::MeshSetupDev md{&c->inc_ptr,      &c->inc_e,    &c->nbr_ptr,  &c->nbr,
                             &c->self_pos,     &c->node_fwd, &c->node_bwd, &c->node_fwd_rec,
                             &c->node_bwd_rec, &c->emap_ptr, &c->emap,     &c->act_ptr,
-                            &c->act_v,        &c->act_pos,  &c->nbr_members};
+                            &c->act_v,        &c->edge,     &c->pair_off};
         fm::MeshSetupHost mh;
         int res = fm::kSetupOk;
         CK(fm::build_mesh_device(n_nodes, n_elems, c->conn.p, md, mh, c->status(), &res,
@@ -1070,7 +1071,7 @@ fm_status fm_set_mesh(fm_ctx* c, uint32_t n_nodes, const double* xyz, uint32_t n
         c->ref_slot.release();
         CK(c->vec_a.reserve(c->n));
         CK(c->vec_b.reserve(c->n));
-        c->max_pairs = std::max(32u, 3 * mh.max_act);
+        c->pair_lane = mh.pair_lane();
         CK(c->fvert.reserve(12 * (size_t)c->ne));
         CK(c->tan_rec.reserve((size_t)c->ne * fm::kTanRecBytes));
         CK(cudaStreamSynchronize(c->stream));

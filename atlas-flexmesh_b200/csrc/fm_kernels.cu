@@ -23,7 +23,14 @@ namespace fm {
 // ===========================================================================
 // Assembly
 // ===========================================================================
-constexpr int kAsmWarps = 8;
+// warps per CTA of the node pass: FP64 takes 96 registers, so that 20 warps
+// are resident in five CTAs of four (at 80 for 24 it spills: 478 against 420
+// us at 64^3), FP32 64 for 32 (four CTAs of eight; 40 warps at 48 registers
+// spill: 352 against 311)
+template <typename KT>
+constexpr int kAsmWarps = sizeof(KT) == 4 ? 8 : 4;
+template <typename KT>
+constexpr int kAsmCtas = sizeof(KT) == 4 ? 4 : 5;
 
 // The element pass leaves per tet the 12 components of its vertex forces
 // vol M dN_a (fvert, FP64: 96 bytes) and, when a tangent is assembled, a
@@ -186,13 +193,13 @@ void launch_gather_forces(const MeshDev& m, double* f, double* R, cudaStream_t s
                                                                m.fvert, m.mask, f, R);
 }
 
-// gradients of a tet's four vertices and its tangent scalars
-__device__ __forceinline__ void load_tan(const TanRec<double>* p, double D[4][3], double s[3]) {
-    const double2* q = reinterpret_cast<const double2*>(p);
+// gradients of a tet's four vertices and its tangent scalars, from a staged
+// record
+__device__ __forceinline__ void load_tan(const uint4* q, double D[4][3], double s[3]) {
     double w[12];
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-        const double2 v = __ldg(q + i);
+        const double2 v = reinterpret_cast<const double2*>(q)[i];
         w[2 * i] = v.x;
         w[2 * i + 1] = v.y;
     }
@@ -205,12 +212,11 @@ __device__ __forceinline__ void load_tan(const TanRec<double>* p, double D[4][3]
         s[c] = w[9 + c];
     }
 }
-__device__ __forceinline__ void load_tan(const TanRec<float>* p, float D[4][3], float s[3]) {
-    const float4* q = reinterpret_cast<const float4*>(p);
+__device__ __forceinline__ void load_tan(const uint4* q, float D[4][3], float s[3]) {
     float w[16];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const float4 v = __ldg(q + i);
+        const float4 v = reinterpret_cast<const float4*>(q)[i];
         w[4 * i] = v.x;
         w[4 * i + 1] = v.y;
         w[4 * i + 2] = v.z;
@@ -224,173 +230,240 @@ __device__ __forceinline__ void load_tan(const TanRec<float>* p, float D[4][3], 
     }
 }
 
+template <int Bytes>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "n"(Bytes)
+                 : "memory");
+}
+
+// A warp's shared memory in the node pass: the staged records (a 16-byte
+// word more than a record apart: no bank conflicts) give way to the blocks,
+// entry (j, p, q) of tet l at (9 (j - 1) + 3 p + q) PL + l, and those to the
+// three rows.
+template <typename KT, int PL>
+struct __align__(16) AsmWarp {
+    static constexpr int kWords = (int)(sizeof(TanRec<KT>) / 16);
+    union {
+        uint4 rec[(PL - 1) * (kWords + 1)];
+        KT block[27 * PL];
+        KT row[3 * 96];
+    };
+    double f[96];        // owner's forces: component c of tet l at 3 l + c
+    uint16_t pair[96];   // the node's pair offsets
+};
+
 // Node pass: one warp owns node n and writes its three CSR rows once (no
 // atomics, every sum in a fixed order).
-//   1. Lane l takes the node's l-th active tet: loads its record, turns it so
-//      that the owner's gradient comes first, and forms the 3x3 blocks
-//      against the tet's three other vertices.  The blocks go to shared
-//      memory grouped by neighbour: block (l, k) in slot start[k] + (number
-//      of tets before l on the edge to k).
-//   2. Lane c takes column c of the rows (c = 3k + q) and sums the slots of
-//      neighbour k, ascending element order, for the three rows at once.
-//   3. The diagonal block is minus the sum of the row's other blocks.
-// Bound: the L1 data pipe (78% busy at 64^3 FP64: about 340 shared-memory and
-// 120 global wavefronts per node, half of the shared ones bank conflicts of
-// the slot exchange).  One lane per neighbour walking its tets kept 15 of 32
-// lanes busy; this keeps 23 (whole assembly: 128^3 FP64 5.67 -> 4.99 ms, 33^3
-// FP32 88 -> 70 us).
-template <typename KT>
-__global__ void __launch_bounds__(kAsmWarps * 32, sizeof(KT) == 4 ? 4 : 3)
+//   1. The warp copies its active tets' records and the owner's forces to
+//      shared memory, neighbouring lanes copying neighbouring words.
+//   2. Lane l takes the l-th tet: turns its record so that the owner's
+//      gradient comes first, forms the 3x3 blocks against the three other
+//      vertices and leaves them in shared memory, entry by entry with
+//      neighbouring tets in neighbouring words.
+//   3. Lane c takes column c of the rows (c = 3k + q) and sums neighbour k's
+//      blocks through the pair list, ascending element order, for the three
+//      rows at once.
+//   4. The diagonal block is minus the sum of the row's other blocks.
+// The loop over nodes loads the next node's lists meanwhile.  Bound: latency
+// and issue (900 instructions per node; the three dependent loads that start
+// a node and the copies take most of its 7 us unless they overlap the node
+// before: 572 -> 478 us with the copies in flight together, 420 with the lists
+// ahead and no spills, FP64 at 64^3).  One lane per neighbour walking its tets
+// took 605.  Whole assembly: 128^3 FP64 5.67 -> 3.96 ms, 33^3 FP32 88 -> 63 us.
+template <typename KT, int PL>
+__global__ void __launch_bounds__(kAsmWarps<KT> * 32, kAsmCtas<KT>)
     k_assemble(MeshDev m, const TanRec<KT>* __restrict__ tan, KT* __restrict__ K,
                double* __restrict__ f, double* __restrict__ R, int apply_bc) {
     extern __shared__ __align__(16) unsigned char asm_smem[];
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    double* F = reinterpret_cast<double*>(asm_smem) + wi * 96;
-    KT* C = reinterpret_cast<KT*>(asm_smem + kAsmWarps * 96 * sizeof(double)) +
-            (size_t)wi * 9 * m.max_pairs;
-    const uint32_t n = blockIdx.x * kAsmWarps + wi;
-    if (n >= m.n_nodes) return;  // uniform per warp
-    const uint32_t nb0 = m.nbr_ptr[n];
-    const int deg = (int)(m.nbr_ptr[n + 1] - nb0);
-    const uint32_t a0 = m.act_ptr[n];
-    const int ma = (int)(m.act_ptr[n + 1] - a0);
-    const uint32_t v = lane < ma ? __ldg(m.act_v + a0 + lane) : 0u;
-    uint32_t pos = lane < ma ? __ldg(m.act_pos + a0 + lane) : 0xffffffffu;
-    const uint32_t my_nbr = lane < deg ? __ldg(m.nbr + nb0 + lane) : 0xffffffffu;
-    const uint32_t memb = lane < deg ? __ldg(m.nbr_members + nb0 + lane) : 0u;
-    const bool bc = apply_bc && m.mask;
-    uint32_t fixed = 0;  // the neighbour's constrained DOFs, one bit each
-    if (bc && lane < deg) {
-        const uint8_t* q = m.mask + 3 * (size_t)my_nbr;
-        fixed = (q[0] ? 1u : 0u) | (q[1] ? 2u : 0u) | (q[2] ? 4u : 0u);
-    }
-    KT D[4][3], sc[3];
-    double fo[3] = {0.0, 0.0, 0.0};
-    if (lane < ma) {
-        load_tan(tan + (v >> 2), D, sc);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) fo[c] = __ldg(m.fvert + 3 * (size_t)v + c);
-    }
-    const int self_k = __ffs(__ballot_sync(kFull, my_nbr == n)) - 1;
-    const int cnt = __popc(memb);
-    int start = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(kFull, start, o);
-        if (lane >= o) start += t;
-    }
-    start -= cnt;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) F[32 * c + lane] = fo[c];
-    // rotate by the owner's local index: D[0] is its gradient
-    const bool r1 = v & 1u, r2 = v & 2u;
-    pos = __funnelshift_r(pos, pos, 8 * (v & 3u));
-    KT dI[3], hI[3], aI[3], bI[3], mI[3];
-    if (lane < ma) {
-        KT T[4][3];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) T[a][c] = r1 ? D[(a + 1) & 3][c] : D[a][c];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) D[a][c] = r2 ? T[(a + 2) & 3][c] : T[a][c];
-        // K_pq = va dI_p dJ_q (p==q) + vb dI_p dJ_q (p!=q)
-        //      + vm (p==q ? sum_{r!=p} dI_r dJ_r : dI_q dJ_p) + (p==q) fI.dJ
-        // with the products by dI formed once per tet
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            dI[c] = D[0][c];
-            bI[c] = sc[1] * dI[c];
-            mI[c] = sc[2] * dI[c];
-            aI[c] = sc[0] * dI[c] - mI[c];
-            hI[c] = (KT)fo[c] + mI[c];
+    AsmWarp<KT, PL>& S = reinterpret_cast<AsmWarp<KT, PL>*>(asm_smem)[wi];
+    const uint32_t step = gridDim.x * kAsmWarps<KT>;
+    // the node's lists, loaded while the node before is worked on
+    struct Node {
+        uint32_t nb0, a0, v, nbr, edge;
+        int deg, ma;
+    } nx;
+    auto pointers = [&](uint32_t n) {
+        if (n >= m.n_nodes) return;
+        nx.nb0 = __ldg(m.nbr_ptr + n);
+        nx.deg = (int)(__ldg(m.nbr_ptr + n + 1) - nx.nb0);
+        nx.a0 = __ldg(m.act_ptr + n);
+        nx.ma = (int)(__ldg(m.act_ptr + n + 1) - nx.a0);
+    };
+    auto lists = [&](uint32_t n) {
+        if (n >= m.n_nodes) return;
+        nx.v = lane < nx.ma ? __ldg(m.act_v + nx.a0 + lane) : 0u;
+        nx.nbr = lane < nx.deg ? __ldg(m.nbr + nx.nb0 + lane) : 0xffffffffu;
+        nx.edge = lane < nx.deg ? __ldg(m.edge + nx.nb0 + lane) : 0u;
+    };
+    uint32_t n = blockIdx.x * kAsmWarps<KT> + wi;
+    pointers(n);
+    lists(n);
+    for (; n < m.n_nodes; n += step) {  // uniform per warp
+        const uint32_t nb0 = nx.nb0, a0 = nx.a0, v = nx.v, my_nbr = nx.nbr, my_edge = nx.edge;
+        const int deg = nx.deg, ma = nx.ma;
+        const bool bc = apply_bc && m.mask;
+        uint32_t fixed = 0;  // the neighbour's constrained DOFs, one bit each
+        if (bc && lane < deg) {
+            const uint8_t* q = m.mask + 3 * (size_t)my_nbr;
+            fixed = (q[0] ? 1u : 0u) | (q[1] ? 2u : 0u) | (q[2] ? 4u : 0u);
         }
-    }
+        // every copy in flight at once (cp.async: no registers, and no copy waits
+        // for the one before)
+        constexpr int W = AsmWarp<KT, PL>::kWords;
 #pragma unroll
-    for (int j = 1; j < 4; ++j) {
-        const uint32_t k = (pos >> (8 * j)) & 0xffu;  // 0xff: no block there
-        const uint32_t mk = __shfl_sync(kFull, memb, k & 31u);
-        const int st = __shfl_sync(kFull, start, k & 31u);
-        if (k != 0xffu && ((mk >> lane) & 1u)) {
-            KT* o = C + 9 * (st + __popc(mk & ((1u << lane) - 1u)));
-            const KT* dJ = D[j];
-            const KT S = hI[0] * dJ[0] + hI[1] * dJ[1] + hI[2] * dJ[2];
-            o[0] = S + aI[0] * dJ[0];
-            o[1] = bI[0] * dJ[1] + mI[1] * dJ[0];
-            o[2] = bI[0] * dJ[2] + mI[2] * dJ[0];
-            o[3] = bI[1] * dJ[0] + mI[0] * dJ[1];
-            o[4] = S + aI[1] * dJ[1];
-            o[5] = bI[1] * dJ[2] + mI[2] * dJ[1];
-            o[6] = bI[2] * dJ[0] + mI[0] * dJ[2];
-            o[7] = bI[2] * dJ[1] + mI[1] * dJ[2];
-            o[8] = S + aI[2] * dJ[2];
+        for (int i = 0; i < W; ++i) {
+            if (32 * i >= W * ma) break;  // uniform
+            const int t = lane + 32 * i, l = t / W, word = t - W * l;
+            const uint32_t e = __shfl_sync(kFull, v, l & 31) >> 2;
+            if (t < W * ma)
+                copy_async<16>(&S.rec[l * (W + 1) + word],
+                               reinterpret_cast<const uint4*>(tan + e) + word);
         }
-    }
-    __syncwarp();
-    if (lane < 3 && (f || R)) {
-        double s = 0.0;
-        for (int l = 0; l < ma; ++l) s += F[32 * lane + l];
-        const uint32_t row = 3 * n + lane;
-        if (f) f[row] = s;
-        if (R) R[row] = (m.mask && m.mask[row]) ? 0.0 : -s;
-    }
-    const int rl = 3 * deg;
-    KT acc[3][3];
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        acc[r][0] = acc[r][1] = acc[r][2] = KT(0);
-        if (32 * r < rl) {  // uniform
-            const int c = lane + 32 * r, k = c / 3;
-            const int st = __shfl_sync(kFull, start, k & 31), ck = __shfl_sync(kFull, cnt, k & 31);
-            if (c < rl) {
-                const KT* q = C + 9 * st + (c - 3 * k);
-                for (int i = 0; i < ck; ++i, q += 9) {
-                    acc[r][0] += q[0];
-                    acc[r][1] += q[3];
-                    acc[r][2] += q[6];
+        for (int i = 0; i < 3; ++i) {
+            if (32 * i >= 3 * ma) break;
+            const int t = lane + 32 * i, l = t / 3;
+            const uint32_t vl = __shfl_sync(kFull, v, l & 31);
+            if (t < 3 * ma) copy_async<8>(&S.f[t], m.fvert + 3 * (size_t)vl + (t - 3 * l));
+        }
+        uint16_t pr[3] = {0, 0, 0};
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            if (lane + 32 * i < 3 * ma) pr[i] = __ldg(m.pair_off + 3 * (size_t)a0 + lane + 32 * i);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) S.pair[lane + 32 * i] = pr[i];
+        pointers(n + step);
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+        const int self_k = __ffs(__ballot_sync(kFull, my_nbr == n)) - 1;
+        __syncwarp();
+        KT D[4][3], sc[3];
+        if (lane < ma) load_tan(S.rec + lane * (W + 1), D, sc);
+        lists(n + step);
+        __syncwarp();  // the records are in registers: their place is the blocks'
+        if (lane < ma) {
+            // rotate by the owner's local index: D[0] is its gradient
+            const bool r1 = v & 1u, r2 = v & 2u;
+            KT T[4][3], dI[3], hI[3], aI[3], bI[3], mI[3];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) T[a][c] = r1 ? D[(a + 1) & 3][c] : D[a][c];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) D[a][c] = r2 ? T[(a + 2) & 3][c] : T[a][c];
+            // K_pq = va dI_p dJ_q (p==q) + vb dI_p dJ_q (p!=q)
+            //      + vm (p==q ? sum_{r!=p} dI_r dJ_r : dI_q dJ_p) + (p==q) fI.dJ
+            // with the products by dI formed once per tet
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                dI[c] = D[0][c];
+                bI[c] = sc[1] * dI[c];
+                mI[c] = sc[2] * dI[c];
+                aI[c] = sc[0] * dI[c] - mI[c];
+                hI[c] = (KT)S.f[3 * lane + c] + mI[c];
+            }
+#pragma unroll
+            for (int j = 1; j < 4; ++j) {
+                KT* o = S.block + (j - 1) * 9 * PL + lane;
+                const KT* dJ = D[j];
+                const KT h = hI[0] * dJ[0] + hI[1] * dJ[1] + hI[2] * dJ[2];
+                o[0 * PL] = h + aI[0] * dJ[0];
+                o[1 * PL] = bI[0] * dJ[1] + mI[1] * dJ[0];
+                o[2 * PL] = bI[0] * dJ[2] + mI[2] * dJ[0];
+                o[3 * PL] = bI[1] * dJ[0] + mI[0] * dJ[1];
+                o[4 * PL] = h + aI[1] * dJ[1];
+                o[5 * PL] = bI[1] * dJ[2] + mI[2] * dJ[1];
+                o[6 * PL] = bI[2] * dJ[0] + mI[0] * dJ[2];
+                o[7 * PL] = bI[2] * dJ[1] + mI[1] * dJ[2];
+                o[8 * PL] = h + aI[2] * dJ[2];
+            }
+        }
+        __syncwarp();
+        if (lane < 3 && (f || R)) {
+            double s = 0.0;
+            for (int l = 0; l < ma; ++l) s += S.f[3 * l + lane];
+            const uint32_t row = 3 * n + lane;
+            if (f) f[row] = s;
+            if (R) R[row] = (m.mask && m.mask[row]) ? 0.0 : -s;
+        }
+        const int rl = 3 * deg;
+        KT acc[3][3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            acc[r][0] = acc[r][1] = acc[r][2] = KT(0);
+            if (32 * r < rl) {  // uniform
+                const int c = lane + 32 * r, k = c / 3;
+                const uint32_t ed = __shfl_sync(kFull, my_edge, k & 31);
+                if (c < rl) {
+                    const KT* base = S.block + (c - 3 * k) * PL;
+                    const uint16_t* pr = S.pair + (ed & 0xffu);
+                    for (uint32_t i = ed >> 8; i; --i, ++pr) {
+                        const KT* q = base + *pr;
+                        acc[r][0] += q[0];
+                        acc[r][1] += q[3 * PL];
+                        acc[r][2] += q[6 * PL];
+                    }
                 }
             }
         }
-    }
-    __syncwarp();  // the slots are read: reuse them for the rows
+        __syncwarp();  // the blocks are read: their place is the rows'
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        const int c = lane + 32 * r;
-        if (c < rl)
-#pragma unroll
-            for (int p = 0; p < 3; ++p) C[p * rl + c] = acc[r][p];
-    }
-    __syncwarp();
-    // diagonal block: lane (third, p, q) sums entry (p, q) of every third
-    // neighbour, then the thirds are added
-    {
-        const int third = lane / 9, pq = lane - 9 * third, p = pq / 3, q = pq - 3 * p;
-        KT s = KT(0);
-        if (lane < 27)
-            for (int k = third; k < deg; k += 3) s += C[p * rl + 3 * k + q];
-        const KT s1 = __shfl_sync(kFull, s, pq + 9), s2 = __shfl_sync(kFull, s, (pq + 18) & 31);
-        if (lane < 9 && deg) C[p * rl + 3 * self_k + q] = -(s + s1 + s2);
-    }
-    __syncwarp();
-    KT* out = K + 9 * (size_t)nb0;
-    const uint32_t fixed_row = __shfl_sync(kFull, fixed, self_k & 31);
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        if (32 * r < rl) {  // uniform
-            const int c = lane + 32 * r, k = c / 3, q = c - 3 * k;
-            const uint32_t fc = (__shfl_sync(kFull, fixed, k & 31) >> q) & 1u;
+        for (int r = 0; r < 3; ++r) {
+            const int c = lane + 32 * r;
             if (c < rl)
 #pragma unroll
-                for (int p = 0; p < 3; ++p) {
-                    KT val = k == self_k ? C[p * rl + c] : acc[r][p];
-                    if (bc && (fc || ((fixed_row >> p) & 1u)))
-                        val = (k == self_k && p == q) ? KT(1) : KT(0);
-                    out[p * rl + c] = val;
-                }
+                for (int p = 0; p < 3; ++p) S.row[p * rl + c] = acc[r][p];
         }
+        __syncwarp();
+        // diagonal block: lane (third, p, q) sums entry (p, q) of every third
+        // neighbour, then the thirds are added
+        {
+            const int third = lane / 9, pq = lane - 9 * third, p = pq / 3, q = pq - 3 * p;
+            KT s = KT(0);
+            if (lane < 27)
+                for (int k = third; k < deg; k += 3) s += S.row[p * rl + 3 * k + q];
+            const KT s1 = __shfl_sync(kFull, s, pq + 9), s2 = __shfl_sync(kFull, s, (pq + 18) & 31);
+            if (lane < 9 && deg) S.row[p * rl + 3 * self_k + q] = -(s + s1 + s2);
+        }
+        __syncwarp();
+        KT* out = K + 9 * (size_t)nb0;
+        const uint32_t fixed_row = __shfl_sync(kFull, fixed, self_k & 31);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            if (32 * r < rl) {  // uniform
+                const int c = lane + 32 * r, k = c / 3, q = c - 3 * k;
+                const uint32_t fc = (__shfl_sync(kFull, fixed, k & 31) >> q) & 1u;
+                if (c < rl)
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        KT val = k == self_k ? S.row[p * rl + c] : acc[r][p];
+                        if (bc && (fc || ((fixed_row >> p) & 1u)))
+                            val = (k == self_k && p == q) ? KT(1) : KT(0);
+                        out[p * rl + c] = val;
+                    }
+            }
+        }
+        __syncwarp();  // the next node's copies overwrite the rows
     }
+}
+
+template <typename KT, int PL>
+static void launch_node_pass(const MeshDev& m, KT* K, double* f, double* R, int apply_bc,
+                             cudaStream_t s) {
+    const unsigned grid = std::min<unsigned>((m.n_nodes + kAsmWarps<KT> - 1) / kAsmWarps<KT>,
+                                             148u * kAsmCtas<KT>);
+    constexpr size_t smem = kAsmWarps<KT> * sizeof(AsmWarp<KT, PL>);
+    // above the 48 KB every kernel may use the limit has to be raised (per
+    // device, on each launch: the call is cheap and keeps no state)
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(k_assemble<KT, PL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem);
+    k_assemble<KT, PL><<<grid, kAsmWarps<KT> * 32, smem, s>>>(
+        m, static_cast<const TanRec<KT>*>(m.tan_rec), K, f, R, apply_bc);
 }
 
 template <typename KT>
@@ -405,15 +478,8 @@ static void launch_assemble_t(const MeshDev& m, const double* u, KT* K, double* 
         return;
     }
     if (ge) k_asm_elements<KT, true><<<ge, 128, 0, s>>>(m, u, m.fvert, tan, status);
-    const unsigned grid = (m.n_nodes + kAsmWarps - 1) / kAsmWarps;
-    const size_t smem = kAsmWarps * (96 * sizeof(double) + 9 * m.max_pairs * sizeof(KT));
-    // at most 8 x (768 + 9 x 96 x 8) = 61,440 bytes: above the 48 KB every
-    // kernel may use, so the limit is raised (per device, on each launch: the
-    // call is cheap and keeps no state)
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_assemble<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    k_assemble<KT><<<grid, kAsmWarps * 32, smem, s>>>(m, tan, K, f, R, apply_bc);
+    if (m.pair_lane == 21) launch_node_pass<KT, 21>(m, K, f, R, apply_bc, s);
+    else launch_node_pass<KT, 33>(m, K, f, R, apply_bc, s);
 }
 void launch_assemble(const MeshDev& m, const double* u, double* K, double* f, double* R,
                      int apply_bc, unsigned* status, cudaStream_t s) {

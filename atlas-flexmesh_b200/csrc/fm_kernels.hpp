@@ -27,16 +27,17 @@ struct MeshDev {
     double* fvert = nullptr;
     void* tan_rec = nullptr;
     // the active (not skipped) tets of each node, ascending, built once per
-    // mesh: act_v[i] = 4 tet + the owner's local index; act_pos[i]: positions
-    // (4 x u8) of the tet's vertices in the owner's neighbour list, 0xff for
-    // a vertex that repeats an earlier one; nbr_members[j]: bit l set when
-    // the owner's l-th active tet holds the edge to neighbour entry j;
-    // max_pairs: most (tet, other vertex) pairs of a node, at least 32
+    // mesh: act_v[i] = 4 tet + the owner's local index.  The tet's three other
+    // vertices follow the owner's in cyclic order (j = 1, 2, 3); pair (tet l
+    // of the node, vertex j) has offset 9 (j - 1) pair_lane + l.  edge[e]:
+    // first pair | pairs << 8 of neighbour entry e; pair_off[3 act_ptr[n] +
+    // s]: offset of the node's pair s, pairs grouped by neighbour and
+    // ascending by tet (a vertex that repeats an earlier one has no pair)
     const uint32_t* act_ptr = nullptr;
     const uint32_t* act_v = nullptr;
-    const uint32_t* act_pos = nullptr;
-    const uint32_t* nbr_members = nullptr;
-    uint32_t max_pairs = 96;
+    const uint16_t* edge = nullptr;
+    const uint16_t* pair_off = nullptr;
+    int pair_lane = 33;  // 21 where no node has more than 20 active tets, else 33
 };
 constexpr size_t kTanRecBytes = 96;
 

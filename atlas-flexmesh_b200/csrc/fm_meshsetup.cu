@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "fm_device.cuh"
+#include "fm_kernels.hpp"
 #include "fm_meshsetup.hpp"
 
 namespace fm {
@@ -255,17 +256,17 @@ __global__ void k_act_count(uint32_t nn, const uint4* __restrict__ conn,
 }
 
 // node-pass scatter structure of the assembly (MeshDev): per active
-// incidence the tet and the owner's local index (its first occurrence) and
-// the 4 vertex positions in the owner's list, per neighbour entry the
-// owner's active tets holding that edge
+// incidence the tet and the owner's local index (its first occurrence), per
+// neighbour entry its pairs, per pair its offset
 __global__ void __launch_bounds__(kSetupWarps * 32)
     k_scatter_struct(uint32_t nn, const uint4* __restrict__ conn,
                      const uint32_t* __restrict__ inc_ptr, const uint32_t* __restrict__ inc_e,
                      const uint32_t* __restrict__ nbr_ptr, const uint32_t* __restrict__ nbr,
-                     const uint32_t* __restrict__ act_ptr, uint32_t* act_v, uint32_t* act_pos,
-                     uint32_t* members) {
+                     const uint32_t* __restrict__ act_ptr, int pair_lane, uint32_t* act_v,
+                     uint16_t* edge, uint16_t* pair_off) {
     __shared__ uint32_t list_s[kSetupWarps][32];
     __shared__ unsigned memb_s[kSetupWarps][32];
+    __shared__ int start_s[kSetupWarps][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (uint32_t n = blockIdx.x * kSetupWarps + w; n < nn; n += gridDim.x * kSetupWarps) {
         const uint32_t b = nbr_ptr[n], deg = nbr_ptr[n + 1] - b;
@@ -281,24 +282,42 @@ __global__ void __launch_bounds__(kSetupWarps * 32)
         }
         const bool act = !(c.x & 0x80000000u);
         const unsigned all = __ballot_sync(kFull, act);
+        const int l = __popc(all & ((1u << lane) - 1u));  // position among the active
+        uint32_t pos[4], own = 0;
         if (act) {
-            const int l = __popc(all & ((1u << lane) - 1u));  // position among the active
-            uint32_t pk = 0, own = 0;
 #pragma unroll
             for (int q = 3; q >= 0; --q) {
                 const uint32_t v = vtx(c, q);
-                uint32_t p = pos_in(list_s[w], deg, v);
+                pos[q] = v == n ? 0xffu : pos_in(list_s[w], deg, v);
                 for (int r = 0; r < q; ++r)
-                    if (vtx(c, r) == v) p = 0xffu;  // repeats an earlier vertex
-                pk |= p << (8 * q);
+                    if (vtx(c, r) == v) pos[q] = 0xffu;  // repeats an earlier vertex
                 if (v == n) own = (uint32_t)q;
-                else if (p != 0xffu) atomicOr(&memb_s[w][p], 1u << l);
+                if (pos[q] != 0xffu) atomicOr(&memb_s[w][pos[q]], 1u << l);
             }
             act_v[ab + l] = 4 * e + own;
-            act_pos[ab + l] = pk;
         }
         __syncwarp();
-        if (lane < (int)deg) members[b + lane] = memb_s[w][lane];
+        const unsigned memb = memb_s[w][lane];
+        const int cnt = __popc(memb);
+        int start = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(kFull, start, o);
+            if (lane >= o) start += t;
+        }
+        start -= cnt;
+        start_s[w][lane] = start;
+        if (lane < (int)deg) edge[b + lane] = (uint16_t)(start | cnt << 8);
+        __syncwarp();
+        if (act)
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q)
+                if (pos[q] != 0xffu) {
+                    const int s = start_s[w][pos[q]] +
+                                  __popc(memb_s[w][pos[q]] & ((1u << l) - 1u));
+                    const int j = (int)((q - own) & 3u);
+                    pair_off[3 * (size_t)ab + s] = (uint16_t)((j - 1) * 9 * pair_lane + l);
+                }
         __syncwarp();
     }
 }
@@ -448,15 +467,17 @@ cudaError_t build_mesh_device(uint32_t nn, uint32_t ne, const uint4* conn, MeshS
     SCK(cudaMemsetAsync(scal.p + 3, 0, sizeof(unsigned), s));
     k_act_count<<<blocks_for((size_t)nn * 32, 256), 256, 0, s>>>(nn, conn, d.inc_ptr->p,
                                                                d.inc_e->p, cnt.p, scal.p + 3);
+    SCK(cudaMemcpyAsync(hs, scal.p, sizeof hs, cudaMemcpyDeviceToHost, s));
     SCK(d.act_ptr->reserve((size_t)nn + 1));
     SCK(exclusive_scan(cnt.p, d.act_ptr->p, nn, tmp, s));
     SCK(d.act_v->reserve(std::max<size_t>(1, 4 * (size_t)ne)));
-    SCK(d.act_pos->reserve(std::max<size_t>(1, 4 * (size_t)ne)));
-    SCK(d.nbr_members->reserve(std::max<uint32_t>(total, 1)));
+    SCK(cudaStreamSynchronize(s));
+    h.max_act = hs[3];
+    SCK(d.edge->reserve(std::max<uint32_t>(total, 1)));
+    SCK(d.pair_off->reserve(std::max<size_t>(1, 12 * (size_t)ne)));
     k_scatter_struct<<<blocks_for(nn, kSetupWarps), kSetupWarps * 32, 0, s>>>(
-        nn, conn, d.inc_ptr->p, d.inc_e->p, d.nbr_ptr->p, d.nbr->p, d.act_ptr->p, d.act_v->p,
-        d.act_pos->p, d.nbr_members->p);
-    SCK(cudaMemcpyAsync(hs, scal.p, sizeof hs, cudaMemcpyDeviceToHost, s));
+        nn, conn, d.inc_ptr->p, d.inc_e->p, d.nbr_ptr->p, d.nbr->p, d.act_ptr->p,
+        h.pair_lane(), d.act_v->p, d.edge->p, d.pair_off->p);
     SCK(cudaGetLastError());
 
     // host copies of the graph
@@ -465,7 +486,6 @@ cudaError_t build_mesh_device(uint32_t nn, uint32_t ne, const uint4* conn, MeshS
     SCK(down(h.graph.nbr, d.nbr->p, total, s));
     SCK(down(h.graph.self, d.self_pos->p, nn, s));
     SCK(cudaStreamSynchronize(s));
-    h.max_act = hs[3];
     return cudaSuccess;
 }
 

@@ -14,8 +14,8 @@
 //               order (a node waits only on nodes with earlier tickets), and
 //               the level lists as a stable sort of the nodes by depth;
 //   ILU maps    fm_setup.hpp ilu_edge_maps; assembly scatter structures
-//               (active tets and vertex positions per node, tet bitmask per
-//               edge).
+//               (active tets per node, and the pairs of a tet and another of its
+//               vertices grouped by neighbour).
 // Every output equals the host construction in fm_setup.cpp entry for entry.
 #pragma once
 
@@ -42,21 +42,22 @@ struct MeshSetupDev {
     DevBuf<uint8_t>* emap;
     DevBuf<uint32_t>* act_ptr;      // n_nodes + 1: active incidences (MeshDev)
     DevBuf<uint32_t>* act_v;
-    DevBuf<uint32_t>* act_pos;      // 4 x u8 per active incidence
-    DevBuf<uint32_t>* nbr_members;  // tet bitmask per neighbour entry
+    DevBuf<uint16_t>* edge;         // per neighbour entry: its pairs
+    DevBuf<uint16_t>* pair_off;     // 3 per active incidence
 };
 
 // host copies that host-side planning and the exports use
 struct MeshSetupHost {
     NodeGraph graph;
     uint32_t max_inc = 0, max_act = 0;  // most incident / active tets of a node
+    int pair_lane() const { return max_act <= 20 ? 21 : 33; }  // MeshDev::pair_lane
     std::vector<uint32_t> lp, lo, up, uo;  // node levels: (ptr, order) forward, backward
 };
 
 enum { kSetupOk = 0, kSetupLimits = 1, kSetupTimeout = 2 };
 
 // conn: n_elems uint4 on the device, bit 31 of .x marking a skipped tet (the
-// incidence and graph include it; the tet bitmasks do not).  status: the
+// incidence and graph include it; the scatter structures do not).  status: the
 // context's status word (its bounded-wait limit follows it).  *result:
 // kSetupLimits when a node has more than 32 neighbours or incident tets,
 // kSetupTimeout when a dependency wait of the level pass expired.
