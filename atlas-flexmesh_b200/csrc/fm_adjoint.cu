@@ -138,6 +138,7 @@ __device__ __forceinline__ bool load_tet(const MeshDev& m, uint32_t e, const dou
 __global__ void __launch_bounds__(128)
     k_exact_elements(MeshDev m, const double* __restrict__ u, const double* __restrict__ v,
                      double* __restrict__ fvert, int transpose) {
+    chain_let_next();
     const uint32_t e = blockIdx.x * 128u + threadIdx.x;
     if (e >= m.n_elems) return;
     uint32_t cn[4];

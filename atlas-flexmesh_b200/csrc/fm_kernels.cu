@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(128, 4)
     k_asm_elements(MeshDev m, const double* __restrict__ u, double* __restrict__ fvert,
                    TanRec<KT>* __restrict__ tan, unsigned* __restrict__ status) {
     __shared__ double stage_s[4][32 * 13];
+    chain_let_next();  // the node pass: its first lists load while this one ends
     const int lane = threadIdx.x & 31;
     double* stage = stage_s[threadIdx.x >> 5];
     const uint32_t e0 = blockIdx.x * 128u + (threadIdx.x & ~31u);  // the warp's first tet
@@ -170,6 +171,7 @@ __global__ void __launch_bounds__(256)
                     const uint32_t* __restrict__ act_v, const double* __restrict__ fvert,
                     const uint8_t* __restrict__ mask, double* __restrict__ f,
                     double* __restrict__ R) {
+    chain_wait();
     const uint32_t row = blockIdx.x * 256u + threadIdx.x;
     if (row >= 3 * n_nodes) return;
     const uint32_t n = row / 3, c = row - 3 * n;
@@ -189,8 +191,8 @@ __global__ void __launch_bounds__(256)
 }
 
 void launch_gather_forces(const MeshDev& m, double* f, double* R, cudaStream_t s) {
-    k_gather_forces<<<(3 * m.n_nodes + 255) / 256, 256, 0, s>>>(m.n_nodes, m.act_ptr, m.act_v,
-                                                               m.fvert, m.mask, f, R);
+    launch_chained(k_gather_forces, (3 * m.n_nodes + 255) / 256, 256, 0, s, m.n_nodes, m.act_ptr,
+                   m.act_v, m.fvert, m.mask, f, R);
 }
 
 // gradients of a tet's four vertices and its tangent scalars, from a staged
@@ -301,6 +303,7 @@ __global__ void __launch_bounds__(kAsmWarps<KT> * 32, kAsmCtas<KT>)
     uint32_t n = blockIdx.x * kAsmWarps<KT> + wi;
     pointers(n);
     lists(n);
+    chain_wait();  // so far only the mesh's own structure was read
     for (; n < m.n_nodes; n += step) {  // uniform per warp
         const uint32_t nb0 = nx.nb0, a0 = nx.a0, v = nx.v, my_nbr = nx.nbr, my_edge = nx.edge;
         const int deg = nx.deg, ma = nx.ma;
@@ -462,8 +465,8 @@ static void launch_node_pass(const MeshDev& m, KT* K, double* f, double* R, int 
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(k_assemble<KT, PL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
-    k_assemble<KT, PL><<<grid, kAsmWarps<KT> * 32, smem, s>>>(
-        m, static_cast<const TanRec<KT>*>(m.tan_rec), K, f, R, apply_bc);
+    launch_chained(k_assemble<KT, PL>, grid, kAsmWarps<KT> * 32, smem, s, m,
+                   static_cast<const TanRec<KT>*>(m.tan_rec), K, f, R, apply_bc);
 }
 
 template <typename KT>
