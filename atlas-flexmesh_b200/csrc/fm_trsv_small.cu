@@ -28,7 +28,7 @@ namespace fm {
 
 namespace {
 
-constexpr int kMaxDepth = 2;  // levels whose entries are in flight
+constexpr int kMaxDepth = 4;  // levels whose entries are in flight
 
 template <int M>
 struct Row {
@@ -61,7 +61,7 @@ __device__ __forceinline__ void solve_row(const Row<M>& E, double* z) {
 
 // one direction, in place on z (z[n] = 0 for the padding); lvl[n_levels ..
 // n_levels + D] = n
-template <int M, int D, bool Upper>
+template <int M, int D, bool Wide, bool Upper>
 __device__ __forceinline__ void sweep(const SmallTri& S, const uint32_t* lvl, uint32_t n,
                                       double* z) {
     Row<M> e[D];
@@ -74,12 +74,12 @@ __device__ __forceinline__ void sweep(const SmallTri& S, const uint32_t* lvl, ui
             if (l < S.n_levels) {  // uniform
                 const uint32_t b = lvl[l], end = lvl[l + 1], next = lvl[l + D];
                 if (b + threadIdx.x < end) solve_row<M, Upper>(e[q], z);
-                // rows of a level beyond the block's width
-                for (uint32_t t = b + threadIdx.x + blockDim.x; t < end; t += blockDim.x) {
-                    Row<M> x;
-                    load_row<M, Upper>(S, t, n, x);
-                    solve_row<M, Upper>(x, z);
-                }
+                if (Wide)  // rows of a level beyond the block's width
+                    for (uint32_t t = b + threadIdx.x + blockDim.x; t < end; t += blockDim.x) {
+                        Row<M> x;
+                        load_row<M, Upper>(S, t, n, x);
+                        solve_row<M, Upper>(x, z);
+                    }
                 load_row<M, Upper>(S, min(next + threadIdx.x, n - 1), n, e[q]);
                 __syncthreads();
             }
@@ -87,7 +87,7 @@ __device__ __forceinline__ void sweep(const SmallTri& S, const uint32_t* lvl, ui
     }
 }
 
-template <int M, int D, int Threads>
+template <int M, int D, int Threads, bool Wide>
 __global__ void __launch_bounds__(Threads, 1)
     k_trsv_small(SmallTri L, SmallTri U, uint32_t n, const double* __restrict__ r,
                  double* __restrict__ out, const unsigned* __restrict__ skip) {
@@ -105,8 +105,8 @@ __global__ void __launch_bounds__(Threads, 1)
     for (uint32_t i = threadIdx.x; i <= U.n_levels + D; i += blockDim.x)
         lb[i] = i < U.n_levels ? __ldg(U.level + i) : n;
     __syncthreads();
-    sweep<M, D, false>(L, lf, n, z);
-    sweep<M, D, true>(U, lb, n, z);
+    sweep<M, D, Wide, false>(L, lf, n, z);
+    sweep<M, D, Wide, true>(U, lb, n, z);
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) out[i] = z[i];
 }
 
@@ -124,18 +124,26 @@ __global__ void k_pack_small(uint32_t n, uint32_t total, const uint32_t* __restr
     }
 }
 
+template <int M, int D, int Threads, bool Wide>
+cudaError_t launch_w(const SmallTri& L, const SmallTri& U, uint32_t n, unsigned th, size_t smem,
+                     const double* r, double* out, const unsigned* skip, cudaStream_t s) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_trsv_small<M, D, Threads, Wide>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return launch_chained(k_trsv_small<M, D, Threads, Wide>, 1, th, smem, s, L, U, n, r, out, skip);
+}
+
 template <int M, int D, int Threads>
 cudaError_t launch_t(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t width,
                      const double* r, double* out, const unsigned* skip, cudaStream_t s) {
     const size_t smem = small_tri_smem(n, L.n_levels, U.n_levels);
-    const cudaError_t e = cudaFuncSetAttribute(
-        k_trsv_small<M, D, Threads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     // no more threads than the widest level has rows (fewer warps, a cheaper
     // barrier) or than the copies in and out can use
     const unsigned th =
         std::min<unsigned>(Threads, std::max(32u, (std::max(width, n / 64) + 31u) & ~31u));
-    return launch_chained(k_trsv_small<M, D, Threads>, 1, th, smem, s, L, U, n, r, out, skip);
+    return width > th ? launch_w<M, D, Threads, true>(L, U, n, th, smem, r, out, skip, s)
+                      : launch_w<M, D, Threads, false>(L, U, n, th, smem, r, out, skip, s);
 }
 
 }  // namespace
