@@ -196,8 +196,7 @@ bool push_plan(const NodeGraph& g, const std::vector<uint32_t>& fwd_ptr,
     for (uint32_t l = 0; l < nlb; ++l)
         for (uint32_t t = bwd_ptr[l]; t < bwd_ptr[l + 1]; ++t) lb[bwd_order[t]] = l;
     // busiest CTA's share of one level, either direction; counting stops once
-    // it exceeds `bound` (the block cannot be the best then: most candidates
-    // end early, which halves the search)
+    // it exceeds `bound`
     std::vector<uint32_t> cf((size_t)nc * nlf), cb((size_t)nc * nlb);
     auto share = [&](uint32_t R, uint32_t bound) {
         std::fill(cf.begin(), cf.end(), 0u);
@@ -210,19 +209,25 @@ bool push_plan(const NodeGraph& g, const std::vector<uint32_t>& fwd_ptr,
         }
         return mx;
     };
+    // Candidates by share.  The best one's slots usually fit, so the others
+    // are counted only as far as they stay within kSlack of it (most end
+    // early); should none of those fit, the rest are counted in full.
+    constexpr uint32_t kSlack = 2;
     std::vector<std::pair<uint32_t, uint32_t>> cand;  // (share, block)
     std::vector<uint32_t> rest;  // blocks whose count was cut short
+    size_t near = 1;  // candidates known to be the best ones
     if (block) {
         cand.push_back({share(block, ~0u), block});
     } else {
-        uint32_t best = ~0u;
+        uint32_t best = ~0u - kSlack;
         for (uint32_t R = 16; R <= 512; R += R < 128 ? 1 : 8) {
-            const uint32_t sh = share(R, best);
-            if (sh > best) rest.push_back(R);
+            const uint32_t sh = share(R, best + kSlack);
+            if (sh > best + kSlack) rest.push_back(R);
             else cand.push_back({sh, R});
             best = std::min(best, sh);
         }
         std::sort(cand.begin(), cand.end());
+        for (near = 0; near < cand.size() && cand[near].first <= best + kSlack;) ++near;
     }
     std::vector<uint32_t> cta(nn);
     auto slots = [&](bool lower, std::vector<uint32_t>& push, std::vector<uint32_t>& nslot,
@@ -258,13 +263,12 @@ bool push_plan(const NodeGraph& g, const std::vector<uint32_t>& fwd_ptr,
         return true;
     };
     for (size_t at = 0; at < cand.size() || !rest.empty(); ++at) {
-        if (at == 1 && !rest.empty()) {
-            // the best block's slots do not fit: the others in order of their
-            // full counts
+        if (at == near && !rest.empty()) {
             for (uint32_t R : rest) cand.push_back({share(R, ~0u), R});
             rest.clear();
-            std::sort(cand.begin() + 1, cand.end());
+            std::sort(cand.begin() + near, cand.end());
         }
+        if (at == cand.size()) break;
         const std::pair<uint32_t, uint32_t> cs = cand[at];
         const uint32_t R = cs.second;
         for (uint32_t n = 0; n < nn; ++n) cta[n] = push_cta(n, nn, n_clusters, cluster, R);

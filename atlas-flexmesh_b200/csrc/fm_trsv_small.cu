@@ -7,14 +7,16 @@
 // next.  Through L2, with a warp per row and a release flag each, a level
 // cost 3.7 us (2.2 ms per apply there).  Here one CTA keeps the whole vector
 // in shared memory and takes a level at a time, one thread per row, with a
-// block barrier between levels: 0.22 us per level.
+// block barrier between levels: 0.19 us per level.
 //
 // The factors come as one stream per direction in level order, entry m of
 // position t at [m * n + t] (rows with fewer entries are padded with zero
 // coefficients that read a zero), packed after each factorization; a
-// thread's entries of the next two levels are in flight in registers (131 us
-// per apply there, 90 of them without any loads; three to six levels ahead
-// took 141 to 178, as did 16-byte packed rows, and a cp.async ring 143).
+// thread's entries of the next level are in flight in registers (113 us per
+// apply there, 90 of them without any loads; two, three and four levels ahead
+// 125, 126 and 141 us: the unrolled loop outgrows the instruction cache more
+// than the deeper prefetch gains; 16-byte packed rows 160, a cp.async ring
+// 143).
 //
 // Used when the vector and the level pointers fit shared memory and no row
 // has more than kSmallMaxEntries off-diagonal entries on one side: longer
@@ -28,7 +30,7 @@ namespace fm {
 
 namespace {
 
-constexpr int kMaxDepth = 4;  // levels whose entries are in flight
+constexpr int kMaxDepth = 1;  // levels whose entries are in flight
 
 template <int M>
 struct Row {
@@ -163,9 +165,9 @@ void launch_pack_small(uint32_t n, uint32_t entries, const uint32_t* src_f, cons
 cudaError_t launch_trsv_small(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t entries,
                               uint32_t width, const double* r, double* out, const unsigned* skip,
                               cudaStream_t s) {
-    if (entries <= 2) return launch_t<2, 2, 1024>(L, U, n, width, r, out, skip, s);
-    if (entries <= 4) return launch_t<4, 2, 512>(L, U, n, width, r, out, skip, s);
-    return launch_t<8, 2, 512>(L, U, n, width, r, out, skip, s);
+    if (entries <= 2) return launch_t<2, 1, 1024>(L, U, n, width, r, out, skip, s);
+    if (entries <= 4) return launch_t<4, 1, 512>(L, U, n, width, r, out, skip, s);
+    return launch_t<8, 1, 512>(L, U, n, width, r, out, skip, s);
 }
 
 }  // namespace fm
