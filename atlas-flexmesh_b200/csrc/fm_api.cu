@@ -507,10 +507,10 @@ fm_status setup_push_solves(fm_ctx* c, const std::vector<uint32_t>& lp,
     // polls, and every further cluster is one more slab boundary, crossed
     // through L2.  Small meshes therefore take clusters of at most 16 warps
     // per CTA, as many as that needs, large ones all clusters and up to 32
-    // warps (FP32; FP64's double-buffered loop 10 or 16).  Per FP32 / FP64 pair
-    // against all clusters with 32 / 16 warps: 8^3 62 -> 45 / 69 -> 52 us, 16^3
-    // 110 -> 83 / 119 -> 102 us, 32^3 201 -> 178 / 220 -> 215 us, 48^3 307 -> 292
-    // us / unchanged; 64^3 takes them all.
+    // warps (FP32; FP64's double-buffered loop 10 or 16).  us per FP32 / FP64
+    // pair against all clusters with 32 / 16 warps: 8^3 62 -> 43 / 69 -> 53,
+    // 16^3 110 -> 85 / 119 -> 104, 32^3 201 -> 173 / 220 -> 214, 48^3 307 ->
+    // 291 / 363 both; 64^3 takes them all.
     const uint32_t levels = std::max<uint32_t>(1, (uint32_t)std::max(lp.size(), up.size()) - 1);
     const uint32_t want = std::max(1u, (7 * c->nn + levels - 1) / levels);  // warps
     fm::PushPlan p;
@@ -720,10 +720,12 @@ fm_status pcg_core(fm_ctx* c, const Op<T>& A, uint32_t n, const T* b, T* x, doub
         A.precond(w.r.p, w.z.p, done, t != nullptr);
         { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_rz<T>(n, w.r.p, w.z.p, tol, part, c->counter(), sc, slot(k), seq0 + (unsigned)k, c->stream); }
     };
-    int iters = max_iter;
+    int iters = max_iter, ran = 0;
+    bool early = false;
     double relres = 0.0;
     for (int k = 0; k <= max_iter; ++k) {
         if (k < max_iter) iteration(k + 1);
+        ran = k;
         fm::PcgReport rep;
         fm_status st = wait_report(c, seq0 + (unsigned)k, &rep);
         if (st == FM_OK) st = check_flags(c, rep.status, "pcg");
@@ -736,6 +738,7 @@ fm_status pcg_core(fm_ctx* c, const Op<T>& A, uint32_t n, const T* b, T* x, doub
         if (k == 0) {
             if (rep.done) {
                 iters = 0;
+                early = true;
                 break;
             }
             continue;
@@ -746,6 +749,17 @@ fm_status pcg_core(fm_ctx* c, const Op<T>& A, uint32_t n, const T* b, T* x, doub
             iters = k;
             break;
         }
+    }
+    // an iteration queued in vain (and the first apply before an early exit)
+    // did no work: its launches stay counted, its groups do not
+    if (c->rep_seq != seq0 + (unsigned)ran) {
+        c->prof_calls[FM_PROF_SPMV] -= 1;
+        c->prof_calls[FM_PROF_TRSV] -= 1;
+        c->prof_calls[FM_PROF_VECTOR] -= ran ? 3 : 2;
+    }
+    if (early) {
+        c->prof_calls[FM_PROF_TRSV] -= 1;
+        c->prof_calls[FM_PROF_VECTOR] -= 1;
     }
     if (iters_out) *iters_out = iters;
     if (relres_out) *relres_out = relres;

@@ -13,10 +13,9 @@
 // position t at [m * n + t] (rows with fewer entries are padded with zero
 // coefficients that read a zero), packed after each factorization; a
 // thread's entries of the next level are in flight in registers (113 us per
-// apply there, 90 of them without any loads; two, three and four levels ahead
-// 125, 126 and 141 us: the unrolled loop outgrows the instruction cache more
-// than the deeper prefetch gains; 16-byte packed rows 160, a cp.async ring
-// 143).
+// apply there; two, three and four levels ahead, with the loop unrolled as
+// often, took 125, 126 and 141; 16-byte packed rows 160, a cp.async ring 143;
+// a build without any loads in the loop 90).
 //
 // Used when the vector and the level pointers fit shared memory and no row
 // has more than kSmallMaxEntries off-diagonal entries on one side: longer

@@ -113,7 +113,9 @@ fm_status fm_sizes(const fm_ctx* ctx, uint32_t* n_nodes, uint32_t* n_elems, uint
                    uint64_t* nnz);
 /* Built-in profiler (no reference counterpart; the reference times whole
  * phases with wall clocks, FEM/adaptive_fem_engine.hpp:1251-1273).
- * Launch groups and kernel launches are always counted per class;
+ * Launch groups and kernel launches are always counted per class (groups of a
+ * PCG iteration that was queued ahead and then not needed count as launches
+ * only);
  * fm_profile_enable(ctx, on) zeroes all counters, and with on = 1 also
  * records a CUDA event pair around every kernel group launched afterwards
  * (device time per class).  fm_profile_read synchronizes the stream and
