@@ -268,12 +268,12 @@ struct __align__(16) AsmWarp {
 //      blocks through the pair list, ascending element order, for the three
 //      rows at once.
 //   4. The diagonal block is minus the sum of the row's other blocks.
-// The loop over nodes loads the next node's lists meanwhile.  Bound: latency
-// and issue (900 instructions per node; the three dependent loads that start
-// a node and the copies take most of its 7 us unless they overlap the node
-// before: 572 -> 478 us with the copies in flight together, 420 with the lists
-// ahead and no spills, FP64 at 64^3).  One lane per neighbour walking its tets
-// took 605.  Whole assembly: 128^3 FP64 5.67 -> 3.96 ms, 33^3 FP32 88 -> 63 us.
+// The loop over nodes loads the next node's lists meanwhile.  Bound: the L1
+// data pipe (89% busy in FP64: 360 shared-memory wavefronts per node).  Before
+// the copies overlapped, a node's three dependent loads were most of its 7 us:
+// 572 -> 478 us with the copies in flight together, 420 with the lists ahead
+// and no spills (FP64 at 64^3).  One lane per neighbour walking its tets took
+// 605.  Whole assembly: 128^3 FP64 5.67 -> 3.97 ms, 33^3 FP32 88 -> 62 us.
 template <typename KT, int PL>
 __global__ void __launch_bounds__(kAsmWarps<KT> * 32, kAsmCtas<KT>)
     k_assemble(MeshDev m, const TanRec<KT>* __restrict__ tan, KT* __restrict__ K,
