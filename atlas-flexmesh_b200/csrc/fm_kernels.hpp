@@ -66,12 +66,12 @@ void launch_elements(uint32_t n, const double* x, const double* u, const double*
 // null also finishes dot(x, y) into *dot through the deterministic grid
 // reduction.  val and nbr must have 16 bytes of room past their end, nbr_ptr
 // 80.  skip (here and below; null: never): a device word that, when set,
-// makes the kernel return at once.
+// makes the kernel return at once.  Returns the launch's status.
 template <typename T>
-void launch_spmv_nodes(uint32_t n_nodes, uint32_t max_deg, const uint32_t* nbr_ptr,
-                       const uint32_t* nbr, const T* val, const T* x, T* y, T* partials,
-                       unsigned* counter, double* dot, unsigned* status, cudaStream_t s,
-                       const unsigned* skip = nullptr);
+cudaError_t launch_spmv_nodes(uint32_t n_nodes, uint32_t max_deg, const uint32_t* nbr_ptr,
+                              const uint32_t* nbr, const T* val, const T* x, T* y, T* partials,
+                              unsigned* counter, double* dot, unsigned* status, cudaStream_t s,
+                              const unsigned* skip = nullptr);
 // Generic scalar CSR SpMV (ascending or any column order)
 template <typename T>
 void launch_spmv_csr(uint32_t n, uint64_t nnz, const uint32_t* rp, const uint32_t* ci,

@@ -225,20 +225,25 @@ __global__ void __launch_bounds__(kStreamThreads)
     }
 }
 
+constexpr size_t kSmStages = 220 * 1024;  // shared memory of an SM for its CTAs' stages
+
 template <typename T, int S>
-void launch_stages(uint32_t nn, const StageLayout& L, int per_sm, const uint32_t* nbr_ptr,
-                   const uint32_t* nbr, const T* val, const T* x, T* y, T* partials,
-                   unsigned* counter, double* dot, unsigned* status, cudaStream_t s,
-                   const unsigned* skip) {
+cudaError_t launch_stages(uint32_t nn, const StageLayout& L, int per_sm, const uint32_t* nbr_ptr,
+                          const uint32_t* nbr, const T* val, const T* x, T* y, T* partials,
+                          unsigned* counter, double* dot, unsigned* status, cudaStream_t s,
+                          const unsigned* skip) {
     const size_t smem = (size_t)S * L.bytes;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_spmv_nodes<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+    // The limit is the kernel's own, shared by every context and thread on the
+    // device: always the same value, so that a thread with a smaller mesh
+    // cannot lower it between another thread's call and launch.
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_spmv_nodes<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmStages / S));
+    if (e != cudaSuccess) return e;
     const uint32_t tiles = (nn + kTile - 1) / kTile;
     // a fixed grid per mesh: the dot product's summation order is fixed
     const unsigned grid = std::min<unsigned>(tiles, 148u * per_sm);
-    launch_chained(k_spmv_nodes<T, S>, grid, kStreamThreads, smem, s, nn, L, nbr_ptr, nbr, val, x,
-                   y, partials, counter, dot, skip, status);
+    return launch_chained(k_spmv_nodes<T, S>, grid, kStreamThreads, smem, s, nn, L, nbr_ptr, nbr,
+                          val, x, y, partials, counter, dot, skip, status);
 }
 
 }  // namespace
@@ -247,26 +252,27 @@ void launch_stages(uint32_t nn, const StageLayout& L, int per_sm, const uint32_t
 // 60 KB in flight per SM either way); a mesh of the largest valence, 32,
 // still fits two.
 template <typename T>
-void launch_spmv_nodes(uint32_t nn, uint32_t max_deg, const uint32_t* nbr_ptr, const uint32_t* nbr,
-                       const T* val, const T* x, T* y, T* partials, unsigned* counter, double* dot,
-                       unsigned* status, cudaStream_t s, const unsigned* skip) {
+cudaError_t launch_spmv_nodes(uint32_t nn, uint32_t max_deg, const uint32_t* nbr_ptr,
+                              const uint32_t* nbr, const T* val, const T* x, T* y, T* partials,
+                              unsigned* counter, double* dot, unsigned* status, cudaStream_t s,
+                              const unsigned* skip) {
     const StageLayout L = stage_layout<T>(max_deg);
-    constexpr size_t kSm = 220 * 1024;
-    if (16 * (size_t)L.bytes <= kSm)
-        launch_stages<T, 4>(nn, L, 4, nbr_ptr, nbr, val, x, y, partials, counter, dot, status, s,
-                            skip);
-    else if (9 * (size_t)L.bytes <= kSm)
-        launch_stages<T, 3>(nn, L, 3, nbr_ptr, nbr, val, x, y, partials, counter, dot, status, s,
-                            skip);
-    else
-        launch_stages<T, 2>(nn, L, 2, nbr_ptr, nbr, val, x, y, partials, counter, dot, status, s,
-                            skip);
+    if (16 * (size_t)L.bytes <= kSmStages)
+        return launch_stages<T, 4>(nn, L, 4, nbr_ptr, nbr, val, x, y, partials, counter, dot,
+                                   status, s, skip);
+    if (9 * (size_t)L.bytes <= kSmStages)
+        return launch_stages<T, 3>(nn, L, 3, nbr_ptr, nbr, val, x, y, partials, counter, dot,
+                                   status, s, skip);
+    return launch_stages<T, 2>(nn, L, 2, nbr_ptr, nbr, val, x, y, partials, counter, dot, status,
+                               s, skip);
 }
-template void launch_spmv_nodes<double>(uint32_t, uint32_t, const uint32_t*, const uint32_t*,
-                                        const double*, const double*, double*, double*, unsigned*,
-                                        double*, unsigned*, cudaStream_t, const unsigned*);
-template void launch_spmv_nodes<float>(uint32_t, uint32_t, const uint32_t*, const uint32_t*,
-                                       const float*, const float*, float*, float*, unsigned*,
-                                       double*, unsigned*, cudaStream_t, const unsigned*);
+template cudaError_t launch_spmv_nodes<double>(uint32_t, uint32_t, const uint32_t*, const uint32_t*,
+                                               const double*, const double*, double*, double*,
+                                               unsigned*, double*, unsigned*, cudaStream_t,
+                                               const unsigned*);
+template cudaError_t launch_spmv_nodes<float>(uint32_t, uint32_t, const uint32_t*, const uint32_t*,
+                                              const float*, const float*, float*, float*,
+                                              unsigned*, double*, unsigned*, cudaStream_t,
+                                              const unsigned*);
 
 }  // namespace fm

@@ -128,9 +128,11 @@ __global__ void k_pack_small(uint32_t n, uint32_t total, const uint32_t* __restr
 template <int M, int D, int Threads, bool Wide>
 cudaError_t launch_w(const SmallTri& L, const SmallTri& U, uint32_t n, unsigned th, size_t smem,
                      const double* r, double* out, const unsigned* skip, cudaStream_t s) {
+    // one limit for every matrix: it is the kernel's, not the call's, and
+    // another thread may be between its own call and launch
     const cudaError_t e =
         cudaFuncSetAttribute(k_trsv_small<M, D, Threads, Wide>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMaxSmem);
     if (e != cudaSuccess) return e;
     return launch_chained(k_trsv_small<M, D, Threads, Wide>, 1, th, smem, s, L, U, n, r, out, skip);
 }
