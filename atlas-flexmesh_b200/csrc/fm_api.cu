@@ -185,9 +185,11 @@ fm_status fail(fm_ctx* c, fm_status st, const char* fmt, ...) {
 #define CK(call)                                                                           \
     do {                                                                                   \
         cudaError_t e_ = (call);                                                           \
-        if (e_ != cudaSuccess)                                                             \
+        if (e_ != cudaSuccess) {                                                           \
+            cudaGetLastError(); /* reported here, not by a later call */                   \
             return fail(c, e_ == cudaErrorMemoryAllocation ? FM_ERR_OOM : FM_ERR_CUDA,     \
                         "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+        }                                                                                  \
     } while (0)
 
 #define TRY(expr)                       \
@@ -284,6 +286,7 @@ fm_status check_flags(fm_ctx* c, uint32_t flags, const char* where) {
 }
 
 fm_status sync_scalars(fm_ctx* c) {
+    CK(cudaGetLastError());  // a refused launch leaves the scalars as they were
     CK(cudaMemcpyAsync(c->h_sc, c->sc.p, sizeof(fm::DevScalars), cudaMemcpyDeviceToHost,
                        c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -582,31 +585,30 @@ fm_status setup_push_solves(fm_ctx* c, const std::vector<uint32_t>& lp,
 // z = U^-1 L^-1 r on the node-block factors (tmp: the intermediate): the
 // slab-partitioned push solves where the context has a plan for this value
 // width, else the grid-wide pipelined ones.  filled: tmp holds the wait
-// sentinel.  Returns the kernels launched.
+// sentinel.
 template <typename T>
-int precond_nodes(fm_ctx* c, const T* lu, const T* dinv, const T* r, T* tmp, T* z,
-                  unsigned* status, const unsigned* skip = nullptr, bool filled = false) {
+cudaError_t precond_nodes(fm_ctx* c, const T* lu, const T* dinv, const T* r, T* tmp, T* z,
+                          unsigned* status, const unsigned* skip = nullptr, bool filled = false) {
     const bool pu = sizeof(T) == 4 ? c->pu_ok32 : c->pu_ok64;
     if (pu && c->nn) {
         const cudaError_t e = fm::launch_trsv_push<T>(c->pu, node_sched(c), lu, dinv, r, tmp, z,
                                                       status, c->stream, skip, filled);
-        if (e == cudaSuccess) return (z != r ? 3 : 4) - (filled ? 1 : 0);
+        if (e == cudaSuccess) return e;
         // a launch the device refuses: the pipelined solves from now on
         cudaGetLastError();
         c->pu_ok32 = c->pu_ok64 = false;
     }
-    fm::launch_trsv_nodes<T>(node_sched(c), lu, dinv, r, tmp, z, status, c->device, c->stream,
-                             skip);
-    return 4;
+    return fm::launch_trsv_nodes<T>(node_sched(c), lu, dinv, r, tmp, z, status, c->device,
+                                    c->stream, skip);
 }
 
 // y = K x on the context's K (dot: also x.y)
 template <typename T>
-void spmv_nodes(fm_ctx* c, const T* K, const T* x, T* y, double* dot,
-                const unsigned* skip = nullptr) {
-    fm::launch_spmv_nodes<T>(c->nn, c->graph.max_deg, c->nbr_ptr.p, c->nbr.p, K, x, y,
-                             reinterpret_cast<T*>(c->partials.p), c->counter(), dot, c->status(),
-                             c->stream, skip);
+cudaError_t spmv_nodes(fm_ctx* c, const T* K, const T* x, T* y, double* dot,
+                       const unsigned* skip = nullptr) {
+    return fm::launch_spmv_nodes<T>(c->nn, c->graph.max_deg, c->nbr_ptr.p, c->nbr.p, K, x, y,
+                                    reinterpret_cast<T*>(c->partials.p), c->counter(), dot,
+                                    c->status(), c->stream, skip);
 }
 
 // A linear operator for PCG: the mesh K (node-block SpMV) or a generic CSR.
@@ -627,42 +629,37 @@ struct Op {
     T* prefill() const {
         return node_block && (sizeof(T) == 4 ? c->pu_ok32 : c->pu_ok64) ? tmp : nullptr;
     }
-    void spmv(const T* x, T* y, double* dot, const unsigned* skip = nullptr) const {
+    cudaError_t spmv(const T* x, T* y, double* dot, const unsigned* skip = nullptr) const {
         PROF(FM_PROF_SPMV, 1);
         T* part = reinterpret_cast<T*>(c->partials.p);
-        if (node_block)
-            spmv_nodes<T>(c, K, x, y, dot, skip);
-        else
-            fm::launch_spmv_csr<T>(S->n, S->nnz, S->rp.p, S->ci.p, K, x, y, part, c->counter(),
-                                   dot, c->stream, skip);
+        if (node_block) return spmv_nodes<T>(c, K, x, y, dot, skip);
+        return fm::launch_spmv_csr<T>(S->n, S->nnz, S->rp.p, S->ci.p, K, x, y, part, c->counter(),
+                                      dot, c->stream, skip);
     }
-    void precond(const T* r, T* z, const unsigned* skip = nullptr, bool filled = false) const {
+    cudaError_t precond(const T* r, T* z, const unsigned* skip = nullptr, bool filled = false) const {
         const bool pu = node_block && (sizeof(T) == 4 ? c->pu_ok32 : c->pu_ok64);
         PROF(FM_PROF_TRSV, pu ? (r != z ? 3 : 4) - (filled ? 1 : 0)
                               : node_block ? 4 : S->small_entries ? 1 : 2);
-        if (node_block) {
-            precond_nodes<T>(c, LU, dinv, r, tmp, z, c->status(), skip, filled);
-            return;
-        }
+        if (node_block)
+            return precond_nodes<T>(c, LU, dinv, r, tmp, z, c->status(), skip, filled);
         if constexpr (sizeof(T) == 8)
             if (S->small_entries) {
                 if (fm::launch_trsv_small(S->tri(true), S->tri(false), S->n, S->small_entries,
                                           S->small_width, r, z, skip, c->stream) == cudaSuccess)
-                    return;
+                    return cudaSuccess;
                 cudaGetLastError();  // refused by the device: the solves below from now on
                 S->small_entries = 0;
             }
         const fm::CsrDev v = S->view();
-        fm::launch_trsv_lower_csr<T>(v, LU, r, tmp, c->done.p, next_epoch(c), c->status(),
-                                     grid_trsv, c->stream, skip);
-        fm::launch_trsv_upper_csr<T>(v, LU, diag, tmp, z, c->done.p, next_epoch(c), c->status(),
-                                     grid_trsv, c->stream, skip);
+        FM_LAUNCH(fm::launch_trsv_lower_csr<T>(v, LU, r, tmp, c->done.p, next_epoch(c),
+                                               c->status(), grid_trsv, c->stream, skip));
+        return fm::launch_trsv_upper_csr<T>(v, LU, diag, tmp, z, c->done.p, next_epoch(c),
+                                            c->status(), grid_trsv, c->stream, skip);
     }
 };
 
 // Waits for report seq (in its slot of the ring).  The kernel that writes it
-// is queued; should the stream end without it (a launch that failed), the
-// stream's error is returned.
+// is queued; should the stream end without it, its error is returned.
 fm_status wait_report(fm_ctx* c, unsigned seq, fm::PcgReport* out) {
     const volatile fm::PcgReport* r = c->h_rep + seq % fm_ctx::kReports;
     for (unsigned spin = 1; __atomic_load_n(&r->seq, __ATOMIC_ACQUIRE) != seq; ++spin) {
@@ -704,30 +701,41 @@ fm_status pcg_core(fm_ctx* c, const Op<T>& A, uint32_t n, const T* b, T* x, doub
     const unsigned* done = &sc->done;
     const unsigned seq0 = c->rep_seq + 1;  // report of step k: seq0 + k (0: the entry)
     auto slot = [&](int k) { return c->d_rep + (seq0 + (unsigned)k) % fm_ctx::kReports; };
-    // r = b - A x
-    if (!zero_x) A.spmv(x, w.r.p, nullptr);
-    T* tmp = A.prefill();
-    { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_init<T>(n, b, w.r.p, zero_x, tmp, tol, part, c->counter(), sc, slot(0), seq0, c->stream); }
-    A.precond(w.r.p, w.z.p, done, tmp != nullptr);
-    { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_start<T>(n, w.r.p, w.z.p, b, w.p.p, part, c->counter(), sc, c->stream); }
-    c->rep_seq = seq0;
-    auto iteration = [&](int k) {
+    auto entry = [&]() -> cudaError_t {
+        c->rep_seq = seq0;
+        // r = b - A x
+        if (!zero_x) FM_LAUNCH(A.spmv(x, w.r.p, nullptr));
+        T* tmp = A.prefill();
+        { PROF(FM_PROF_VECTOR, 1); FM_LAUNCH(fm::launch_pcg_init<T>(n, b, w.r.p, zero_x, tmp, tol, part, c->counter(), sc, slot(0), seq0, c->stream)); }
+        FM_LAUNCH(A.precond(w.r.p, w.z.p, done, tmp != nullptr));
+        { PROF(FM_PROF_VECTOR, 1); return fm::launch_pcg_start<T>(n, w.r.p, w.z.p, b, w.p.p, part, c->counter(), sc, c->stream); }
+    };
+    auto iteration = [&](int k) -> cudaError_t {
         c->rep_seq = seq0 + (unsigned)k;
-        if (k > 1) { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_update_p<T>(n, w.z.p, w.p.p, sc, c->stream); }
-        A.spmv(w.p.p, w.Ap.p, &sc->pAp, done);
+        if (k > 1) { PROF(FM_PROF_VECTOR, 1); FM_LAUNCH(fm::launch_pcg_update_p<T>(n, w.z.p, w.p.p, sc, c->stream)); }
+        FM_LAUNCH(A.spmv(w.p.p, w.Ap.p, &sc->pAp, done));
         T* t = A.prefill();
-        { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_update_xr<T>(n, w.p.p, w.Ap.p, x, w.r.p, t, sc, c->stream); }
-        A.precond(w.r.p, w.z.p, done, t != nullptr);
-        { PROF(FM_PROF_VECTOR, 1); fm::launch_pcg_rz<T>(n, w.r.p, w.z.p, tol, part, c->counter(), sc, slot(k), seq0 + (unsigned)k, c->stream); }
+        { PROF(FM_PROF_VECTOR, 1); FM_LAUNCH(fm::launch_pcg_update_xr<T>(n, w.p.p, w.Ap.p, x, w.r.p, t, sc, c->stream)); }
+        FM_LAUNCH(A.precond(w.r.p, w.z.p, done, t != nullptr));
+        { PROF(FM_PROF_VECTOR, 1); return fm::launch_pcg_rz<T>(n, w.r.p, w.z.p, tol, part, c->counter(), sc, slot(k), seq0 + (unsigned)k, c->stream); }
+    };
+    // A kernel that could not be launched ends the solve: the kernels behind it
+    // would compute on what the ones before left.
+    auto launched = [&](cudaError_t e) -> fm_status {
+        if (e == cudaSuccess) return FM_OK;
+        cudaGetLastError();  // reported here, not by a later call
+        return fail(c, FM_ERR_CUDA, "pcg: a kernel launch failed: %s", cudaGetErrorString(e));
     };
     int iters = max_iter, ran = 0;
     bool early = false;
     double relres = 0.0;
+    fm_status queued = launched(entry());
     for (int k = 0; k <= max_iter; ++k) {
-        if (k < max_iter) iteration(k + 1);
+        if (k < max_iter && queued == FM_OK) queued = launched(iteration(k + 1));
         ran = k;
         fm::PcgReport rep;
-        fm_status st = wait_report(c, seq0 + (unsigned)k, &rep);
+        fm_status st = queued;
+        if (st == FM_OK) st = wait_report(c, seq0 + (unsigned)k, &rep);
         if (st == FM_OK) st = check_flags(c, rep.status, "pcg");
         if (st != FM_OK) {
             cudaStreamSynchronize(c->stream);
@@ -1304,8 +1312,7 @@ fm_status fm_ilu0_apply(fm_ctx* c, const double* r, double* y) {
     if (!r || !y) return fail(c, FM_ERR_ARG, "null argument");
     Op<double> A{c, &c->fem, true, c->w64.K.p, c->w64.LU.p, c->w64.diag.p, c->w64.t.p,
                  c->grid_trsv64, c->w64.dinv.p};
-    A.precond(r, y);
-    CK(cudaGetLastError());
+    CK(A.precond(r, y));
     uint32_t flags;
     TRY(device_flags(c, &flags));
     return check_flags(c, flags, "fm_ilu0_apply");
@@ -1369,8 +1376,7 @@ fm_status fm_ilu0_apply_noalloc(fm_ctx* c, const double* r, double* y) {
     CK(cudaMemsetAsync(&sp->status, 0, sizeof(unsigned), c->stream));
     CK(cudaMemcpyAsync(&sp->wait_budget, &c->sc.p->wait_budget, sizeof(unsigned),
                        cudaMemcpyDeviceToDevice, c->stream));
-    precond_nodes<double>(c, c->w64.LU.p, c->w64.dinv.p, r, sp->z, y, &sp->status);
-    CK(cudaGetLastError());
+    CK(precond_nodes<double>(c, c->w64.LU.p, c->w64.dinv.p, r, sp->z, y, &sp->status));
     unsigned flags = 0;
     CK(cudaMemcpyAsync(&flags, &sp->status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -1381,8 +1387,7 @@ fm_status fm_spmv(fm_ctx* c, const double* x, double* y) {
     TRY(need_mesh(c));
     if (!x || !y || !c->w64.K.p) return fail(c, FM_ERR_ARG, "null argument or no K");
     Op<double> A{c, &c->fem, true, c->w64.K.p, nullptr, nullptr, nullptr, 0};
-    A.spmv(x, y, nullptr);
-    CK(cudaGetLastError());
+    CK(A.spmv(x, y, nullptr));
     return FM_OK;
 }
 
@@ -1544,7 +1549,7 @@ fm_status fm_newton_step_cfg(fm_ctx* c, double* u, double load_frac, const fm_ne
                 float* part = reinterpret_cast<float*>(c->partials.p);
                 {
                     PROF(FM_PROF_SPMV, 1);
-                    spmv_nodes<float>(c, c->w32.K.p, c->w32.x.p, c->w32.Ap.p, nullptr);
+                    CK(spmv_nodes<float>(c, c->w32.K.p, c->w32.x.p, c->w32.Ap.p, nullptr));
                 }
                 {
                     PROF(FM_PROF_VECTOR, 2);
@@ -1612,13 +1617,13 @@ fm_status fm_newton_step_cfg(fm_ctx* c, double* u, double load_frac, const fm_ne
             double* f = c->vec_c.p;
             if (mixed) {
                 { PROF(FM_PROF_ASSEMBLE, 1); fm::launch_assemble(m, u, c->w32.K.p, f, nullptr, 0, c->status(), c->stream); }
-                { PROF(FM_PROF_SPMV, 1); spmv_nodes<float>(c, c->w32.K.p, c->w32.b.p, c->w32.Ap.p, nullptr); }
+                { PROF(FM_PROF_SPMV, 1); CK(spmv_nodes<float>(c, c->w32.K.p, c->w32.b.p, c->w32.Ap.p, nullptr)); }
                 { PROF(FM_PROF_VECTOR, 1); fm::launch_predictor_rhs<float>(c->n, c->mask.p, f, c->w32.Ap.p, R, c->stream); }
                 { PROF(FM_PROF_VECTOR, 1); fm::launch_apply_bc_nodes<float>(c->nn, c->nbr_ptr.p, c->nbr.p, c->mask.p,
                                                  c->w32.K.p, c->stream); }
             } else {
                 { PROF(FM_PROF_ASSEMBLE, 1); fm::launch_assemble(m, u, c->w64.K.p, f, nullptr, 0, c->status(), c->stream); }
-                { PROF(FM_PROF_SPMV, 1); spmv_nodes<double>(c, c->w64.K.p, v, c->w64.Ap.p, nullptr); }
+                { PROF(FM_PROF_SPMV, 1); CK(spmv_nodes<double>(c, c->w64.K.p, v, c->w64.Ap.p, nullptr)); }
                 { PROF(FM_PROF_VECTOR, 1); fm::launch_predictor_rhs<double>(c->n, c->mask.p, f, c->w64.Ap.p, R, c->stream); }
                 { PROF(FM_PROF_VECTOR, 1); fm::launch_apply_bc_nodes<double>(c->nn, c->nbr_ptr.p, c->nbr.p, c->mask.p,
                                                   c->w64.K.p, c->stream); }

@@ -100,14 +100,19 @@ __device__ __forceinline__ void chain_begin() {
     chain_let_next();
     chain_wait();
 }
-template <typename... P, typename... A>
-cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
-                           cudaStream_t s, A... args) {
+inline cudaLaunchConfig_t launch_config(unsigned grid, unsigned block, size_t smem,
+                                        cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
+    return cfg;
+}
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                           cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = launch_config(grid, block, smem, s);
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -115,6 +120,20 @@ cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, 
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
+// an ordinary launch that returns its own status (<<<>>> leaves it to be
+// fetched from the thread's last error, with whatever was there before)
+template <typename... P, typename... A>
+cudaError_t launch_plain(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                         cudaStream_t s, A... args) {
+    const cudaLaunchConfig_t cfg = launch_config(grid, block, smem, s);
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+// a launcher of several kernels stops at the first one that is refused
+#define FM_LAUNCH(call)                              \
+    do {                                             \
+        const cudaError_t e_ = (call);               \
+        if (e_ != cudaSuccess) return e_;            \
+    } while (0)
 
 // *skip set (null: never): the kernel has nothing to do
 __device__ __forceinline__ bool skipped(const unsigned* skip) {

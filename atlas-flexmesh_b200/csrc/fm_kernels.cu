@@ -698,26 +698,26 @@ __global__ void __launch_bounds__(256)
 }
 
 template <typename T, int G>
-static void launch_spmv_csr_g(uint32_t n, const uint32_t* rp, const uint32_t* ci, const T* val,
-                              const T* x, T* y, T* partials, unsigned* counter, double* dot,
-                              cudaStream_t s, const unsigned* skip) {
+static cudaError_t launch_spmv_csr_g(uint32_t n, const uint32_t* rp, const uint32_t* ci,
+                                     const T* val, const T* x, T* y, T* partials,
+                                     unsigned* counter, double* dot, cudaStream_t s,
+                                     const unsigned* skip) {
     const uint32_t per = 256 / G;  // rows per block and step
     const int grid = (int)std::min<uint32_t>(kSpmvBlocks, std::max(1u, (n + per - 1) / per));
-    launch_chained(k_spmv_csr<T, G>, grid, 256, 0, s, n, rp, ci, val, x, y, partials, counter, dot,
-                   skip);
+    return launch_chained(k_spmv_csr<T, G>, grid, 256, 0, s, n, rp, ci, val, x, y, partials,
+                          counter, dot, skip);
 }
 
 template <typename T>
-void launch_spmv_csr(uint32_t n, uint64_t nnz, const uint32_t* rp, const uint32_t* ci,
-                     const T* val, const T* x, T* y, T* partials, unsigned* counter, double* dot,
-                     cudaStream_t s, const unsigned* skip) {
+cudaError_t launch_spmv_csr(uint32_t n, uint64_t nnz, const uint32_t* rp, const uint32_t* ci,
+                            const T* val, const T* x, T* y, T* partials, unsigned* counter,
+                            double* dot, cudaStream_t s, const unsigned* skip) {
     const uint64_t mean = n ? nnz / n : 0;
     if (mean <= 6)
-        launch_spmv_csr_g<T, 4>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
-    else if (mean <= 16)
-        launch_spmv_csr_g<T, 8>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
-    else
-        launch_spmv_csr_g<T, 32>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
+        return launch_spmv_csr_g<T, 4>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
+    if (mean <= 16)
+        return launch_spmv_csr_g<T, 8>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
+    return launch_spmv_csr_g<T, 32>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
 }
 
 // ===========================================================================
@@ -881,19 +881,20 @@ void launch_ilu0_csr(const CsrDev& A, const T* a_val, T* lu, T* diag, unsigned* 
                                                                              done, epoch, status);
 }
 template <typename T>
-void launch_trsv_lower_csr(const CsrDev& A, const T* lu, const T* r, T* z, unsigned* done,
-                           unsigned epoch, unsigned* status, int grid, cudaStream_t s,
-                           const unsigned* skip) {
-    if (!A.n) return;
-    k_trsv_lower_csr<T><<<grid, kSfWarps * 32, 0, s>>>(A, lu, r, z, done, epoch, status, skip);
+cudaError_t launch_trsv_lower_csr(const CsrDev& A, const T* lu, const T* r, T* z, unsigned* done,
+                                  unsigned epoch, unsigned* status, int grid, cudaStream_t s,
+                                  const unsigned* skip) {
+    if (!A.n) return cudaSuccess;
+    return launch_plain(k_trsv_lower_csr<T>, grid, kSfWarps * 32, 0, s, A, lu, r, z, done, epoch,
+                        status, skip);
 }
 template <typename T>
-void launch_trsv_upper_csr(const CsrDev& A, const T* lu, const T* diag, const T* z, T* y,
-                           unsigned* done, unsigned epoch, unsigned* status, int grid,
-                           cudaStream_t s, const unsigned* skip) {
-    if (!A.n) return;
-    k_trsv_upper_csr<T><<<grid, kSfWarps * 32, 0, s>>>(A, lu, diag, z, y, done, epoch, status,
-                                                       skip);
+cudaError_t launch_trsv_upper_csr(const CsrDev& A, const T* lu, const T* diag, const T* z, T* y,
+                                  unsigned* done, unsigned epoch, unsigned* status, int grid,
+                                  cudaStream_t s, const unsigned* skip) {
+    if (!A.n) return cudaSuccess;
+    return launch_plain(k_trsv_upper_csr<T>, grid, kSfWarps * 32, 0, s, A, lu, diag, z, y, done,
+                        epoch, status, skip);
 }
 
 // All blocks of a sync-free kernel must be resident at once (rows wait on
@@ -970,11 +971,11 @@ __global__ void __launch_bounds__(kVecThreads)
     });
 }
 template <typename T>
-void launch_pcg_init(uint32_t n, const T* b, T* r, bool zero_x, T* tmp, double tol, T* partials,
-                     unsigned* counter, DevScalars* sc, PcgReport* rep, unsigned seq,
-                     cudaStream_t s) {
-    launch_chained(k_pcg_init<T>, red_blocks(n), kVecThreads, 0, s, n, b, r, zero_x, tmp, tol,
-                   partials, counter, sc, rep, seq);
+cudaError_t launch_pcg_init(uint32_t n, const T* b, T* r, bool zero_x, T* tmp, double tol,
+                            T* partials, unsigned* counter, DevScalars* sc, PcgReport* rep,
+                            unsigned seq, cudaStream_t s) {
+    return launch_chained(k_pcg_init<T>, red_blocks(n), kVecThreads, 0, s, n, b, r, zero_x, tmp,
+                          tol, partials, counter, sc, rep, seq);
 }
 
 // p = z; rz = r.z; bb = b.b.  Two sums share one pass (partials: 2 slots per block)
@@ -1005,10 +1006,10 @@ __global__ void __launch_bounds__(kVecThreads)
                           [&](T total) { sc->bb = (double)total; });
 }
 template <typename T>
-void launch_pcg_start(uint32_t n, const T* r, const T* z, const T* b, T* p, T* partials,
-                      unsigned* counter, DevScalars* sc, cudaStream_t s) {
-    launch_chained(k_pcg_start<T>, red_blocks(n), kVecThreads, 0, s, n, r, z, b, p, partials,
-                   counter, sc);
+cudaError_t launch_pcg_start(uint32_t n, const T* r, const T* z, const T* b, T* p, T* partials,
+                             unsigned* counter, DevScalars* sc, cudaStream_t s) {
+    return launch_chained(k_pcg_start<T>, red_blocks(n), kVecThreads, 0, s, n, r, z, b, p,
+                          partials, counter, sc);
 }
 
 // alpha = rz/pAp (current rz is rz_new); breakdown |pAp| < 1e-60 stops
@@ -1036,10 +1037,10 @@ __global__ void __launch_bounds__(kVecThreads)
     }
 }
 template <typename T>
-void launch_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* x, T* r, T* tmp, DevScalars* sc,
-                          cudaStream_t s) {
-    launch_chained(k_pcg_update_xr<T>, 2 * red_blocks(n), kVecThreads, 0, s, n, p, Ap, x, r, tmp,
-                   sc);
+cudaError_t launch_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* x, T* r, T* tmp,
+                                 DevScalars* sc, cudaStream_t s) {
+    return launch_chained(k_pcg_update_xr<T>, 2 * red_blocks(n), kVecThreads, 0, s, n, p, Ap, x, r,
+                          tmp, sc);
 }
 
 // rz <- rz_new (old value kept for beta), rz_new <- r.z, relres, the stop
@@ -1075,10 +1076,11 @@ __global__ void __launch_bounds__(kVecThreads)
     });
 }
 template <typename T>
-void launch_pcg_rz(uint32_t n, const T* r, const T* z, double tol, T* partials, unsigned* counter,
-                   DevScalars* sc, PcgReport* rep, unsigned seq, cudaStream_t s) {
-    launch_chained(k_pcg_rz<T>, red_blocks(n), kVecThreads, 0, s, n, r, z, tol, partials, counter,
-                   sc, rep, seq);
+cudaError_t launch_pcg_rz(uint32_t n, const T* r, const T* z, double tol, T* partials,
+                          unsigned* counter, DevScalars* sc, PcgReport* rep, unsigned seq,
+                          cudaStream_t s) {
+    return launch_chained(k_pcg_rz<T>, red_blocks(n), kVecThreads, 0, s, n, r, z, tol, partials,
+                          counter, sc, rep, seq);
 }
 
 template <typename T>
@@ -1093,8 +1095,8 @@ __global__ void __launch_bounds__(kVecThreads)
         p[i] = z[i] + beta * p[i];
 }
 template <typename T>
-void launch_pcg_update_p(uint32_t n, const T* z, T* p, DevScalars* sc, cudaStream_t s) {
-    launch_chained(k_pcg_update_p<T>, 2 * red_blocks(n), kVecThreads, 0, s, n, z, p, sc);
+cudaError_t launch_pcg_update_p(uint32_t n, const T* z, T* p, DevScalars* sc, cudaStream_t s) {
+    return launch_chained(k_pcg_update_p<T>, 2 * red_blocks(n), kVecThreads, 0, s, n, z, p, sc);
 }
 
 __global__ void k_set_bc_values(uint32_t n, const uint8_t* __restrict__ mask,
@@ -1267,28 +1269,30 @@ template void launch_apply_bc_nodes<double>(uint32_t, const uint32_t*, const uin
 template void launch_apply_bc_nodes<float>(uint32_t, const uint32_t*, const uint32_t*,
                                            const uint8_t*, float*, cudaStream_t);
 #define FM_INST(T)                                                                              \
-    template void launch_spmv_csr<T>(uint32_t, uint64_t, const uint32_t*, const uint32_t*,      \
-                                     const T*, const T*, T*, T*, unsigned*, double*,            \
-                                     cudaStream_t, const unsigned*);                            \
+    template cudaError_t launch_spmv_csr<T>(uint32_t, uint64_t, const uint32_t*,                \
+                                            const uint32_t*, const T*, const T*, T*, T*,        \
+                                            unsigned*, double*, cudaStream_t, const unsigned*); \
     template void launch_ilu0_csr<T>(const CsrDev&, const T*, T*, T*, unsigned*, unsigned,      \
                                      unsigned*, int, cudaStream_t);                             \
-    template void launch_trsv_lower_csr<T>(const CsrDev&, const T*, const T*, T*, unsigned*,    \
-                                           unsigned, unsigned*, int, cudaStream_t,              \
-                                           const unsigned*);                                    \
-    template void launch_trsv_upper_csr<T>(const CsrDev&, const T*, const T*, const T*, T*,     \
-                                           unsigned*, unsigned, unsigned*, int, cudaStream_t,   \
-                                           const unsigned*);                                    \
+    template cudaError_t launch_trsv_lower_csr<T>(const CsrDev&, const T*, const T*, T*,        \
+                                                  unsigned*, unsigned, unsigned*, int,          \
+                                                  cudaStream_t, const unsigned*);               \
+    template cudaError_t launch_trsv_upper_csr<T>(const CsrDev&, const T*, const T*, const T*,  \
+                                                  T*, unsigned*, unsigned, unsigned*, int,      \
+                                                  cudaStream_t, const unsigned*);               \
     template void launch_dot<T>(uint32_t, const T*, const T*, T*, unsigned*, double*,           \
                                 cudaStream_t);                                                  \
-    template void launch_pcg_init<T>(uint32_t, const T*, T*, bool, T*, double, T*, unsigned*,   \
-                                     DevScalars*, PcgReport*, unsigned, cudaStream_t);          \
-    template void launch_pcg_start<T>(uint32_t, const T*, const T*, const T*, T*, T*,           \
-                                      unsigned*, DevScalars*, cudaStream_t);                    \
-    template void launch_pcg_update_xr<T>(uint32_t, const T*, const T*, T*, T*, T*,             \
-                                          DevScalars*, cudaStream_t);                           \
-    template void launch_pcg_rz<T>(uint32_t, const T*, const T*, double, T*, unsigned*,         \
-                                   DevScalars*, PcgReport*, unsigned, cudaStream_t);            \
-    template void launch_pcg_update_p<T>(uint32_t, const T*, T*, DevScalars*, cudaStream_t);
+    template cudaError_t launch_pcg_init<T>(uint32_t, const T*, T*, bool, T*, double, T*,       \
+                                            unsigned*, DevScalars*, PcgReport*, unsigned,       \
+                                            cudaStream_t);                                      \
+    template cudaError_t launch_pcg_start<T>(uint32_t, const T*, const T*, const T*, T*, T*,    \
+                                             unsigned*, DevScalars*, cudaStream_t);             \
+    template cudaError_t launch_pcg_update_xr<T>(uint32_t, const T*, const T*, T*, T*, T*,      \
+                                                 DevScalars*, cudaStream_t);                    \
+    template cudaError_t launch_pcg_rz<T>(uint32_t, const T*, const T*, double, T*, unsigned*,  \
+                                          DevScalars*, PcgReport*, unsigned, cudaStream_t);     \
+    template cudaError_t launch_pcg_update_p<T>(uint32_t, const T*, T*, DevScalars*,            \
+                                                cudaStream_t);
 FM_INST(double)
 FM_INST(float)
 #undef FM_INST

@@ -72,11 +72,13 @@ cudaError_t launch_spmv_nodes(uint32_t n_nodes, uint32_t max_deg, const uint32_t
                               const uint32_t* nbr, const T* val, const T* x, T* y, T* partials,
                               unsigned* counter, double* dot, unsigned* status, cudaStream_t s,
                               const unsigned* skip = nullptr);
-// Generic scalar CSR SpMV (ascending or any column order)
+// Generic scalar CSR SpMV (ascending or any column order).  This and the
+// launchers below that return a cudaError_t return their first launch's
+// failure, with the kernels before it already queued.
 template <typename T>
-void launch_spmv_csr(uint32_t n, uint64_t nnz, const uint32_t* rp, const uint32_t* ci,
-                     const T* val, const T* x, T* y, T* partials, unsigned* counter, double* dot,
-                     cudaStream_t s, const unsigned* skip = nullptr);
+cudaError_t launch_spmv_csr(uint32_t n, uint64_t nnz, const uint32_t* rp, const uint32_t* ci,
+                            const T* val, const T* x, T* y, T* partials, unsigned* counter,
+                            double* dot, cudaStream_t s, const unsigned* skip = nullptr);
 
 // Sync-free ILU(0) and triangular solves on a CSR with ascending columns.
 // order: a topological order of the rows (dependency levels); done: one
@@ -95,13 +97,13 @@ template <typename T>
 void launch_ilu0_csr(const CsrDev& A, const T* a_val, T* lu, T* diag, unsigned* done,
                      unsigned epoch, unsigned* status, int grid, cudaStream_t s);
 template <typename T>
-void launch_trsv_lower_csr(const CsrDev& A, const T* lu, const T* r, T* z, unsigned* done,
-                           unsigned epoch, unsigned* status, int grid, cudaStream_t s,
-                           const unsigned* skip = nullptr);
+cudaError_t launch_trsv_lower_csr(const CsrDev& A, const T* lu, const T* r, T* z, unsigned* done,
+                                  unsigned epoch, unsigned* status, int grid, cudaStream_t s,
+                                  const unsigned* skip = nullptr);
 template <typename T>
-void launch_trsv_upper_csr(const CsrDev& A, const T* lu, const T* diag, const T* z, T* y,
-                           unsigned* done, unsigned epoch, unsigned* status, int grid,
-                           cudaStream_t s, const unsigned* skip = nullptr);
+cudaError_t launch_trsv_upper_csr(const CsrDev& A, const T* lu, const T* diag, const T* z, T* y,
+                                  unsigned* done, unsigned epoch, unsigned* status, int grid,
+                                  cudaStream_t s, const unsigned* skip = nullptr);
 // persistent grid sizes (all blocks co-resident) for the sync-free kernels
 int persistent_grid_ilu0_csr(int device, bool fp32, const CsrDev& A);
 int persistent_grid_trsv_csr(int device, bool fp32);
@@ -140,24 +142,25 @@ void launch_dot(uint32_t n, const T* x, const T* y, T* partials, unsigned* count
 // r = b - r (r holds A x on entry; zero_x: r = b), rr = r.r, stop = 0, done =
 // early exit (sqrt(rr) < tol 1e-3); tmp (nullable) = wait sentinel
 template <typename T>
-void launch_pcg_init(uint32_t n, const T* b, T* r, bool zero_x, T* tmp, double tol, T* partials,
-                     unsigned* counter, DevScalars* sc, PcgReport* rep, unsigned seq,
-                     cudaStream_t s);
+cudaError_t launch_pcg_init(uint32_t n, const T* b, T* r, bool zero_x, T* tmp, double tol,
+                            T* partials, unsigned* counter, DevScalars* sc, PcgReport* rep,
+                            unsigned seq, cudaStream_t s);
 // p = z; rz = r.z; bb = b.b (both into sc)
 template <typename T>
-void launch_pcg_start(uint32_t n, const T* r, const T* z, const T* b, T* p, T* partials,
-                      unsigned* counter, DevScalars* sc, cudaStream_t s);
+cudaError_t launch_pcg_start(uint32_t n, const T* r, const T* z, const T* b, T* p, T* partials,
+                             unsigned* counter, DevScalars* sc, cudaStream_t s);
 // alpha = rz/pAp; x += alpha p; r -= alpha Ap; tmp (nullable) = wait sentinel
 template <typename T>
-void launch_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* x, T* r, T* tmp, DevScalars* sc,
-                          cudaStream_t s);
+cudaError_t launch_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* x, T* r, T* tmp,
+                                 DevScalars* sc, cudaStream_t s);
 // rz_new = r.z; relres = sqrt(rz_new / max(bb,1e-300)); done when relres < tol
 template <typename T>
-void launch_pcg_rz(uint32_t n, const T* r, const T* z, double tol, T* partials, unsigned* counter,
-                   DevScalars* sc, PcgReport* rep, unsigned seq, cudaStream_t s);
+cudaError_t launch_pcg_rz(uint32_t n, const T* r, const T* z, double tol, T* partials,
+                          unsigned* counter, DevScalars* sc, PcgReport* rep, unsigned seq,
+                          cudaStream_t s);
 // beta = rz_new/rz; p = z + beta p
 template <typename T>
-void launch_pcg_update_p(uint32_t n, const T* z, T* p, DevScalars* sc, cudaStream_t s);
+cudaError_t launch_pcg_update_p(uint32_t n, const T* z, T* p, DevScalars* sc, cudaStream_t s);
 
 // Newton helpers
 void launch_set_bc_values(uint32_t n, const uint8_t* mask, const double* val, double frac,

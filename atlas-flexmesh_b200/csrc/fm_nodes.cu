@@ -451,8 +451,8 @@ static int grid_for(int resident, uint32_t max_width) {
 }
 
 template <typename T>
-void launch_fill_sentinel(uint32_t n, T* x, cudaStream_t s) {
-    k_fill_sentinel<T><<<592, 256, 0, s>>>(n, x);
+cudaError_t launch_fill_sentinel(uint32_t n, T* x, cudaStream_t s) {
+    return launch_plain(k_fill_sentinel<T>, 592, 256, 0, s, n, x);
 }
 
 template <typename T>
@@ -480,7 +480,7 @@ template void launch_ilu0_nodes<double>(const NodeSched&, const double*, double*
                                         double*, double*, unsigned*, int, cudaStream_t);
 template void launch_ilu0_nodes<float>(const NodeSched&, const float*, float*, uint64_t, float*,
                                        float*, unsigned*, int, cudaStream_t);
-template void launch_fill_sentinel<double>(uint32_t, double*, cudaStream_t);
-template void launch_fill_sentinel<float>(uint32_t, float*, cudaStream_t);
+template cudaError_t launch_fill_sentinel<double>(uint32_t, double*, cudaStream_t);
+template cudaError_t launch_fill_sentinel<float>(uint32_t, float*, cudaStream_t);
 
 }  // namespace fm

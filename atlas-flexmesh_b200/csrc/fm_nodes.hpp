@@ -28,11 +28,12 @@ struct NodeSched {
 
 // y = U^-1 L^-1 r using tmp for the intermediate (both overwritten);
 // dinv holds the reciprocal pivots written by the factorization; skip (null:
-// never): a device word that, when set, makes the kernels return at once
+// never): a device word that, when set, makes the kernels return at once.
+// Returns the first launch error.
 template <typename T>
-void launch_trsv_nodes(const NodeSched& S, const T* lu, const T* dinv, const T* r, T* tmp, T* y,
-                       unsigned* status, int device, cudaStream_t s,
-                       const unsigned* skip = nullptr);
+cudaError_t launch_trsv_nodes(const NodeSched& S, const T* lu, const T* dinv, const T* r, T* tmp,
+                              T* y, unsigned* status, int device, cudaStream_t s,
+                              const unsigned* skip = nullptr);
 // LU (nnz entries, a_ii kept on diagonal slots), pivots d and their
 // reciprocals dinv (three kernels: LU and dinv filled with the wait
 // sentinel, then the factorization)
@@ -40,7 +41,7 @@ template <typename T>
 void launch_ilu0_nodes(const NodeSched& S, const T* a, T* lu, uint64_t nnz, T* d, T* dinv,
                        unsigned* status, int device, cudaStream_t s);
 template <typename T>
-void launch_fill_sentinel(uint32_t n, T* x, cudaStream_t s);
+cudaError_t launch_fill_sentinel(uint32_t n, T* x, cudaStream_t s);
 
 // Slab-partitioned push solves (fm_trsv_push.cu) on the plan of
 // fm_setup.cpp push_plan: CTA g of the grid (clusters of `cluster` CTAs)

@@ -222,28 +222,29 @@ static int trsv_grid(int resident, uint32_t max_width) {
 }
 
 template <typename T>
-void launch_trsv_nodes(const NodeSched& S, const T* lu, const T* dinv, const T* r, T* tmp, T* y,
-                       unsigned* status, int device, cudaStream_t s, const unsigned* skip) {
-    if (!S.n_nodes) return;
+cudaError_t launch_trsv_nodes(const NodeSched& S, const T* lu, const T* dinv, const T* r, T* tmp,
+                              T* y, unsigned* status, int device, cudaStream_t s,
+                              const unsigned* skip) {
+    if (!S.n_nodes) return cudaSuccess;
     static int res_lo[2] = {0, 0}, res_up[2] = {0, 0};
     const int f = sizeof(T) == 4;
     if (!res_lo[f]) res_lo[f] = resident_grid_trsv(k_trsv_lower_pipe<T>, device);
     if (!res_up[f]) res_up[f] = resident_grid_trsv(k_trsv_upper_pipe<T>, device);
     static const unsigned backoff = env_u("FM_TRSV_BACKOFF_NS", 0);
     const uint32_t n = 3 * S.n_nodes;
-    launch_fill_sentinel<T>(n, tmp, s);
-    k_trsv_lower_pipe<T><<<trsv_grid(res_lo[f], S.max_width_fwd), kTrsvWarps * 32, 0, s>>>(
-        S, lu, r, tmp, status, backoff, skip);
-    launch_fill_sentinel<T>(n, y, s);
-    k_trsv_upper_pipe<T><<<trsv_grid(res_up[f], S.max_width_bwd), kTrsvWarps * 32, 0, s>>>(
-        S, lu, dinv, tmp, y, status, backoff, skip);
+    FM_LAUNCH(launch_fill_sentinel<T>(n, tmp, s));
+    FM_LAUNCH(launch_plain(k_trsv_lower_pipe<T>, trsv_grid(res_lo[f], S.max_width_fwd),
+                           kTrsvWarps * 32, 0, s, S, lu, r, tmp, status, backoff, skip));
+    FM_LAUNCH(launch_fill_sentinel<T>(n, y, s));
+    return launch_plain(k_trsv_upper_pipe<T>, trsv_grid(res_up[f], S.max_width_bwd),
+                        kTrsvWarps * 32, 0, s, S, lu, dinv, tmp, y, status, backoff, skip);
 }
 
-template void launch_trsv_nodes<double>(const NodeSched&, const double*, const double*,
-                                        const double*, double*, double*, unsigned*, int,
-                                        cudaStream_t, const unsigned*);
-template void launch_trsv_nodes<float>(const NodeSched&, const float*, const float*, const float*,
-                                       float*, float*, unsigned*, int, cudaStream_t,
-                                       const unsigned*);
+template cudaError_t launch_trsv_nodes<double>(const NodeSched&, const double*, const double*,
+                                               const double*, double*, double*, unsigned*, int,
+                                               cudaStream_t, const unsigned*);
+template cudaError_t launch_trsv_nodes<float>(const NodeSched&, const float*, const float*,
+                                              const float*, float*, float*, unsigned*, int,
+                                              cudaStream_t, const unsigned*);
 
 }  // namespace fm

@@ -439,14 +439,12 @@ cudaError_t launch_trsv_push(const PushSolve& P, const NodeSched& S, const T* lu
                              const unsigned* skip, bool filled) {
     if (!S.n_nodes) return cudaSuccess;
     const uint32_t n = 3 * S.n_nodes;
-    if (!filled) launch_fill_sentinel<T>(n, tmp, s);
+    if (!filled) FM_LAUNCH(launch_fill_sentinel<T>(n, tmp, s));
     // in place (y == r) the forward solve still reads r: fill y after it
     const bool fuse = y != r;
-    cudaError_t e =
-        launch_dir<T, true>(P, S, lu, dinv, r, tmp, fuse ? y : nullptr, fuse ? n : 0, status, skip,
-                            s);
-    if (e != cudaSuccess) return e;
-    if (!fuse) launch_fill_sentinel<T>(n, y, s);
+    FM_LAUNCH((launch_dir<T, true>(P, S, lu, dinv, r, tmp, fuse ? y : nullptr, fuse ? n : 0,
+                                   status, skip, s)));
+    if (!fuse) FM_LAUNCH(launch_fill_sentinel<T>(n, y, s));
     return launch_dir<T, false>(P, S, lu, dinv, tmp, y, nullptr, 0, status, skip, s);
 }
 

@@ -80,6 +80,24 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const
     *n = 1;
     return cudaSuccess;
 }
+cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t*) {
+    *n = 15;
+    return cudaSuccess;
+}
+cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) {
+    std::memset(a, 0, sizeof *a);
+    a->ptxVersion = a->binaryVersion = 100;
+    return cudaSuccess;
+}
+cudaError_t cudaGetDeviceCount(int* n) {
+    *n = 1;
+    return cudaSuccess;
+}
+cudaError_t cudaGetSymbolAddress(void** p, const void*) {
+    static char scratch[16 << 20];
+    *p = scratch;
+    return cudaSuccess;
+}
 cudaError_t cudaMalloc(void** p, size_t n) {
     *p = std::calloc(n ? n : 1, 1);
     return *p ? cudaSuccess : fake::done(cudaErrorMemoryAllocation);

@@ -48,3 +48,12 @@ def run(prog, *args):
 
 def test_one_shared_memory_limit_per_kernel(exe):
     run(exe("launch_limits_check", ["fm_spmv.cu", "fm_trsv_small.cu"]))
+
+
+LIB = ["fm_api.cu", "fm_kernels.cu", "fm_nodes.cu", "fm_trsv.cu", "fm_trsv_push.cu",
+       "fm_trsv_small.cu", "fm_spmv.cu", "fm_adjoint.cu", "fm_states.cu", "fm_meshsetup.cu",
+       "fm_setup.cpp", "fm_checkpoint.cpp"]
+
+
+def test_refused_launches_are_reported(exe):
+    run(exe("launch_failures_check", LIB))
