@@ -730,7 +730,7 @@ fm_status pcg_core(fm_ctx* c, const Op<T>& A, uint32_t n, const T* b, T* x, doub
     bool early = false;
     double relres = 0.0;
     fm_status queued = launched(entry());
-    for (int k = 0; k <= max_iter; ++k) {
+    for (int k = 0; k == 0 || k <= max_iter; ++k) {  // the entry is judged whatever the cap
         if (k < max_iter && queued == FM_OK) queued = launched(iteration(k + 1));
         ran = k;
         fm::PcgReport rep;

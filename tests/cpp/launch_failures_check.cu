@@ -124,6 +124,28 @@ int main() {
     each_launch("csr_pcg, warp per row", csr, "k_trsv_small");
     refuse_all = nullptr;
 
+    // without iterations (a cap of zero or below) the entry still counts: its
+    // early exit is zero iterations, and its flags are an error
+    for (int cap : {0, -1}) {
+        fm_ctx* c = nullptr;
+        EXPECT(fm_create(&c, 0, nullptr) == FM_OK, "fm_create");
+        for (unsigned done : {0u, 1u}) {
+            init_done = done;
+            it = 77;
+            const fm_status st = fm_csr_pcg_ilu0(c, n, rp.data(), ci.data(), val.data(), b.data(),
+                                                 x.data(), 1e-8, cap, &it, &rel);
+            EXPECT(st == FM_OK && it == (done ? 0 : cap), "cap %d, early exit %u: status %d, %d",
+                   cap, done, (int)st, it);
+        }
+        init_done = 0;
+        report_status = FM_FLAG_NONFINITE;
+        const fm_status st = fm_csr_pcg_ilu0(c, n, rp.data(), ci.data(), val.data(), b.data(),
+                                             x.data(), 1e-8, cap, &it, &rel);
+        EXPECT(st == FM_ERR_NONFINITE, "cap %d: a non-finite entry returns %d", cap, (int)st);
+        report_status = 0;
+        fm_destroy(c);
+    }
+
     // on a mesh: one tet, whose structures the fake leaves empty
     const double xyz[12] = {0, 0, 0, 1, 0, 0, 0, 1, 0, 0, 0, 1};
     const uint32_t conn[4] = {0, 1, 2, 3};
