@@ -109,6 +109,22 @@ inline cudaLaunchConfig_t launch_config(unsigned grid, unsigned block, size_t sm
     cfg.stream = s;
     return cfg;
 }
+// A value that an earlier kernel of the chain wrote.  A chained kernel's life
+// begins before its predecessor's ends, so such a value is not constant over
+// it, as __ldg and a const __restrict__ parameter would promise (they may read
+// it through the read-only path and ahead of the wait); volatile keeps this
+// load behind chain_wait.  What was complete before the chain began (matrix,
+// factors, plans) may be read either way.
+__device__ __forceinline__ double ld_prev(const double* p) {
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_prev(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
 template <typename... P, typename... A>
 cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
                            cudaStream_t s, A... args) {

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(128, 4)
 // zero on constrained DOFs.
 __global__ void __launch_bounds__(256)
     k_gather_forces(uint32_t n_nodes, const uint32_t* __restrict__ act_ptr,
-                    const uint32_t* __restrict__ act_v, const double* __restrict__ fvert,
+                    const uint32_t* __restrict__ act_v, const double* fvert,
                     const uint8_t* __restrict__ mask, double* __restrict__ f,
                     double* __restrict__ R) {
     chain_wait();
@@ -181,11 +181,11 @@ __global__ void __launch_bounds__(256)
     for (; i + 8 <= e; i += 8) {  // eight gathers in flight
         double v[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = __ldg(fvert + 3 * (size_t)__ldg(act_v + i + q) + c);
+        for (int q = 0; q < 8; ++q) v[q] = ld_prev(fvert + 3 * (size_t)__ldg(act_v + i + q) + c);
 #pragma unroll
         for (int q = 0; q < 8; ++q) s += v[q];
     }
-    for (; i < e; ++i) s += __ldg(fvert + 3 * (size_t)__ldg(act_v + i) + c);
+    for (; i < e; ++i) s += ld_prev(fvert + 3 * (size_t)__ldg(act_v + i) + c);
     if (f) f[row] = s;
     if (R) R[row] = (mask && mask[row]) ? 0.0 : -s;
 }
@@ -667,8 +667,8 @@ constexpr int kSpmvBlocks = 148 * 8;
 template <typename T, int G>
 __global__ void __launch_bounds__(256)
     k_spmv_csr(uint32_t n, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
-               const T* __restrict__ val, const T* __restrict__ x, T* __restrict__ y,
-               T* partials, unsigned* counter, double* dot, const unsigned* __restrict__ skip) {
+               const T* __restrict__ val, const T* x, T* __restrict__ y, T* partials,
+               unsigned* counter, double* dot, const unsigned* skip) {
     chain_begin();
     if (skipped(skip)) return;
     const int lane = threadIdx.x & (G - 1);
@@ -682,12 +682,12 @@ __global__ void __launch_bounds__(256)
         T s = T(0);
         if (i < n)
             for (uint32_t k = rp[i] + lane; k < rp[i + 1]; k += G)
-                s += __ldg(val + k) * __ldg(x + ci[k]);
+                s += __ldg(val + k) * ld_prev(x + ci[k]);
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
         if (i < n && lane == 0) {
             y[i] = s;
-            if (dot) dsum += s * x[i];
+            if (dot) dsum += s * ld_prev(x + i);
         }
     }
     if (dot) {
@@ -948,15 +948,18 @@ void launch_dot(uint32_t n, const T* x, const T* y, T* partials, unsigned* count
 // wait sentinel into tmp (null: none) for the solve that follows.
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
-    k_pcg_init(uint32_t n, const T* __restrict__ b, T* __restrict__ r, int zero_x,
-               T* __restrict__ tmp, double tol, T* partials, unsigned* counter, DevScalars* sc,
-               PcgReport* rep, unsigned seq) {
-    chain_begin();
+    k_pcg_init(uint32_t n, const T* b, T* __restrict__ r, int zero_x, T* __restrict__ tmp,
+               double tol, T* partials, unsigned* counter, DevScalars* sc, PcgReport* rep,
+               unsigned seq) {
+    // in this order: the kernels behind this one start when all that ran before
+    // it (the factorization among them) is complete
+    chain_wait();
+    chain_let_next();
     T s = T(0);
 #pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x) {
-        const T v = zero_x ? b[i] : b[i] - r[i];
+        const T bi = ld_prev(b + i), v = zero_x ? bi : bi - r[i];
         r[i] = v;
         if (tmp) tmp[i] = Sentinel<T>::value();
         s += v * v;
@@ -981,19 +984,18 @@ cudaError_t launch_pcg_init(uint32_t n, const T* b, T* r, bool zero_x, T* tmp, d
 // p = z; rz = r.z; bb = b.b.  Two sums share one pass (partials: 2 slots per block)
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
-    k_pcg_start(uint32_t n, const T* __restrict__ r, const T* __restrict__ z,
-                const T* __restrict__ b, T* __restrict__ p, T* partials, unsigned* counter,
-                DevScalars* sc) {
+    k_pcg_start(uint32_t n, const T* r, const T* z, const T* b, T* __restrict__ p, T* partials,
+                unsigned* counter, DevScalars* sc) {
     chain_begin();
     if (skipped(&sc->done)) return;
     T s1 = T(0), s2 = T(0);
 #pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x) {
-        const T zi = z[i];
+        const T zi = ld_prev(z + i), bi = ld_prev(b + i);
         p[i] = zi;
-        s1 += r[i] * zi;
-        s2 += b[i] * b[i];
+        s1 += ld_prev(r + i) * zi;
+        s2 += bi * bi;
     }
     __shared__ T sbuf[32];
     const T b1 = block_sum(s1, sbuf);
@@ -1018,8 +1020,8 @@ cudaError_t launch_pcg_start(uint32_t n, const T* r, const T* z, const T* b, T* 
 // triangular solves that follow.
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
-    k_pcg_update_xr(uint32_t n, const T* __restrict__ p, const T* __restrict__ Ap,
-                    T* __restrict__ x, T* __restrict__ r, T* __restrict__ tmp, DevScalars* sc) {
+    k_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* __restrict__ x, T* __restrict__ r,
+                    T* __restrict__ tmp, DevScalars* sc) {
     chain_begin();
     if (skipped(&sc->done)) return;
     const double pAp = sc->pAp;
@@ -1031,8 +1033,8 @@ __global__ void __launch_bounds__(kVecThreads)
 #pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x) {
-        x[i] += alpha * p[i];
-        r[i] -= alpha * Ap[i];
+        x[i] += alpha * ld_prev(p + i);
+        r[i] -= alpha * ld_prev(Ap + i);
         if (tmp) tmp[i] = Sentinel<T>::value();
     }
 }
@@ -1047,8 +1049,8 @@ cudaError_t launch_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* x, T* r
 // tests, and the report.  After a breakdown only the report.
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
-    k_pcg_rz(uint32_t n, const T* __restrict__ r, const T* __restrict__ z, double tol, T* partials,
-             unsigned* counter, DevScalars* sc, PcgReport* rep, unsigned seq) {
+    k_pcg_rz(uint32_t n, const T* r, const T* z, double tol, T* partials, unsigned* counter,
+             DevScalars* sc, PcgReport* rep, unsigned seq) {
     chain_begin();
     if (skipped(&sc->done)) return;
     if (ld_volatile_u32(&sc->stop)) {
@@ -1063,7 +1065,7 @@ __global__ void __launch_bounds__(kVecThreads)
 #pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x)
-        s += r[i] * z[i];
+        s += ld_prev(r + i) * ld_prev(z + i);
     __shared__ T sbuf[32];
     const T bt = block_sum(s, sbuf);
     grid_reduce_finish<T>(bt, partials, counter, [&](T total) {
@@ -1085,14 +1087,14 @@ cudaError_t launch_pcg_rz(uint32_t n, const T* r, const T* z, double tol, T* par
 
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
-    k_pcg_update_p(uint32_t n, const T* __restrict__ z, T* __restrict__ p, const DevScalars* sc) {
+    k_pcg_update_p(uint32_t n, const T* z, T* __restrict__ p, const DevScalars* sc) {
     chain_begin();
     if (skipped(&sc->done)) return;
     const T beta = (T)(sc->rz_new / sc->rz);
 #pragma unroll 4
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x)
-        p[i] = z[i] + beta * p[i];
+        p[i] = ld_prev(z + i) + beta * p[i];
 }
 template <typename T>
 cudaError_t launch_pcg_update_p(uint32_t n, const T* z, T* p, DevScalars* sc, cudaStream_t s) {

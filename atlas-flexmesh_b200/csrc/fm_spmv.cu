@@ -115,8 +115,8 @@ template <typename T, int S>
 __global__ void __launch_bounds__(kStreamThreads)
     k_spmv_nodes(uint32_t nn, StageLayout L, const uint32_t* __restrict__ nbr_ptr,
                   const uint32_t* __restrict__ nbr, const T* __restrict__ val,
-                  const T* __restrict__ x, T* __restrict__ y, T* partials, unsigned* counter,
-                  double* dot, const unsigned* __restrict__ skip, unsigned* status) {
+                  const T* x, T* __restrict__ y, T* partials, unsigned* counter, double* dot,
+                  const unsigned* skip, unsigned* status) {
     extern __shared__ __align__(16) unsigned char stream_smem[];
     __shared__ __align__(8) unsigned long long full_s[S], empty_s[S];
     chain_let_next();
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kStreamThreads)
 #pragma unroll
             for (int r = 0; r < kRounds; ++r) {  // gathers in flight together
                 xv[r] = T(0);
-                if (hl + 16 * r < rl) xv[r] = __ldg(x + (3u * nl[ck[r]] + (unsigned)cq[r]));
+                if (hl + 16 * r < rl) xv[r] = ld_prev(x + (3u * nl[ck[r]] + (unsigned)cq[r]));
             }
 #pragma unroll
             for (int r = 0; r < kRounds; ++r)
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kStreamThreads)
                 }
             // nodes of more than 21 neighbours
             for (int idx = hl + 16 * kRounds; 16 * kRounds < most && idx < rl; idx += 16) {
-                const T xi = __ldg(x + (3u * nl[idx / 3] + (unsigned)(idx % 3)));
+                const T xi = ld_prev(x + (3u * nl[idx / 3] + (unsigned)(idx % 3)));
                 s0 += v[idx - hl] * xi;
                 s1 += v[rl + idx - hl] * xi;
                 s2 += v[2 * rl + idx - hl] * xi;
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kStreamThreads)
             if ((hl & 3) == 0 && hl < 12 && n < nn) {  // lanes 0, 4, 8 of the half
                 const uint32_t row = 3 * n + (uint32_t)(hl >> 2);
                 y[row] = yv;
-                if (dot) dsum += yv * x[row];
+                if (dot) dsum += yv * ld_prev(x + row);
             }
         }
     }

@@ -110,9 +110,9 @@ __device__ __forceinline__ void push_pre(const PushSolve& P, const NodeSched& S,
             for (int q = 0; q < 3; ++q) Q.a[3 * p + q] = __ldg(row + (size_t)p * rl + 3 * k + q);
     }
     const size_t b = 3 * (size_t)n;
-    Q.c[0] = __ldg(rhs + b);
-    Q.c[1] = __ldg(rhs + b + 1);
-    Q.c[2] = __ldg(rhs + b + 2);
+    Q.c[0] = ld_prev(rhs + b);
+    Q.c[1] = ld_prev(rhs + b + 1);
+    Q.c[2] = ld_prev(rhs + b + 2);
     if (Lower) {
         Q.c[3] = __ldg(row + rl + ds);          // L(3n+1, 3n)
         Q.c[4] = __ldg(row + 2 * rl + ds);      // L(3n+2, 3n)
@@ -258,9 +258,8 @@ __device__ __forceinline__ uint4 shfl4(uint4 v, int src, unsigned m) {
 template <typename T, bool Lower>
 __global__ void __launch_bounds__(push_max_warps(sizeof(T)) * 32, 1)
     k_trsv_push(PushSolve P, NodeSched S, const T* __restrict__ lu, const T* __restrict__ dinv,
-                const T* __restrict__ rhs, T* __restrict__ out, T* __restrict__ fill,
-                uint32_t n_fill, unsigned* __restrict__ status,
-                const unsigned* __restrict__ skip) {
+                const T* rhs, T* __restrict__ out, T* __restrict__ fill, uint32_t n_fill,
+                unsigned* __restrict__ status, const unsigned* skip) {
     chain_let_next();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(16) T zero_slot[4];

@@ -90,8 +90,8 @@ __device__ __forceinline__ void sweep(const SmallTri& S, const uint32_t* lvl, ui
 
 template <int M, int D, int Threads, bool Wide>
 __global__ void __launch_bounds__(Threads, 1)
-    k_trsv_small(SmallTri L, SmallTri U, uint32_t n, const double* __restrict__ r,
-                 double* __restrict__ out, const unsigned* __restrict__ skip) {
+    k_trsv_small(SmallTri L, SmallTri U, uint32_t n, const double* r, double* out,
+                 const unsigned* skip) {
     chain_begin();
     if (skipped(skip)) return;
     extern __shared__ __align__(16) unsigned char small_smem[];
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(Threads, 1)
     uint32_t* lf = reinterpret_cast<uint32_t*>(z + n + 1);
     uint32_t* lb = lf + L.n_levels + 1 + D;
 #pragma unroll 8
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) z[i] = r[i];
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) z[i] = ld_prev(r + i);
     if (threadIdx.x == 0) z[n] = 0.0;
     for (uint32_t i = threadIdx.x; i <= L.n_levels + D; i += blockDim.x)
         lf[i] = i < L.n_levels ? __ldg(L.level + i) : n;
