@@ -336,12 +336,13 @@ fm_status setup_small_tri(fm_ctx* c, SolverCsr& S, const std::vector<uint32_t>& 
         most = std::max({most, dpos[i] - rp[i], rp[i + 1] - upos[i]});
     S.nl_f = (uint32_t)fp.size() - 1;
     S.nl_b = (uint32_t)bp.size() - 1;
+    const uint32_t M = most <= 2 ? 2 : most <= 4 ? 4 : 8;
     if (most > fm::kSmallMaxEntries ||
-        fm::small_tri_smem(n, S.nl_f, S.nl_b) > fm::kSmallMaxSmem)
+        fm::small_tri_smem(n, S.nl_f, S.nl_b) > fm::kSmallMaxSmem ||
+        !fm::small_tri_pays(M, n, fp, bp))
         return FM_OK;
     for (const auto* p : {&fp, &bp})
         for (size_t l = 0; l + 1 < p->size(); ++l) width = std::max(width, (*p)[l + 1] - (*p)[l]);
-    const uint32_t M = most <= 2 ? 2 : most <= 4 ? 4 : 8;
     std::vector<uint32_t> col((size_t)M * n), src((size_t)M * n);
     for (int lower = 1; lower >= 0; --lower) {
         const std::vector<uint32_t>& ord = lower ? fr : br;

@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <vector>
 
 #include "fm_device.cuh"
 
@@ -123,6 +124,10 @@ struct SmallTri {
 constexpr uint32_t kSmallMaxEntries = 8;
 constexpr size_t kSmallMaxSmem = 220 * 1024;
 size_t small_tri_smem(uint32_t n, uint32_t nlf, uint32_t nlb);
+// whether levels of these widths (level pointers of both directions) are
+// solved faster in one CTA than with a warp per row; entries: 2, 4 or 8
+bool small_tri_pays(uint32_t entries, uint32_t n, const std::vector<uint32_t>& fwd_ptr,
+                    const std::vector<uint32_t>& bwd_ptr);
 // gathers the packed coefficients of both directions from LU (src ~0u: zero)
 // and the reciprocal pivots in the backward order
 void launch_pack_small(uint32_t n, uint32_t entries, const uint32_t* src_f, const uint32_t* src_b,

@@ -17,11 +17,12 @@
 // often, took 125, 126 and 141; 16-byte packed rows 160, a cp.async ring 143;
 // a build without any loads in the loop 90).
 //
-// Used when the vector and the level pointers fit shared memory and no row
-// has more than kSmallMaxEntries off-diagonal entries on one side: longer
-// rows would leave a thread with a long serial sum, and belong to the
-// warp-per-row solves.
+// Used when the vector and the level pointers fit shared memory, no row has
+// more than kSmallMaxEntries off-diagonal entries on one side (longer rows
+// would leave a thread with a long serial sum) and the levels are not too wide
+// (small_tri_pays).  The rest belongs to the warp-per-row solves.
 #include <algorithm>
+#include <vector>
 
 #include "fm_kernels.hpp"
 
@@ -137,14 +138,20 @@ cudaError_t launch_w(const SmallTri& L, const SmallTri& U, uint32_t n, unsigned 
     return launch_chained(k_trsv_small<M, D, Threads, Wide>, 1, th, smem, s, L, U, n, r, out, skip);
 }
 
+// threads of the widest block that the registers of a row allow
+constexpr unsigned max_threads(uint32_t entries) { return entries <= 2 ? 1024 : 512; }
+// no more threads than the widest level has rows (fewer warps, a cheaper
+// barrier) or than the copies in and out can use
+unsigned threads_for(uint32_t entries, uint32_t n, uint32_t width) {
+    return std::min(max_threads(entries),
+                    std::max(32u, (std::max(width, n / 64) + 31u) & ~31u));
+}
+
 template <int M, int D, int Threads>
 cudaError_t launch_t(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t width,
                      const double* r, double* out, const unsigned* skip, cudaStream_t s) {
     const size_t smem = small_tri_smem(n, L.n_levels, U.n_levels);
-    // no more threads than the widest level has rows (fewer warps, a cheaper
-    // barrier) or than the copies in and out can use
-    const unsigned th =
-        std::min<unsigned>(Threads, std::max(32u, (std::max(width, n / 64) + 31u) & ~31u));
+    const unsigned th = threads_for(M, n, width);
     return width > th ? launch_w<M, D, Threads, true>(L, U, n, th, smem, r, out, skip, s)
                       : launch_w<M, D, Threads, false>(L, U, n, th, smem, r, out, skip, s);
 }
@@ -153,6 +160,27 @@ cudaError_t launch_t(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t 
 
 size_t small_tri_smem(uint32_t n, uint32_t nlf, uint32_t nlb) {
     return 8 * ((size_t)n + 1) + 4 * ((size_t)nlf + nlb + 2 + 2 * kMaxDepth);
+}
+
+// A level costs the warp-per-row solves about 3.9 us whatever its width (148
+// SMs take its rows at once), and one CTA half a microsecond for every block's
+// width of rows in it.  us per apply on both paths, warp per row / one CTA:
+// diagonal of 7,000 rows 17.9 / 15.1, of 14,000 21.9 / 21.6, of 27,000 27.1 /
+// 36.0; red-black five-point 90 x 90 25.7 / 21.0, 120 x 120 26.6 / 31.4, 164 x
+// 164 27.0 / 53.6; 26,000 rows in four levels 40.8 / 35.2, in three 31.5 / 33.8
+// (two entries per side), in eleven 101 / 59 (four), in eight 79 / 76 and in
+// six 54 / 75 (eight).
+bool small_tri_pays(uint32_t entries, uint32_t n, const std::vector<uint32_t>& fwd_ptr,
+                    const std::vector<uint32_t>& bwd_ptr) {
+    uint64_t turns = 0, levels = 0;
+    uint32_t width = 0;
+    for (const auto* p : {&fwd_ptr, &bwd_ptr})
+        for (size_t l = 0; l + 1 < p->size(); ++l) width = std::max(width, (*p)[l + 1] - (*p)[l]);
+    const uint32_t th = threads_for(entries, n, width);
+    for (const auto* p : {&fwd_ptr, &bwd_ptr})
+        for (size_t l = 0; l + 1 < p->size(); ++l, ++levels)
+            turns += ((*p)[l + 1] - (*p)[l] + th - 1) / th;
+    return (entries <= 4 ? 50 : 55) * turns <= 390 * levels + 250;
 }
 
 void launch_pack_small(uint32_t n, uint32_t entries, const uint32_t* src_f, const uint32_t* src_b,
@@ -166,9 +194,9 @@ void launch_pack_small(uint32_t n, uint32_t entries, const uint32_t* src_f, cons
 cudaError_t launch_trsv_small(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t entries,
                               uint32_t width, const double* r, double* out, const unsigned* skip,
                               cudaStream_t s) {
-    if (entries <= 2) return launch_t<2, 1, 1024>(L, U, n, width, r, out, skip, s);
-    if (entries <= 4) return launch_t<4, 1, 512>(L, U, n, width, r, out, skip, s);
-    return launch_t<8, 1, 512>(L, U, n, width, r, out, skip, s);
+    if (entries <= 2) return launch_t<2, 1, max_threads(2)>(L, U, n, width, r, out, skip, s);
+    if (entries <= 4) return launch_t<4, 1, max_threads(4)>(L, U, n, width, r, out, skip, s);
+    return launch_t<8, 1, max_threads(8)>(L, U, n, width, r, out, skip, s);
 }
 
 }  // namespace fm
