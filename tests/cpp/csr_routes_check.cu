@@ -63,6 +63,13 @@ static void one_cta(const char* what, bool want, uint32_t n, const Pairs& pairs)
            want ? "not in one CTA" : "in one CTA");
 }
 
+static void lanes(const char* what, int want, uint32_t n, const Pairs& pairs) {
+    solve(n, pairs);
+    for (int g : {4, 8, 32})
+        EXPECT(was(("k_spmv_csrIdLi" + std::to_string(g) + "E").c_str()) == (g == want),
+               "%s: %d lanes a row", what, g);
+}
+
 static Pairs band(uint32_t n, uint32_t k, uint32_t step) {
     Pairs p;
     for (uint32_t q = 1; q <= k; ++q)
@@ -81,6 +88,13 @@ static Pairs grid(uint32_t g, bool red_black) {
             if (i) add(id(i, j), id(i - 1, j));
             if (j) add(id(i, j), id(i, j - 1));
         }
+    return p;
+}
+// k arrowheads of m rows: each one's last row is full
+static Pairs arrows(uint32_t m, uint32_t k) {
+    Pairs p;
+    for (uint32_t q = 0; q < k; ++q)
+        for (uint32_t j = 0; j + 1 < m; ++j) p.push_back({q * m + m - 1, q * m + j});
     return p;
 }
 int main() {
@@ -113,6 +127,17 @@ int main() {
     // beyond its limits: entries, and the vector
     one_cta("nine per side", false, 900, band(900, 9, 5));
     one_cta("28600 rows", false, 28600, band(28600, 2, 7000));
+
+    // lanes per row: by the mean length, more where a long row decides
+    lanes("diagonal", 4, 3000, {});
+    lanes("five-point 64 x 64", 4, 4096, grid(64, false));
+    lanes("nine per row", 8, 4000, band(4000, 4, 9));
+    lanes("seventeen per row", 32, 4000, band(4000, 9, 9));
+    lanes("arrowhead 500", 32, 500, arrows(500, 1));
+    lanes("40 arrowheads 500", 32, 20000, arrows(500, 40));
+    lanes("400 arrowheads 500", 8, 200000, arrows(500, 400));
+    lanes("8 arrowheads 60", 32, 480, arrows(60, 8));
+    lanes("2000 arrowheads 200", 4, 400000, arrows(200, 2000));
     if (!bad) std::printf("ok\n");
     return bad != 0;
 }

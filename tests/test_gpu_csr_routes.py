@@ -1,8 +1,10 @@
-"""Generic CSR PCG on both sides of the rule that sends its triangular solves
-to one CTA: levels wider than that CTA's block with up to 4 and 8 entries per
-row and side, and shallow matrices that the warp-per-row solves take.
-Diagonally dominant matrices, so the iterates of both sides differ by
-roundings only: equal counts, x to 1e-12 of its largest entry."""
+"""Generic CSR PCG on both sides of the rules that choose its kernels: levels
+wider than the single CTA's block with up to 4 and 8 entries per row and side,
+shallow matrices that the warp-per-row solves take, and rows much longer than
+the mean (4, 8 and 32 lanes per row of the product).  Diagonally dominant
+matrices, so the iterates of both sides differ by roundings only (a row of 500
+terms rounds 500 times: 500 x 2^-53 < 1e-13 of its terms): equal counts, x to
+1e-12 of its largest entry."""
 import numpy as np
 import pytest
 
@@ -48,6 +50,10 @@ def red_black(g):
     return [(max(a, b), min(a, b)) for x, y in e for a, b in zip(x, y)]
 
 
+def arrows(m, k):
+    return [(q * m + m - 1, q * m + j) for q in range(k) for j in range(m - 1)]
+
+
 CASES = {
     # one CTA, levels wider than its block (512 threads), up to 4 and 8 entries
     "wide_three_per_side": (6000, band(6000, 3, 1100)),
@@ -60,6 +66,10 @@ CASES = {
     "red_black_60": (3600, red_black(60)),
     "red_black_120": (14400, red_black(120)),
     "two_levels": (26000, band(26000, 2, 14336)),
+    # long rows: 32 lanes, and 8 where there are too many rows for 32
+    "arrow_500": (500, arrows(500, 1)),
+    "arrows_60": (480, arrows(60, 8)),
+    "arrows_200": (50000, arrows(200, 250)),
 }
 
 
