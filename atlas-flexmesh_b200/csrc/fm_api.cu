@@ -634,8 +634,8 @@ struct Op {
         PROF(FM_PROF_SPMV, 1);
         T* part = reinterpret_cast<T*>(c->partials.p);
         if (node_block) return spmv_nodes<T>(c, K, x, y, dot, skip);
-        return fm::launch_spmv_csr<T>(S->n, S->nnz, S->rp.p, S->ci.p, K, x, y, part, c->counter(),
-                                      dot, c->stream, skip);
+        return fm::launch_spmv_csr<T>(S->n, S->nnz, S->max_row, S->rp.p, S->ci.p, K, x, y, part,
+                                      c->counter(), dot, c->stream, skip);
     }
     cudaError_t precond(const T* r, T* z, const unsigned* skip = nullptr, bool filled = false) const {
         const bool pu = node_block && (sizeof(T) == 4 ? c->pu_ok32 : c->pu_ok64);

@@ -662,8 +662,8 @@ void launch_assemble_slotmap(const MeshDev& m, const double* u, const int32_t* s
 // ===========================================================================
 constexpr int kSpmvBlocks = 148 * 8;
 
-// G lanes per row (a power of two near the mean row length: a warp per
-// five-entry row leaves 27 of its lanes idle)
+// G lanes per row (spmv_csr_lanes: a warp per five-entry row leaves 27 of its
+// lanes idle)
 template <typename T, int G>
 __global__ void __launch_bounds__(256)
     k_spmv_csr(uint32_t n, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
@@ -697,6 +697,22 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// Lanes per row from the mean length, and more where a long row is what the
+// product waits for: G lanes take about 0.156 us per G entries of the longest
+// row, and each lane more costs a row 4 ps.  us with 4 / 8 / 32 lanes: a
+// 22,500-row five-point matrix 10.5 / 11.1 / 14.2, an arrowhead matrix with a
+// row of 500 entries 28.5 / 19.9 / 13.8, 40 of them (20,000 rows) 32.6 / 23.8 /
+// 19.7, 400 of them 38.3 / 30.5 / 40.3, 2,000 of 200 26.2 / 27.6 / 61.
+static uint32_t spmv_csr_lanes(uint32_t n, uint64_t nnz, uint32_t max_row) {
+    const uint64_t mean = n ? nnz / n : 0;
+    uint32_t lanes = mean <= 6 ? 4 : mean <= 16 ? 8 : 32;
+    if (max_row <= 4 * lanes) return lanes;
+    auto cost = [&](uint32_t g) { return (uint64_t)n * g + 39000ull * max_row / g; };
+    for (uint32_t g : {8u, 32u})
+        if (g > lanes && cost(g) < cost(lanes)) lanes = g;
+    return lanes;
+}
+
 template <typename T, int G>
 static cudaError_t launch_spmv_csr_g(uint32_t n, const uint32_t* rp, const uint32_t* ci,
                                      const T* val, const T* x, T* y, T* partials,
@@ -709,15 +725,18 @@ static cudaError_t launch_spmv_csr_g(uint32_t n, const uint32_t* rp, const uint3
 }
 
 template <typename T>
-cudaError_t launch_spmv_csr(uint32_t n, uint64_t nnz, const uint32_t* rp, const uint32_t* ci,
-                            const T* val, const T* x, T* y, T* partials, unsigned* counter,
-                            double* dot, cudaStream_t s, const unsigned* skip) {
-    const uint64_t mean = n ? nnz / n : 0;
-    if (mean <= 6)
-        return launch_spmv_csr_g<T, 4>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
-    if (mean <= 16)
-        return launch_spmv_csr_g<T, 8>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
-    return launch_spmv_csr_g<T, 32>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
+cudaError_t launch_spmv_csr(uint32_t n, uint64_t nnz, uint32_t max_row, const uint32_t* rp,
+                            const uint32_t* ci, const T* val, const T* x, T* y, T* partials,
+                            unsigned* counter, double* dot, cudaStream_t s,
+                            const unsigned* skip) {
+    switch (spmv_csr_lanes(n, nnz, max_row)) {
+        case 4:
+            return launch_spmv_csr_g<T, 4>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
+        case 8:
+            return launch_spmv_csr_g<T, 8>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
+        default:
+            return launch_spmv_csr_g<T, 32>(n, rp, ci, val, x, y, partials, counter, dot, s, skip);
+    }
 }
 
 // ===========================================================================
@@ -1271,7 +1290,7 @@ template void launch_apply_bc_nodes<double>(uint32_t, const uint32_t*, const uin
 template void launch_apply_bc_nodes<float>(uint32_t, const uint32_t*, const uint32_t*,
                                            const uint8_t*, float*, cudaStream_t);
 #define FM_INST(T)                                                                              \
-    template cudaError_t launch_spmv_csr<T>(uint32_t, uint64_t, const uint32_t*,                \
+    template cudaError_t launch_spmv_csr<T>(uint32_t, uint64_t, uint32_t, const uint32_t*,      \
                                             const uint32_t*, const T*, const T*, T*, T*,        \
                                             unsigned*, double*, cudaStream_t, const unsigned*); \
     template void launch_ilu0_csr<T>(const CsrDev&, const T*, T*, T*, unsigned*, unsigned,      \

@@ -77,9 +77,10 @@ cudaError_t launch_spmv_nodes(uint32_t n_nodes, uint32_t max_deg, const uint32_t
 // launchers below that return a cudaError_t return their first launch's
 // failure, with the kernels before it already queued.
 template <typename T>
-cudaError_t launch_spmv_csr(uint32_t n, uint64_t nnz, const uint32_t* rp, const uint32_t* ci,
-                            const T* val, const T* x, T* y, T* partials, unsigned* counter,
-                            double* dot, cudaStream_t s, const unsigned* skip = nullptr);
+cudaError_t launch_spmv_csr(uint32_t n, uint64_t nnz, uint32_t max_row, const uint32_t* rp,
+                            const uint32_t* ci, const T* val, const T* x, T* y, T* partials,
+                            unsigned* counter, double* dot, cudaStream_t s,
+                            const unsigned* skip = nullptr);
 
 // Sync-free ILU(0) and triangular solves on a CSR with ascending columns.
 // order: a topological order of the rows (dependency levels); done: one
