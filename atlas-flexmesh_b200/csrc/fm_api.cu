@@ -475,8 +475,9 @@ static std::vector<uint4> node_records(const fm::NodeGraph& g, const std::vector
 // 0.436 against 0.450 ms per FP32 pair, 0.616 against 0.708 FP64, at 64^3).
 // The default path; FM_TRSV_PATH=pipe selects the grid-wide pipelined solves
 // (fm_trsv.cu) instead.  FM_TRSV_PUSH_WARPS caps the warps per CTA (default:
-// 32 in FP32, 16 in FP64; smaller meshes take fewer), FM_TRSV_PUSH_BLOCK sets the interleave block
-// (default: chosen by the plan), FM_TRSV_PUSH_CLUSTER the cluster size.
+// 32 in FP32, 16 in FP64; fm_setup.hpp push_shape takes fewer on smaller
+// meshes), FM_TRSV_PUSH_BLOCK sets the interleave block (default: chosen by
+// the plan), FM_TRSV_PUSH_CLUSTER the cluster size.
 fm_status setup_push_solves(fm_ctx* c, const std::vector<uint32_t>& lp,
                             const std::vector<uint32_t>& lo, const std::vector<uint32_t>& up,
                             const std::vector<uint32_t>& uo) {
@@ -505,40 +506,26 @@ fm_status setup_push_solves(fm_ctx* c, const std::vector<uint32_t>& lp,
     std::stable_sort(sizes.begin(), sizes.end(), [](const auto& a, const auto& b) {
         return a.first * a.second > b.first * b.second;
     });
-    // Warps and clusters for the mesh's size.  A warp holds two nodes, and
-    // about 14 nodes in flight per node of an average level keep the front
-    // fed (later levels' loads overlap its hops); every further warp only
-    // polls, and every further cluster is one more slab boundary, crossed
-    // through L2.  Small meshes therefore take clusters of at most 16 warps
-    // per CTA, as many as that needs, large ones all clusters and up to 32
-    // warps (FP32; FP64's double-buffered loop 10 or 16).  us per FP32 / FP64
-    // pair against all clusters with 32 / 16 warps: 8^3 62 -> 43 / 69 -> 53,
-    // 16^3 110 -> 85 / 119 -> 104, 32^3 201 -> 173 / 220 -> 214, 48^3 307 ->
-    // 291 / 363 both; 64^3 takes them all.
-    const uint32_t levels = std::max<uint32_t>(1, (uint32_t)std::max(lp.size(), up.size()) - 1);
-    const uint32_t want = std::max(1u, (7 * c->nn + levels - 1) / levels);  // warps
+    const double width = fm::level_width(c->nn, lp, up);
     fm::PushPlan p;
     bool planned = false;
     int warps32 = cap32, warps64 = cap64;
-    auto plan = [&](uint32_t ncl, uint32_t cs) {
-        return fm::push_plan(c->graph, lp, lo, up, uo, ncl, cs, block,
-                             (uint32_t)(kMaxSmem / fm::push_smem_bytes(1, 8)), p) ||
-               fm::push_plan(c->graph, lp, lo, up, uo, ncl, cs, block,
-                             (uint32_t)(kMaxSmem / fm::push_smem_bytes(1, 4)), p);
-    };
+    const uint32_t slots64 = (uint32_t)(kMaxSmem / fm::push_smem_bytes(1, 8));
+    const uint32_t slots32 = (uint32_t)(kMaxSmem / fm::push_smem_bytes(1, 4));
     for (const auto& sz : sizes) {
         const uint32_t cs = sz.second, all = (uint32_t)sz.first;
-        const uint32_t few = std::min(all, (want + 16 * cs - 1) / (16 * cs));
+        fm::PushShape sh = fm::push_shape(width, all, cs);
         // fewer clusters only where FP64 slots fit as well
-        planned = few < all &&
-                  fm::push_plan(c->graph, lp, lo, up, uo, few, cs, block,
-                                (uint32_t)(kMaxSmem / fm::push_smem_bytes(1, 8)), p);
-        uint32_t ncl = few;
-        if (!planned) planned = plan(ncl = all, cs);
+        planned = sh.clusters < all &&
+                  fm::push_plan(c->graph, lp, lo, up, uo, sh.clusters, cs, block, slots64, p);
+        if (!planned) {
+            sh = fm::push_shape(width, all, cs, true);
+            planned = fm::push_plan(c->graph, lp, lo, up, uo, all, cs, block, slots64, p) ||
+                      fm::push_plan(c->graph, lp, lo, up, uo, all, cs, block, slots32, p);
+        }
         if (planned) {
-            const uint32_t per = (want + ncl * cs - 1) / (ncl * cs);
-            warps32 = std::min(cap32, (int)std::max(8u, (per + 3) & ~3u));
-            warps64 = std::min(cap64, warps32 <= 16 ? 10 : 16);
+            warps32 = std::min(cap32, (int)sh.warps32);
+            warps64 = std::min(cap64, (int)sh.warps64);
             break;
         }
     }

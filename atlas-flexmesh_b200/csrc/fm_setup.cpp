@@ -2,6 +2,7 @@
 #include "fm_setup.hpp"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 namespace fm {
@@ -157,6 +158,36 @@ uint32_t csr_levels(uint32_t n, const uint32_t* row_ptr, const uint32_t* col_idx
         maxd = std::max(maxd, d);
     }
     return levels_from_depth(depth, maxd, ptr, rows);
+}
+
+double level_width(uint32_t n_nodes, const std::vector<uint32_t>& fwd_ptr,
+                   const std::vector<uint32_t>& bwd_ptr) {
+    double most = 0.0;
+    for (const auto* p : {&fwd_ptr, &bwd_ptr}) {
+        double sum = 0.0;
+        for (size_t l = 0; l + 1 < p->size(); ++l) {
+            const double w = (*p)[l + 1] - (*p)[l];
+            sum += w * w;
+        }
+        most = std::max(most, sum / std::max(1u, n_nodes));
+    }
+    return most;
+}
+
+PushShape push_shape(double width, uint32_t available, uint32_t cluster, bool all) {
+    PushShape s;
+    if (!all && width <= 73.0) {
+        const bool narrow = width < 30.0;
+        s.warps64 = narrow ? 8 : 10;
+        s.warps32 = narrow ? 8 : 12;
+        return s;
+    }
+    const double fill = width / (2.6 * cluster);  // clusters the level fills
+    s.clusters = all ? available : std::min(available, (uint32_t)std::ceil(fill));
+    const double per = 4.8 * width / (s.clusters * cluster);  // warps per CTA it asks for
+    s.warps64 = per > 14.0 ? 16 : width > 230.0 ? 14 : 12;
+    s.warps32 = per <= 16.0 ? 16 : per >= 32.0 ? 32 : 4 * (uint32_t)std::ceil(per / 4.0);
+    return s;
 }
 
 bool push_plan(const NodeGraph& g, const std::vector<uint32_t>& fwd_ptr,

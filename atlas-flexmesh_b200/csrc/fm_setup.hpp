@@ -128,4 +128,31 @@ bool push_plan(const NodeGraph& g, const std::vector<uint32_t>& fwd_ptr,
                const std::vector<uint32_t>& bwd_order, uint32_t n_clusters, uint32_t cluster,
                uint32_t block, uint32_t max_slots, PushPlan& plan);
 
+// Clusters and warps per CTA of the push solves, before the caps on either,
+// from the level the typical node lies in (level_width: the mean level width
+// over nodes, not over levels; the wider direction).  A mean over levels
+// misses that a level's nodes may sit in few levels and few slabs, as on
+// breadth-first numberings.  A warp holds two nodes; every further warp only
+// polls, every further cluster is one more slab boundary, crossed through L2.
+//   * Up to 73 nodes a level one cluster keeps the front fed: 8 warps per CTA
+//     up to 30 nodes, else 10 (FP64) and 12 (FP32).
+//   * Above, a cluster for every 23 or so (its 9 CTAs at 12 warps hold 9 times
+//     that: later levels' loads overlap the front's hops), with 12 warps, 14
+//     beyond 230, and 16 in both once all clusters are taken and each CTA's
+//     part of the level asks for more than 14; FP32 then goes up to 32.
+// us per PCG iteration, FP64 / FP32, all 15 clusters with 16 / 32 warps -> this:
+// lattice cubes 8^3 101 / 96 -> 60 / 52, 16^3 157 / 145 -> 114 / 93, 32^3 280 /
+// 247 -> 246 / 199, 48^3 467 / 385 -> 426 / 340; the same cubes numbered breadth
+// first 20^3 273 / 247 -> 243 / 196, 32^3 476 / 420 -> 478 / 358, 40^3 638 /
+// 528 -> 615 / 488 (787 / 538 with the clusters sized by the mean over levels);
+// 4 x 4 x 800 beams 648-751 / 600-676 -> 602-611 / 512-525 (635-700 / 530-602).
+struct PushShape {
+    uint32_t clusters = 1, warps32 = 8, warps64 = 8;
+};
+double level_width(uint32_t n_nodes, const std::vector<uint32_t>& fwd_ptr,
+                   const std::vector<uint32_t>& bwd_ptr);
+// available: clusters of `cluster` CTAs that can be resident; all: take them
+// all whatever the width (a plan on fewer did not fit)
+PushShape push_shape(double width, uint32_t available, uint32_t cluster, bool all = false);
+
 }  // namespace fm
