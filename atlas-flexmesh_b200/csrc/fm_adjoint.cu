@@ -40,11 +40,11 @@ __device__ __forceinline__ Inv3 inverse3(const double F[9], double J) {
     return r;
 }
 
-// contributions of one tet to (K v) (transpose = 0) or (K^T w) (transpose =
-// 1) at its four vertices; ve: the tet's 12 direction values
-__device__ __forceinline__ void exact_contrib(const TetKin& k, double mu, double lam,
-                                              const double ve[12], int transpose,
-                                              double out[12]) {
+// one tet's part of (K v) (transpose = 0) or (K^T w) (transpose = 1): the
+// matrix Q whose product with a vertex's shape gradient, times vol, is the
+// contribution at that vertex; ve: the tet's 12 direction values
+__device__ __forceinline__ void exact_matrix(const TetKin& k, double mu, double lam,
+                                             const double ve[12], int transpose, double Q[9]) {
     double V[9];  // V_ik = sum_b v_b,i g_b,k
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -57,7 +57,7 @@ __device__ __forceinline__ void exact_contrib(const TetKin& k, double mu, double
     Inv3 Fi;
     if (vol_term) Fi = inverse3(F, k.J);
     if (!transpose) {
-        double dM[9];
+        double* dM = Q;
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -78,15 +78,8 @@ __device__ __forceinline__ void exact_contrib(const TetKin& k, double mu, double
             dM[4] += add;
             dM[8] += add;
         }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-                out[3 * a + i] = k.vol * (dM[3 * i] * k.d[a][0] + dM[3 * i + 1] * k.d[a][1] +
-                                          dM[3 * i + 2] * k.d[a][2]);
     } else {
         // V holds L here (same construction from w)
-        double Q[9];
 #pragma unroll
         for (int j = 0; j < 3; ++j)
 #pragma unroll
@@ -103,13 +96,15 @@ __device__ __forceinline__ void exact_contrib(const TetKin& k, double mu, double
 #pragma unroll
                 for (int c = 0; c < 3; ++c) Q[3 * j + c] += tr * Fi.m[3 * c + j];
         }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int j = 0; j < 3; ++j)
-                out[3 * a + j] = k.vol * (Q[3 * j] * k.d[a][0] + Q[3 * j + 1] * k.d[a][1] +
-                                          Q[3 * j + 2] * k.d[a][2]);
     }
+}
+
+// its contribution at the vertex with shape gradient g
+__device__ __forceinline__ void vertex_part(double vol, const double Q[9], const double g[3],
+                                            double out[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        out[i] = vol * (Q[3 * i] * g[0] + Q[3 * i + 1] * g[1] + Q[3 * i + 2] * g[2]);
 }
 
 __device__ __forceinline__ bool load_tet(const MeshDev& m, uint32_t e, const double* u,
@@ -131,6 +126,23 @@ __device__ __forceinline__ bool load_tet(const MeshDev& m, uint32_t e, const dou
     return tet_kinematics(x, ue, k);
 }
 
+// Q of tet e at displacement u and direction v; false: no contribution
+__device__ __forceinline__ bool tet_matrix(const MeshDev& m, uint32_t e, const double* u,
+                                           const double* v, int transpose, TetKin& k,
+                                           double Q[9]) {
+    uint32_t cn[4];
+    if (!load_tet(m, e, u, cn, k)) return false;
+    double mu, lam;
+    material_of(m.mat_mode, m.m0, m.m1, e, m.mu_s, m.lam_s, m.c_mu, m.c_lam, mu, lam);
+    double ve[12];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) ve[3 * a + d] = __ldg(v + 3 * (size_t)cn[a] + d);
+    exact_matrix(k, mu, lam, ve, transpose, Q);
+    return true;
+}
+
 // One thread per tet: the product's contributions at its four vertices into
 // fvert (12 per tet); a gather over each node's tets sums them.  Evaluating
 // each tet once instead of once per vertex, and without the 8 of 32 idle
@@ -141,24 +153,54 @@ __global__ void __launch_bounds__(128)
     chain_let_next();
     const uint32_t e = blockIdx.x * 128u + threadIdx.x;
     if (e >= m.n_elems) return;
-    uint32_t cn[4];
     TetKin k;
-    double out[12];
+    double Q[9], out[12];
 #pragma unroll
     for (int i = 0; i < 12; ++i) out[i] = 0.0;
-    if (load_tet(m, e, u, cn, k)) {
-        double mu, lam;
-        material_of(m.mat_mode, m.m0, m.m1, e, m.mu_s, m.lam_s, m.c_mu, m.c_lam, mu, lam);
-        double ve[12];
+    if (tet_matrix(m, e, u, v, transpose, k, Q))
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int d = 0; d < 3; ++d) ve[3 * a + d] = __ldg(v + 3 * (size_t)cn[a] + d);
-        exact_contrib(k, mu, lam, ve, transpose, out);
-    }
+        for (int a = 0; a < 4; ++a) vertex_part(k.vol, Q, k.d[a], out + 3 * a);
     double2* o = reinterpret_cast<double2*>(fvert + 12 * (size_t)e);
 #pragma unroll
     for (int i = 0; i < 6; ++i) o[i] = make_double2(out[2 * i], out[2 * i + 1]);
+}
+
+// The product on a mesh of few nodes: one warp per node, its lanes the node's
+// tets, each evaluated once per vertex but in a single kernel (kNodePass
+// below).  The sums run in the same order over the same terms.
+constexpr int kExactWarps = 8;
+__global__ void __launch_bounds__(kExactWarps * 32)
+    k_exact_nodes(MeshDev m, const double* __restrict__ u, const double* __restrict__ v,
+                  double* __restrict__ y, int transpose) {
+    __shared__ double part_s[kExactWarps][3 * 32];
+    const int lane = threadIdx.x & 31;
+    double* part = part_s[threadIdx.x >> 5];
+    const uint32_t n = blockIdx.x * kExactWarps + (threadIdx.x >> 5);
+    if (n >= m.n_nodes) return;  // uniform per warp
+    const uint32_t b = __ldg(m.act_ptr + n);
+    const int ma = (int)(__ldg(m.act_ptr + n + 1) - b);
+    double out[3] = {0.0, 0.0, 0.0};
+    if (lane < ma) {
+        const uint32_t at = __ldg(m.act_v + b + lane);
+        TetKin k;
+        double Q[9];
+        if (tet_matrix(m, at >> 2, u, v, transpose, k, Q)) {
+            const uint32_t a = at & 3u;  // selects: a runtime index would spill d
+            double g[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                g[c] = a == 0 ? k.d[0][c] : a == 1 ? k.d[1][c] : a == 2 ? k.d[2][c] : k.d[3][c];
+            vertex_part(k.vol, Q, g, out);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) part[3 * lane + c] = out[c];
+    __syncwarp();
+    if (lane < 3) {
+        double s = 0.0;
+        for (int l = 0; l < ma; ++l) s += part[3 * l + lane];
+        y[3 * (size_t)n + lane] = s;
+    }
 }
 
 // dL/dmu_e = -vol (C - I) : L_e, dL/dlam_e = -vol lnJ tr(L_e)
@@ -221,9 +263,20 @@ __global__ void k_adj_update(uint32_t n, const uint8_t* __restrict__ mask,
         if (!(mask && mask[i])) w[i] += dw[i];
 }
 
+// Up to this many nodes (two CTAs of eight warps on each of 148 SMs: one wave)
+// the product takes the node kernel: device us per product, node kernel /
+// element kernel and gather, 4^3 3.9 / 6.4, 8^3 4.1 / 6.7, 12^3 (2,197 nodes)
+// 5.1 / 7.2, 13^3 7.0 / 7.0, 16^3 10.3 / 8.0, 24^3 25 / 14.
+constexpr uint32_t kNodePass = 2368;
+
 void launch_exact_apply(const MeshDev& m, const double* u, const double* v, double* y,
                         int transpose, cudaStream_t s) {
     if (!m.n_nodes) return;
+    if (m.n_nodes <= kNodePass) {
+        k_exact_nodes<<<(m.n_nodes + kExactWarps - 1) / kExactWarps, kExactWarps * 32, 0, s>>>(
+            m, u, v, y, transpose);
+        return;
+    }
     if (m.n_elems)
         k_exact_elements<<<(m.n_elems + 127) / 128, 128, 0, s>>>(m, u, v, m.fvert, transpose);
     launch_gather_forces(m, y, nullptr, s);
