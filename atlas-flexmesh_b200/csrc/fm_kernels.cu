@@ -595,19 +595,19 @@ __global__ void __launch_bounds__(kElemWarps * 32)
         __syncwarp();
         double* o = K + 144 * (size_t)e0 + 36 * i;
 #pragma unroll 6
-        for (int t = lane; t < 32 * 36; t += 32) {
+        for (int t = lane; t < 36 * (int)n_rec; t += 32) {
             const int rec = t / 36, w = t - 36 * rec;
-            if (rec < (int)n_rec) o[144 * (size_t)rec + w] = stage[rec * 37 + w];
+            o[144 * (size_t)rec + w] = stage[rec * 37 + w];
         }
         __syncwarp();
     }
 #pragma unroll
     for (int q = 0; q < 12; ++q) stage[lane * 13 + q] = fI[q];
     __syncwarp();
-#pragma unroll
-    for (int t = lane; t < 32 * 12; t += 32) {
+#pragma unroll 4
+    for (int t = lane; t < 12 * (int)n_rec; t += 32) {
         const int rec = t / 12;
-        if (rec < (int)n_rec) f[12 * (size_t)e0 + t] = stage[rec * 13 + (t - 12 * rec)];
+        f[12 * (size_t)e0 + t] = stage[rec * 13 + (t - 12 * rec)];
     }
     if (flags) raise_flag(status, flags);
 }
