@@ -790,10 +790,12 @@ fm_status need_material(fm_ctx* c) {
     return FM_OK;
 }
 
+constexpr size_t kMatrixRoom = 4;  // entries of K past its end: 16-byte copies of the last ones
+
 template <typename T>
 fm_status ensure_matrix(fm_ctx* c) {
     Work<T>& w = work<T>(c);
-    CK(w.K.reserve(c->nnz + 4));  // room for 16-byte copies of its last entries
+    CK(w.K.reserve(c->nnz + kMatrixRoom));
     CK(w.LU.reserve(c->nnz));
     CK(w.diag.reserve(c->n));
     CK(w.dinv.reserve(c->n));
@@ -1373,7 +1375,10 @@ fm_status fm_ilu0_apply_noalloc(fm_ctx* c, const double* r, double* y) {
 
 fm_status fm_spmv(fm_ctx* c, const double* x, double* y) {
     TRY(need_mesh(c));
-    if (!x || !y || !c->w64.K.p) return fail(c, FM_ERR_ARG, "null argument or no K");
+    if (!x || !y) return fail(c, FM_ERR_ARG, "null argument");
+    // a K of an earlier mesh may be smaller than the copies of its tiles
+    if (c->w64.K.n < c->nnz + kMatrixRoom)
+        return fail(c, FM_ERR_ARG, "no K of this mesh: call fm_assemble(FM_FP64) first");
     Op<double> A{c, &c->fem, true, c->w64.K.p, nullptr, nullptr, nullptr, 0};
     CK(A.spmv(x, y, nullptr));
     return FM_OK;
