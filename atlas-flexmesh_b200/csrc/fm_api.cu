@@ -1017,6 +1017,14 @@ fm_status fm_set_mesh(fm_ctx* c, uint32_t n_nodes, const double* xyz, uint32_t n
         for (size_t q = 0; q < 4 * (size_t)n_elems; ++q)
             if (conn[q] >= n_nodes)
                 return fail(c, FM_ERR_ARG, "conn[%zu] = %u out of range", q, conn[q]);
+        // A call that fails from here on leaves the context without a mesh: on
+        // half of a new one, kernels would run past the end of the other half.
+        struct Unset {
+            fm_ctx* c;
+            ~Unset() {
+                if (c) c->nn = c->ne = c->n = 0, c->nnz = 0;
+            }
+        } unset{c};
         c->nn = n_nodes;
         c->ne = n_elems;
         c->n = 3 * n_nodes;
@@ -1087,6 +1095,7 @@ fm_status fm_set_mesh(fm_ctx* c, uint32_t n_nodes, const double* xyz, uint32_t n
         CK(c->fvert.reserve(12 * (size_t)c->ne));
         CK(c->tan_rec.reserve((size_t)c->ne * fm::kTanRecBytes));
         CK(cudaStreamSynchronize(c->stream));
+        unset.c = nullptr;
     } catch (const std::bad_alloc&) {
         return fail(c, FM_ERR_OOM, "host allocation failed in fm_set_mesh");
     }

@@ -139,7 +139,9 @@ fm_status fm_unit_cube(int N, double* xyz, uint32_t* conn);
  * incidence, the node neighbour sets, the ILU(0) dependency levels and
  * schedules and the assembly's scatter structure on the device (the
  * reference builds its neighbour sets per node with std::set, :1076-1085),
- * and the triangular-solve plan on the host.  Clears the flags. */
+ * and the triangular-solve plan on the host.  Clears the flags.  Arguments that
+ * are refused leave the context as it was; a call that fails after that leaves
+ * it without a mesh. */
 fm_status fm_set_mesh(fm_ctx* ctx, uint32_t n_nodes, const double* xyz, uint32_t n_elems,
                       const uint32_t* conn, const double* elem_volume);
 
@@ -240,7 +242,8 @@ fm_status fm_ilu0_apply(fm_ctx* ctx, const double* r_dev, double* y_dev);
 fm_status fm_ilu0_apply_noalloc(fm_ctx* ctx, const double* r_dev, double* y_dev);
 
 /* ---- A17/A18: SpMV and PCG on the context's K -----------------------------
- * fm_spmv replaces SparseCSR::matvec (FEM/fem_types.hpp:310-319).
+ * fm_spmv replaces SparseCSR::matvec (FEM/fem_types.hpp:310-319); FM_ERR_ARG
+ * before the first FP64 assembly on a mesh larger than the ones before it.
  * fm_pcg replaces pcg_solve_ilu0 (FEM/adaptive_fem_engine.hpp:1283-1341) with
  * the same stop tests; the factorization from fm_ilu0 is reused (call
  * fm_ilu0 first, as the reference refactors on entry).  *iters = iterations

@@ -204,6 +204,31 @@ int main() {
                 return st != FM_OK ? st : fm_newton_step_cfg(c, u.data(), 0.5, &cfg, &res);
             }, "k_trsv_push");
 
+    // a mesh that could not be set leaves none: later calls launch nothing
+    {
+        fm_ctx* c = nullptr;
+        EXPECT(fm_create(&c, 0, nullptr) == FM_OK && mesh(c) == FM_OK, "no first mesh");
+        launches.clear();
+        EXPECT(mesh(c) == FM_OK, "no second mesh");
+        for (int k = 0, all = (int)launches.size(); k < all; ++k) {
+            launches.clear();
+            refuse = k;
+            EXPECT(mesh(c) == FM_ERR_CUDA, "launch %d of fm_set_mesh refused", k);
+            refuse = -1;
+            launches.clear();
+            uint32_t nodes = 7;
+            EXPECT(fm_sizes(c, &nodes, nullptr, nullptr, nullptr) == FM_OK && nodes == 0,
+                   "launch %d: %u nodes", k, nodes);
+            EXPECT(fm_residual(c, u.data(), f.data()) == FM_ERR_ARG &&
+                       fm_assemble(c, u.data(), nullptr, f.data(), FM_FP64, 0) == FM_ERR_ARG &&
+                       fm_spmv(c, f.data(), y.data()) == FM_ERR_ARG && launches.empty(),
+                   "launch %d: half a mesh is used", k);
+            EXPECT(mesh(c) == FM_OK && fm_residual(c, u.data(), f.data()) == FM_OK,
+                   "launch %d: no mesh afterwards", k);
+        }
+        fm_destroy(c);
+    }
+
     if (!bad) std::printf("ok\n");
     return bad != 0;
 }
