@@ -460,11 +460,7 @@ static void launch_node_pass(const MeshDev& m, KT* K, double* f, double* R, int 
     const unsigned grid = std::min<unsigned>((m.n_nodes + kAsmWarps<KT> - 1) / kAsmWarps<KT>,
                                              148u * kAsmCtas<KT>);
     constexpr size_t smem = kAsmWarps<KT> * sizeof(AsmWarp<KT, PL>);
-    // above the 48 KB every kernel may use the limit has to be raised (per
-    // device, on each launch: the call is cheap and keeps no state)
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_assemble<KT, PL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+    static_assert(smem <= 48 * 1024, "what a kernel may use without raising its limit");
     launch_chained(k_assemble<KT, PL>, grid, kAsmWarps<KT> * 32, smem, s, m,
                    static_cast<const TanRec<KT>*>(m.tan_rec), K, f, R, apply_bc);
 }

@@ -248,9 +248,10 @@ cudaError_t launch_stages(uint32_t nn, const StageLayout& L, int per_sm, const u
 
 }  // namespace
 
-// Four CTAs per SM with as many stages as their shared memory holds (about
-// 60 KB in flight per SM either way); a mesh of the largest valence, 32,
-// still fits two.
+// As many CTAs per SM as each has stages: four of four where an SM's shared
+// memory holds 16 stages (FP64 up to 11 neighbours, FP32 up to 21; 64^3 FP32 4 x
+// 49.2 KB), else three of three (FP64 up to 20, 64^3 3 x 69.7 KB; FP32 up to the
+// limit of 32), else two of two (FP64 up to 32, 2 x 78.1 KB).
 template <typename T>
 cudaError_t launch_spmv_nodes(uint32_t nn, uint32_t max_deg, const uint32_t* nbr_ptr,
                               const uint32_t* nbr, const T* val, const T* x, T* y, T* partials,
@@ -260,11 +261,14 @@ cudaError_t launch_spmv_nodes(uint32_t nn, uint32_t max_deg, const uint32_t* nbr
     if (16 * (size_t)L.bytes <= kSmStages)
         return launch_stages<T, 4>(nn, L, 4, nbr_ptr, nbr, val, x, y, partials, counter, dot,
                                    status, s, skip);
-    if (9 * (size_t)L.bytes <= kSmStages)
+    // (in FP32 the largest valence still fits three)
+    if (sizeof(T) == 4 || 9 * (size_t)L.bytes <= kSmStages)
         return launch_stages<T, 3>(nn, L, 3, nbr_ptr, nbr, val, x, y, partials, counter, dot,
                                    status, s, skip);
-    return launch_stages<T, 2>(nn, L, 2, nbr_ptr, nbr, val, x, y, partials, counter, dot, status,
-                               s, skip);
+    if constexpr (sizeof(T) == 8)
+        return launch_stages<T, 2>(nn, L, 2, nbr_ptr, nbr, val, x, y, partials, counter, dot,
+                                   status, s, skip);
+    return cudaErrorInvalidValue;  // not reached
 }
 template cudaError_t launch_spmv_nodes<double>(uint32_t, uint32_t, const uint32_t*, const uint32_t*,
                                                const double*, const double*, double*, double*,

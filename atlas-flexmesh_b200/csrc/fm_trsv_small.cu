@@ -30,8 +30,6 @@ namespace fm {
 
 namespace {
 
-constexpr int kMaxDepth = 1;  // levels whose entries are in flight
-
 template <int M>
 struct Row {
     double v[M];
@@ -61,35 +59,28 @@ __device__ __forceinline__ void solve_row(const Row<M>& E, double* z) {
     z[E.row] = Upper ? s * E.d : s;
 }
 
-// one direction, in place on z (z[n] = 0 for the padding); lvl[n_levels ..
-// n_levels + D] = n
-template <int M, int D, bool Wide, bool Upper>
+// one direction, in place on z (z[n] = 0 for the padding); lvl[n_levels] and
+// lvl[n_levels + 1] = n
+template <int M, bool Wide, bool Upper>
 __device__ __forceinline__ void sweep(const SmallTri& S, const uint32_t* lvl, uint32_t n,
                                       double* z) {
-    Row<M> e[D];
-#pragma unroll
-    for (int q = 0; q < D; ++q) load_row<M, Upper>(S, min(lvl[q] + threadIdx.x, n - 1), n, e[q]);
-    for (uint32_t l0 = 0; l0 < S.n_levels; l0 += D) {
-#pragma unroll
-        for (int q = 0; q < D; ++q) {
-            const uint32_t l = l0 + q;
-            if (l < S.n_levels) {  // uniform
-                const uint32_t b = lvl[l], end = lvl[l + 1], next = lvl[l + D];
-                if (b + threadIdx.x < end) solve_row<M, Upper>(e[q], z);
-                if (Wide)  // rows of a level beyond the block's width
-                    for (uint32_t t = b + threadIdx.x + blockDim.x; t < end; t += blockDim.x) {
-                        Row<M> x;
-                        load_row<M, Upper>(S, t, n, x);
-                        solve_row<M, Upper>(x, z);
-                    }
-                load_row<M, Upper>(S, min(next + threadIdx.x, n - 1), n, e[q]);
-                __syncthreads();
+    Row<M> e;
+    load_row<M, Upper>(S, min(lvl[0] + threadIdx.x, n - 1), n, e);
+    for (uint32_t l = 0; l < S.n_levels; ++l) {
+        const uint32_t b = lvl[l], end = lvl[l + 1];
+        if (b + threadIdx.x < end) solve_row<M, Upper>(e, z);
+        if (Wide)  // rows of a level beyond the block's width
+            for (uint32_t t = b + threadIdx.x + blockDim.x; t < end; t += blockDim.x) {
+                Row<M> x;
+                load_row<M, Upper>(S, t, n, x);
+                solve_row<M, Upper>(x, z);
             }
-        }
+        load_row<M, Upper>(S, min(end + threadIdx.x, n - 1), n, e);
+        __syncthreads();
     }
 }
 
-template <int M, int D, int Threads, bool Wide>
+template <int M, int Threads, bool Wide>
 __global__ void __launch_bounds__(Threads, 1)
     k_trsv_small(SmallTri L, SmallTri U, uint32_t n, const double* r, double* out,
                  const unsigned* skip) {
@@ -98,17 +89,17 @@ __global__ void __launch_bounds__(Threads, 1)
     extern __shared__ __align__(16) unsigned char small_smem[];
     double* z = reinterpret_cast<double*>(small_smem);
     uint32_t* lf = reinterpret_cast<uint32_t*>(z + n + 1);
-    uint32_t* lb = lf + L.n_levels + 1 + D;
+    uint32_t* lb = lf + L.n_levels + 2;
 #pragma unroll 8
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) z[i] = ld_prev(r + i);
     if (threadIdx.x == 0) z[n] = 0.0;
-    for (uint32_t i = threadIdx.x; i <= L.n_levels + D; i += blockDim.x)
+    for (uint32_t i = threadIdx.x; i <= L.n_levels + 1; i += blockDim.x)
         lf[i] = i < L.n_levels ? __ldg(L.level + i) : n;
-    for (uint32_t i = threadIdx.x; i <= U.n_levels + D; i += blockDim.x)
+    for (uint32_t i = threadIdx.x; i <= U.n_levels + 1; i += blockDim.x)
         lb[i] = i < U.n_levels ? __ldg(U.level + i) : n;
     __syncthreads();
-    sweep<M, D, Wide, false>(L, lf, n, z);
-    sweep<M, D, Wide, true>(U, lb, n, z);
+    sweep<M, Wide, false>(L, lf, n, z);
+    sweep<M, Wide, true>(U, lb, n, z);
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) out[i] = z[i];
 }
 
@@ -126,16 +117,16 @@ __global__ void k_pack_small(uint32_t n, uint32_t total, const uint32_t* __restr
     }
 }
 
-template <int M, int D, int Threads, bool Wide>
+template <int M, int Threads, bool Wide>
 cudaError_t launch_w(const SmallTri& L, const SmallTri& U, uint32_t n, unsigned th, size_t smem,
                      const double* r, double* out, const unsigned* skip, cudaStream_t s) {
     // one limit for every matrix: it is the kernel's, not the call's, and
     // another thread may be between its own call and launch
     const cudaError_t e =
-        cudaFuncSetAttribute(k_trsv_small<M, D, Threads, Wide>,
+        cudaFuncSetAttribute(k_trsv_small<M, Threads, Wide>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMaxSmem);
     if (e != cudaSuccess) return e;
-    return launch_chained(k_trsv_small<M, D, Threads, Wide>, 1, th, smem, s, L, U, n, r, out, skip);
+    return launch_chained(k_trsv_small<M, Threads, Wide>, 1, th, smem, s, L, U, n, r, out, skip);
 }
 
 // threads of the widest block that the registers of a row allow
@@ -147,19 +138,19 @@ unsigned threads_for(uint32_t entries, uint32_t n, uint32_t width) {
                     std::max(32u, (std::max(width, n / 64) + 31u) & ~31u));
 }
 
-template <int M, int D, int Threads>
+template <int M, int Threads>
 cudaError_t launch_t(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t width,
                      const double* r, double* out, const unsigned* skip, cudaStream_t s) {
     const size_t smem = small_tri_smem(n, L.n_levels, U.n_levels);
     const unsigned th = threads_for(M, n, width);
-    return width > th ? launch_w<M, D, Threads, true>(L, U, n, th, smem, r, out, skip, s)
-                      : launch_w<M, D, Threads, false>(L, U, n, th, smem, r, out, skip, s);
+    return width > th ? launch_w<M, Threads, true>(L, U, n, th, smem, r, out, skip, s)
+                      : launch_w<M, Threads, false>(L, U, n, th, smem, r, out, skip, s);
 }
 
 }  // namespace
 
 size_t small_tri_smem(uint32_t n, uint32_t nlf, uint32_t nlb) {
-    return 8 * ((size_t)n + 1) + 4 * ((size_t)nlf + nlb + 2 + 2 * kMaxDepth);
+    return 8 * ((size_t)n + 1) + 4 * ((size_t)nlf + nlb + 4);
 }
 
 // A level costs the warp-per-row solves about 3.9 us whatever its width (148
@@ -194,9 +185,9 @@ void launch_pack_small(uint32_t n, uint32_t entries, const uint32_t* src_f, cons
 cudaError_t launch_trsv_small(const SmallTri& L, const SmallTri& U, uint32_t n, uint32_t entries,
                               uint32_t width, const double* r, double* out, const unsigned* skip,
                               cudaStream_t s) {
-    if (entries <= 2) return launch_t<2, 1, max_threads(2)>(L, U, n, width, r, out, skip, s);
-    if (entries <= 4) return launch_t<4, 1, max_threads(4)>(L, U, n, width, r, out, skip, s);
-    return launch_t<8, 1, max_threads(8)>(L, U, n, width, r, out, skip, s);
+    if (entries <= 2) return launch_t<2, max_threads(2)>(L, U, n, width, r, out, skip, s);
+    if (entries <= 4) return launch_t<4, max_threads(4)>(L, U, n, width, r, out, skip, s);
+    return launch_t<8, max_threads(8)>(L, U, n, width, r, out, skip, s);
 }
 
 }  // namespace fm
