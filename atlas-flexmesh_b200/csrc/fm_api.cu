@@ -1441,12 +1441,14 @@ fm_status fm_csr_pcg_ilu0(fm_ctx* c, uint32_t n, const uint32_t* row_ptr,
         for (uint32_t i = 0; i < n; ++i) {
             if (rp[i + 1] < rp[i] || rp[i + 1] > nnz)
                 return fail(c, FM_ERR_ARG, "row_ptr not monotone at row %u", i);
-            row.clear();
+            bool sorted = true;
             for (uint32_t k = rp[i]; k < rp[i + 1]; ++k) {
                 if (ci[k] >= n) return fail(c, FM_ERR_ARG, "column %u out of range", ci[k]);
-                row.emplace_back(ci[k], v[k]);
+                sorted = sorted && (k == rp[i] || ci[k - 1] <= ci[k]);
             }
-            if (std::is_sorted(ci.begin() + rp[i], ci.begin() + rp[i + 1])) continue;
+            if (sorted) continue;
+            row.clear();
+            for (uint32_t k = rp[i]; k < rp[i + 1]; ++k) row.emplace_back(ci[k], v[k]);
             std::stable_sort(row.begin(), row.end(),
                              [](const auto& a, const auto& b2) { return a.first < b2.first; });
             for (size_t q = 0; q < row.size(); ++q) {
@@ -1471,6 +1473,9 @@ fm_status fm_csr_pcg_ilu0(fm_ctx* c, uint32_t n, const uint32_t* row_ptr,
                                   c->gen.bwd.p, c->gen_LU.p, c->gen_diag.p, c->gen.val_f.p,
                                   c->gen.val_b.p, c->gen.dinv_b.p, c->stream);
             CK(cudaGetLastError());
+            // an ordinary operation: the packed factors are complete before any
+            // kernel of the chain starts (ld_prev)
+            CK(cudaMemsetAsync(&c->sc.p->stop, 0, sizeof(unsigned), c->stream));
         }
         Op<double> A{c, &c->gen, false, c->gen_K.p, c->gen_LU.p, c->gen_diag.p, c->w64.t.p,
                      c->grid_trsv64};

@@ -114,7 +114,9 @@ inline cudaLaunchConfig_t launch_config(unsigned grid, unsigned block, size_t sm
 // it, as __ldg and a const __restrict__ parameter would promise (they may read
 // it through the read-only path and ahead of the wait); volatile keeps this
 // load behind chain_wait.  What was complete before the chain began (matrix,
-// factors, plans) may be read either way.
+// factors, plans) may be read either way: between those and the first chained
+// kernel either the host has waited or the stream has an ordinary operation (a
+// copy, a fill, a kernel of its own), which starts when they are complete.
 __device__ __forceinline__ double ld_prev(const double* p) {
     double v;
     asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));

@@ -675,15 +675,17 @@ __global__ void __launch_bounds__(256)
     const uint32_t steps = (n + ngroups - 1) / ngroups;
     for (uint32_t q = 0; q < steps; ++q) {
         const uint32_t i = group + q * ngroups;
-        T s = T(0);
-        if (i < n)
+        T s = T(0), xi = T(0);
+        if (i < n) {
+            if (dot && lane == 0) xi = ld_prev(x + i);
             for (uint32_t k = rp[i] + lane; k < rp[i + 1]; k += G)
                 s += __ldg(val + k) * ld_prev(x + ci[k]);
+        }
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
         if (i < n && lane == 0) {
             y[i] = s;
-            if (dot) dsum += s * ld_prev(x + i);
+            dsum += s * xi;
         }
     }
     if (dot) {
@@ -961,24 +963,40 @@ void launch_dot(uint32_t n, const T* x, const T* y, T* partials, unsigned* count
 // PCG entry: r = b - r (zero_x: r = b, the start vector is zero), rr = r.r,
 // the early exit ||r|| < tol 1e-3 as the reference takes it (:1298), and the
 // wait sentinel into tmp (null: none) for the solve that follows.
+// The grid's elements four at a time: load(q, i) for each of them, then use(q,
+// i), in ascending order.  A store may alias a later load as far as the
+// compiler can tell, so loads written behind stores wait for them.
+template <typename Load, typename Use>
+__device__ __forceinline__ void by_four(uint32_t n, Load load, Use use) {
+    const uint32_t step = gridDim.x * blockDim.x;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * step) {
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+            if (i0 + q * step < n) load(q, i0 + q * step);
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+            if (i0 + q * step < n) use(q, i0 + q * step);
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads)
     k_pcg_init(uint32_t n, const T* b, T* __restrict__ r, int zero_x, T* __restrict__ tmp,
                double tol, T* partials, unsigned* counter, DevScalars* sc, PcgReport* rep,
                unsigned seq) {
-    // in this order: the kernels behind this one start when all that ran before
-    // it (the factorization among them) is complete
-    chain_wait();
-    chain_let_next();
-    T s = T(0);
-#pragma unroll 4
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x) {
-        const T bi = ld_prev(b + i), v = zero_x ? bi : bi - r[i];
-        r[i] = v;
-        if (tmp) tmp[i] = Sentinel<T>::value();
-        s += v * v;
-    }
+    chain_begin();
+    T s = T(0), v[4];
+    by_four(
+        n,
+        [&](uint32_t q, uint32_t i) {
+            v[q] = ld_prev(b + i);
+            if (!zero_x) v[q] -= r[i];
+        },
+        [&](uint32_t q, uint32_t i) {
+            r[i] = v[q];
+            if (tmp) tmp[i] = Sentinel<T>::value();
+            s += v[q] * v[q];
+        });
     __shared__ T sbuf[32];
     const T bt = block_sum(s, sbuf);
     grid_reduce_finish<T>(bt, partials, counter, [&](T total) {
@@ -1003,15 +1021,19 @@ __global__ void __launch_bounds__(kVecThreads)
                 unsigned* counter, DevScalars* sc) {
     chain_begin();
     if (skipped(&sc->done)) return;
-    T s1 = T(0), s2 = T(0);
-#pragma unroll 4
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x) {
-        const T zi = ld_prev(z + i), bi = ld_prev(b + i);
-        p[i] = zi;
-        s1 += ld_prev(r + i) * zi;
-        s2 += bi * bi;
-    }
+    T s1 = T(0), s2 = T(0), zv[4], rv[4], bv[4];
+    by_four(
+        n,
+        [&](uint32_t q, uint32_t i) {
+            zv[q] = ld_prev(z + i);
+            rv[q] = ld_prev(r + i);
+            bv[q] = ld_prev(b + i);
+        },
+        [&](uint32_t q, uint32_t i) {
+            p[i] = zv[q];
+            s1 += rv[q] * zv[q];
+            s2 += bv[q] * bv[q];
+        });
     __shared__ T sbuf[32];
     const T b1 = block_sum(s1, sbuf);
     const T b2 = block_sum(s2, sbuf);
@@ -1045,13 +1067,20 @@ __global__ void __launch_bounds__(kVecThreads)
         return;
     }
     const T alpha = (T)(sc->rz_new / pAp);
-#pragma unroll 4
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x) {
-        x[i] += alpha * ld_prev(p + i);
-        r[i] -= alpha * ld_prev(Ap + i);
-        if (tmp) tmp[i] = Sentinel<T>::value();
-    }
+    T pv[4], av[4], xv[4], rv[4];
+    by_four(
+        n,
+        [&](uint32_t q, uint32_t i) {
+            pv[q] = ld_prev(p + i);
+            av[q] = ld_prev(Ap + i);
+            xv[q] = x[i];
+            rv[q] = r[i];
+        },
+        [&](uint32_t q, uint32_t i) {
+            x[i] = xv[q] + alpha * pv[q];
+            r[i] = rv[q] - alpha * av[q];
+            if (tmp) tmp[i] = Sentinel<T>::value();
+        });
 }
 template <typename T>
 cudaError_t launch_pcg_update_xr(uint32_t n, const T* p, const T* Ap, T* x, T* r, T* tmp,
@@ -1106,10 +1135,14 @@ __global__ void __launch_bounds__(kVecThreads)
     chain_begin();
     if (skipped(&sc->done)) return;
     const T beta = (T)(sc->rz_new / sc->rz);
-#pragma unroll 4
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x)
-        p[i] = ld_prev(z + i) + beta * p[i];
+    T zv[4], pv[4];
+    by_four(
+        n,
+        [&](uint32_t q, uint32_t i) {
+            zv[q] = ld_prev(z + i);
+            pv[q] = p[i];
+        },
+        [&](uint32_t q, uint32_t i) { p[i] = zv[q] + beta * pv[q]; });
 }
 template <typename T>
 cudaError_t launch_pcg_update_p(uint32_t n, const T* z, T* p, DevScalars* sc, cudaStream_t s) {
