@@ -530,7 +530,7 @@ __device__ __forceinline__ bool element_full(const double x[12], const double ue
 // time and leaves through the warp's stage, neighbouring lanes storing
 // neighbouring words (a lane's own stores, 1,152 bytes from the next lane's,
 // wrote a quarter of a sector each: 457 us for a call with 200,003 tets, now
-// 87, 44 of them the bytes at copy bandwidth).  Stage rows of 37 doubles have no
+// 85, 44 of them the bytes at copy bandwidth).  Stage rows of 37 doubles have no
 // bank conflicts on the way in.
 constexpr int kElemWarps = 4;
 

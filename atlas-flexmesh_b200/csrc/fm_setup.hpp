@@ -141,11 +141,11 @@ bool push_plan(const NodeGraph& g, const std::vector<uint32_t>& fwd_ptr,
 //     beyond 230, and 16 in both once all clusters are taken and each CTA's
 //     part of the level asks for more than 14; FP32 then goes up to 32.
 // us per PCG iteration, FP64 / FP32, all 15 clusters with 16 / 32 warps -> this:
-// lattice cubes 8^3 101 / 96 -> 60 / 52, 16^3 157 / 145 -> 114 / 93, 32^3 280 /
-// 247 -> 246 / 199, 48^3 467 / 385 -> 426 / 340; the same cubes numbered breadth
-// first 20^3 273 / 247 -> 243 / 196, 32^3 476 / 420 -> 478 / 358, 40^3 638 /
-// 528 -> 615 / 488 (787 / 538 with the clusters sized by the mean over levels);
-// 4 x 4 x 800 beams 648-751 / 600-676 -> 602-611 / 512-525 (635-700 / 530-602).
+// lattice cubes 8^3 101 / 96 -> 60 / 52, 16^3 158 / 145 -> 114 / 95, 32^3 280 /
+// 247 -> 246 / 199, 48^3 467 / 385 -> 423 / 338; the same cubes numbered breadth
+// first 20^3 273 / 247 -> 243 / 196, 32^3 476 / 420 -> 478 / 355, 40^3 638 /
+// 528 -> 626 / 499 (788 / 538 with the clusters sized by the mean over levels);
+// 4 x 4 x 800 beams 648-751 / 600-676 -> 600-611 / 511-524 (635-700 / 530-602).
 struct PushShape {
     uint32_t clusters = 1, warps32 = 8, warps64 = 8;
 };
